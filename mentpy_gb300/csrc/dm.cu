@@ -44,24 +44,47 @@ static int launch_dm_fact(const DmArgs &a, int64_t batch, cudaStream_t s) {
   return check_launch("dm_fwd_fact");
 }
 
-// Windows 9..11: R in the workspace, one 1024-thread block per resident run.
+// Windows 9..11: R in the workspace, a cluster of 512-thread blocks per run in flight.
 static int64_t dm_ws_slots(int64_t batch) { return std::min<int64_t>(batch, (int64_t)sm_count()); }
 
+template <int W, int CS>
+static int launch_dm_fact_cluster(const DmArgs &a, int64_t slots, float2 *ws, cudaStream_t s) {
+  const size_t smem = dm_fact_slice_bytes<W>(a.maxm);
+  if (smem > (size_t)227 * 1024)
+    return fail(MBQC_E_UNSUPPORTED, "dm_forward: %d steps need %zu bytes of shared memory", a.maxm, smem);
+  auto k = dm_fwd_fact_ws<W, CS>;
+  int rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                      "dm smem attribute");
+  if (rc) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(slots * CS));
+  cfg.blockDim = dim3(kFactWsThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  rc = cuda_check(cudaLaunchKernelEx(&cfg, k, a, ws), "dm_fwd_fact_ws cluster launch");
+  return rc ? rc : check_launch("dm_fwd_fact_ws");
+}
+
+// Blocks per run: as many as keep all runs resident at two 512-thread blocks
+// an SM, eight (the portable cluster size) at most and two at least.
 template <int W>
 static int launch_dm_fact_ws(const DmArgs &a, int64_t batch, void *ws, size_t ws_bytes, cudaStream_t s) {
   const size_t per = (size_t)DmFactCfg<W>::N * sizeof(float2);
   const int64_t slots = std::min<int64_t>(dm_ws_slots(batch), (int64_t)(ws_bytes / per));
   if (!ws || slots < 1)
     return fail(MBQC_E_INVALID, "dm_forward: window %d needs a workspace of at least %zu bytes", W, per);
-  const size_t smem = dm_fact_slice_bytes<W>(a.maxm);
-  if (smem > (size_t)227 * 1024)
-    return fail(MBQC_E_UNSUPPORTED, "dm_forward: %d steps need %zu bytes of shared memory", a.maxm, smem);
-  auto k = dm_fwd_fact_ws<W>;
-  int rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "dm smem attribute");
-  if (rc) return rc;
-  k<<<(int)slots, 1024, smem, s>>>(a, static_cast<float2 *>(ws));
-  return check_launch("dm_fwd_fact_ws");
+  float2 *w = static_cast<float2 *>(ws);
+  const int64_t room = 2 * (int64_t)sm_count();
+  if (slots * 8 <= room) return launch_dm_fact_cluster<W, 8>(a, slots, w, s);
+  if (slots * 4 <= room) return launch_dm_fact_cluster<W, 4>(a, slots, w, s);
+  return launch_dm_fact_cluster<W, 2>(a, slots, w, s);
 }
 
 template <int W>

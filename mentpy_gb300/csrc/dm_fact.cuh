@@ -25,12 +25,13 @@
 // from the initial pure window state directly.
 #pragma once
 
+#include "cluster_sum.cuh"
 #include "dm.cuh"
 
 namespace mbqc {
 
 // Windows up to 8 keep R in shared memory; windows 9..11 (R of 512 KB to
-// 8 MB) keep it in a device workspace, one 1024-thread block per run.
+// 8 MB) keep it in a device workspace, a cluster of blocks per run.
 constexpr int kDmFactSmemMaxWindow = 8;
 constexpr int kDmFactMaxWindow = 11;
 
@@ -42,9 +43,9 @@ template <int W> struct DmFactCfg {
   static constexpr int NB = N / 4;        // 2x2 blocks per step
   static constexpr int DW = 1 << W;       // amplitudes of the initial window
   static constexpr bool kSmemR = W <= kDmFactSmemMaxWindow;
-  // threads per run: ~8 blocks each, one warp at least, a block at most
-  // (1024 threads for a workspace-resident R)
-  static constexpr int TPR = !kSmemR ? 1024 : (NB / 8 < 32 ? 32 : (NB / 8 > 256 ? 256 : NB / 8));
+  // threads per run (shared-memory windows): ~8 blocks each, one warp at
+  // least, a block at most
+  static constexpr int TPR = NB / 8 < 32 ? 32 : (NB / 8 > 256 ? 256 : NB / 8);
 };
 
 // Per-step word of the factored pass (staged once per run):
@@ -107,16 +108,72 @@ __device__ __forceinline__ float2 group_sum2_db(float v, float2 *scratch, int ti
   return make_float2(s, lo - (s - hi));
 }
 
+// Step words and final positions, every step on its own: the qubit at
+// schedule index s (initial window or entering) is always stored at position
+// (s - 1) mod (W - 1), since an entering qubit takes the position of the qubit
+// measured W - 1 steps later than its predecessor there.  (As one thread's
+// walk over the steps with a running position table this took ~10 us of a
+// 66-step window-7 run.)
+template <int W>
+__device__ __forceinline__ void fact_tables(const DevStep *steps, int M, uint2 *sSt, int8_t *sPos, int tid, int n) {
+  for (int k = tid; k < M; k += n) {
+    uint32_t aux = steps[k].plane == MBQC_PLANE_Z ? kFactZ : 0u, sgn = 0u;
+    if (k > 0) {
+      const uint32_t pmask = steps[k - 1].mask;
+      const int q = k % W;
+      aux |= (uint32_t)((k - 1) % (W - 1));
+      if (pmask & kDead) {
+        aux |= kFactDead;
+      } else {
+        if ((pmask >> q) & 1u) aux |= kFactMq;
+#pragma unroll
+        for (int d = 1; d < W - 1; ++d)  // the qubits d places after the measured one (d = W - 1: the slot)
+          if ((pmask >> ((q + d) % W)) & 1u) sgn |= 1u << ((k + d - 1) % (W - 1));
+      }
+    }
+    sSt[k] = make_uint2(aux, sgn);
+  }
+  if (tid < W) sPos[tid] = (int8_t)((M + (tid + W - M % W) % W + W - 2) % (W - 1));
+}
+
+// Outputs of one 2x2 block from its entries x_ab (a: row half, b: column
+// half); hA, hB, hR, hI: the functional with the step's scale folded in.
+__device__ __forceinline__ void fact_combine(float hA, float hB, float hR, float hI, bool pdead, bool mq, float2 x00,
+                                             float2 x01, float2 x10, float2 x11, uint32_t pr, uint32_t pc,
+                                             float2 &o00, float2 &o01, float2 &o10, float2 &o11) {
+  // sA = G00 x00 + G11 x11, dA = G00 x00 - G11 x11 (a == b terms)
+  const float px = hA * x00.x, py = hA * x00.y;
+  const float2 sA = make_float2(fmaf(hB, x11.x, px), fmaf(hB, x11.y, py));
+  // sB = G01 x01 + conj(G01) x10 (a != b terms), dB = conj(G01) x10 - G01 x01
+  const float2 u = make_float2(x01.x + x10.x, x01.y + x10.y), v = make_float2(x01.x - x10.x, x01.y - x10.y);
+  const float2 sB = make_float2(fmaf(hR, u.x, -hI * v.y), fmaf(hR, u.y, hI * v.x));
+  o00 = make_float2(sA.x + sB.x, sA.y + sB.y);
+  if (pdead) {
+    o01 = o10 = o11 = make_float2(0.f, 0.f);
+  } else if (!mq) {
+    o01 = flip_sign(o00, pc);
+    o10 = flip_sign(o00, pr);
+    o11 = flip_sign(o00, pr ^ pc);
+  } else {
+    // signs (-1)^{a' a + b' b} on the terms: T01 = dA + dB, T10 = dA - dB, T11 = sA - sB
+    const float2 dA = make_float2(fmaf(-hB, x11.x, px), fmaf(-hB, x11.y, py));
+    const float2 dB = make_float2(fmaf(hI, u.y, -hR * v.x), fmaf(-hI, u.x, -hR * v.y));
+    o01 = flip_sign(make_float2(dA.x + dB.x, dA.y + dB.y), pc);
+    o10 = flip_sign(make_float2(dA.x - dB.x, dA.y - dB.y), pr);
+    o11 = flip_sign(make_float2(sA.x - sB.x, sA.y - sB.y), pr ^ pc);
+  }
+}
+
 // One run of the factored sweep by a group of TPR threads.  ``base`` is the
 // group's slice of shared memory; every thread of the group calls this with
 // the same slot.
 template <int W, int TPR>
 __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int tid, int group,
-                                            unsigned char *base, float2 *R_ws = nullptr) {
+                                            unsigned char *base) {
   using Cfg = DmFactCfg<W>;
   constexpr int D = Cfg::D, N = Cfg::N, H = Cfg::H, NB = Cfg::NB, DW = Cfg::DW;
-  float2 *R = Cfg::kSmemR ? reinterpret_cast<float2 *>(base) : R_ws;
-  float2 *psi = reinterpret_cast<float2 *>(base) + (Cfg::kSmemR ? N : 0);
+  float2 *R = reinterpret_cast<float2 *>(base);
+  float2 *psi = R + N;
   float4 *sF = reinterpret_cast<float4 *>(psi + DW);
   uint2 *sSt = reinterpret_cast<uint2 *>(sF + A.maxm);
   float2 *sRed = reinterpret_cast<float2 *>(sSt + A.maxm);  // 2 x 32 entries (one per warp of the group)
@@ -146,38 +203,7 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     sF[k] = make_float4(a_n * 0.5f * (1.f + nz) + b_n, a_n * 0.5f * (1.f - nz) + b_n, a_n * 0.5f * nx,
                         a_n * 0.5f * ny);
   }
-  if (tid == 0) {
-    int8_t pos_of[W];
-    pos_of[0] = -1;  // after step 0 bit 0 is the fresh slot; bit b > 0 is stored at position b - 1
-#pragma unroll
-    for (int b = 1; b < W; ++b) pos_of[b] = (int8_t)(b - 1);
-    int p = 0;
-    uint32_t pmask = steps[0].mask;
-    sSt[0] = make_uint2(steps[0].plane == MBQC_PLANE_Z ? kFactZ : 0u, 0u);
-    for (int k = 1; k < M; ++k) {
-      const int q = k % W;
-      const int pos = pos_of[q];
-      const bool dead = (pmask & kDead) != 0u;
-      uint32_t aux = (uint32_t)pos, sgn = 0u;
-      if (dead) {
-        aux |= kFactDead;
-      } else {
-        if ((pmask >> q) & 1u) aux |= kFactMq;
-#pragma unroll
-        for (int b = 0; b < W; ++b)
-          if (b != p && b != q && ((pmask >> b) & 1u)) sgn |= 1u << pos_of[b];
-      }
-      const DevStep st = steps[k];
-      if (st.plane == MBQC_PLANE_Z) aux |= kFactZ;
-      sSt[k] = make_uint2(aux, sgn);
-      pos_of[p] = (int8_t)pos;
-      pos_of[q] = -1;
-      p = q;
-      pmask = st.mask;
-    }
-#pragma unroll
-    for (int b = 0; b < W; ++b) sPos[b] = pos_of[b];
-  }
+  fact_tables<W>(steps, M, sSt, sPos, tid, TPR);
   // ---- the initial window |psi_0> (input, |+> padding, initial CZ signs)
   {
     const float2 *in = A.psi_in + (A.istride ? run * A.istride : 0);
@@ -294,30 +320,9 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     const uint32_t sgn = ss.y;
     const float half = pdead ? inv : 0.5f * inv;
     const float hA = g00 * half, hB = g11 * half, hR = gr * half, hI = gi * half;
-    // outputs of one block from its entries x_ab (a: row half, b: column half)
     auto combine = [&](float2 x00, float2 x01, float2 x10, float2 x11, uint32_t pr, uint32_t pc, float2 &o00,
                        float2 &o01, float2 &o10, float2 &o11) {
-      // sA = G00 x00 + G11 x11, dA = G00 x00 - G11 x11 (a == b terms)
-      const float px = hA * x00.x, py = hA * x00.y;
-      const float2 sA = make_float2(fmaf(hB, x11.x, px), fmaf(hB, x11.y, py));
-      // sB = G01 x01 + conj(G01) x10 (a != b terms), dB = conj(G01) x10 - G01 x01
-      const float2 u = make_float2(x01.x + x10.x, x01.y + x10.y), v = make_float2(x01.x - x10.x, x01.y - x10.y);
-      const float2 sB = make_float2(fmaf(hR, u.x, -hI * v.y), fmaf(hR, u.y, hI * v.x));
-      o00 = make_float2(sA.x + sB.x, sA.y + sB.y);
-      if (pdead) {
-        o01 = o10 = o11 = make_float2(0.f, 0.f);
-      } else if (!mq) {
-        o01 = flip_sign(o00, pc);
-        o10 = flip_sign(o00, pr);
-        o11 = flip_sign(o00, pr ^ pc);
-      } else {
-        // signs (-1)^{a' a + b' b} on the terms: T01 = dA + dB, T10 = dA - dB, T11 = sA - sB
-        const float2 dA = make_float2(fmaf(-hB, x11.x, px), fmaf(-hB, x11.y, py));
-        const float2 dB = make_float2(fmaf(hI, u.y, -hR * v.x), fmaf(-hI, u.x, -hR * v.y));
-        o01 = flip_sign(make_float2(dA.x + dB.x, dA.y + dB.y), pc);
-        o10 = flip_sign(make_float2(dA.x - dB.x, dA.y - dB.y), pr);
-        o11 = flip_sign(make_float2(sA.x - sB.x, sA.y - sB.y), pr ^ pc);
-      }
+      fact_combine(hA, hB, hR, hI, pdead, mq, x00, x01, x10, x11, pr, pc, o00, o01, o10, o11);
     };
     float4 *R4 = reinterpret_cast<float4 *>(R);
     if (pos == 0) {
@@ -448,14 +453,306 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
   group_sync(TPR, group);  // the slice is reused by the caller's next run
 }
 
-// Windows 9..11: one 1024-thread block per run, R in the workspace (one
-// slice of N complex64 per resident block), blocks looping over the runs.
-template <int W>
-__global__ void __launch_bounds__(1024) dm_fwd_fact_ws(DmArgs A, float2 *ws) {
+// Windows 9..11: R (512 KB to 8 MB) in the workspace, one slice per cluster of
+// CS blocks; the cluster takes a run at a time.  Every block reads the step's
+// diagonal and sums the probability itself (no exchange), the 2x2 blocks of
+// the pass are dealt over all CS x 512 threads, and a cluster barrier ends the
+// step.  In place: a block arrives at a second barrier once it has read the
+// diagonal and waits there only before its first store, so the reduction
+// overlaps it.  What bounds it is the L2: a step moves the slice in and out
+// once.  One 1024-thread block a run left the rest of the GPU idle and ran at
+// what one SM draws from L2: 24 runs of an 8 x 6 grid (window 9) took
+// 711 us, XXX us with eight blocks a run.
+constexpr int kFactWsThreads = 512;
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Sum of the hi + lo pairs of the block's threads, the same bits in each
+// (two-sum at every addition); scratch double-buffered as in group_sum2_db.
+__device__ __forceinline__ float2 block_pair_sum(float hi, float lo, float2 *scratch, int &par) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+    const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+    two_sum_acc(hi, lo, oh, ol);
+  }
+  float2 *buf = scratch + par * 32;
+  par ^= 1;
+  if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = make_float2(hi, lo);
+  __syncthreads();
+  constexpr int NW = kFactWsThreads / 32;
+  const float2 w = buf[threadIdx.x & (NW - 1)];
+  hi = w.x;
+  lo = w.y;
+#pragma unroll
+  for (int o = NW / 2; o >= 1; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+    const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+    two_sum_acc(hi, lo, oh, ol);
+  }
+  const float s = hi + lo;  // renormalise
+  return make_float2(s, lo - (s - hi));
+}
+
+template <int W, int CS>
+__global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, float2 *ws) {
+  using Cfg = DmFactCfg<W>;
+  constexpr int D = Cfg::D, H = Cfg::H, NB = Cfg::NB, DW = Cfg::DW, BT = kFactWsThreads, TT = BT * CS;
   extern __shared__ __align__(16) unsigned char smem_w[];
-  float2 *R = ws + (size_t)blockIdx.x * DmFactCfg<W>::N;
-  for (int64_t slot = blockIdx.x; slot < A.B; slot += gridDim.x)
-    dm_fact_run<W, 1024>(A, slot, threadIdx.x, 0, smem_w, R);
+  float2 *psi = reinterpret_cast<float2 *>(smem_w);
+  float4 *sF = reinterpret_cast<float4 *>(psi + DW);
+  uint2 *sSt = reinterpret_cast<uint2 *>(sF + A.maxm);
+  float2 *sRed = reinterpret_cast<float2 *>(sSt + A.maxm);  // 2 x 32 entries
+  int8_t *sPos = reinterpret_cast<int8_t *>(sRed + 64);
+  const int tid = threadIdx.x;
+  const int crank = (int)cooperative_groups::this_cluster().block_rank();
+  const int g = crank * BT + tid;  // thread of the cluster
+  float2 *R = ws + (size_t)(blockIdx.x / CS) * Cfg::N;
+  float4 *R4 = reinterpret_cast<float4 *>(R);
+  const float qn = f64_to_f32_rn(A.noise);
+  const float a_n = 1.f - (4.f / 3.f) * qn, b_n = (2.f / 3.f) * qn;
+  const float tr_noise = a_n + 2.f * b_n;
+  int par = 0;
+
+  // every block of a cluster runs the same loops: each barrier is reached by all
+  for (int64_t slot = blockIdx.x / CS; slot < A.B; slot += gridDim.x / CS) {
+    const int ci = A.run_circuit ? A.run_circuit[slot] : 0;
+    const int64_t run = A.run_circuit ? (int64_t)ci : slot;
+    const DevCircuit &C = A.circ[ci];
+    const int M = C.n_steps;
+    const DevStep *steps = A.steps + C.step_off;
+    if (C.w != W || M > A.maxm || M < 1 || C.map_off < 0 || !(steps[M - 1].mask & kDead)) {
+      if (g == 0 && A.status) A.status[run] = MBQC_RUN_NAN;  // the host routes such plans elsewhere
+      continue;
+    }
+    const int2 *map = A.maps + C.map_off;
+    const double *ang = A.angles + run * A.astride;
+    for (int k = tid; k < M; k += BT) {
+      const DevStep st = steps[k];
+      const double th = st.aidx >= 0 ? ang[st.aidx] : st.fixed;
+      float nx, ny, nz;
+      bloch(st.plane, th, nx, ny, nz);
+      sF[k] = make_float4(a_n * 0.5f * (1.f + nz) + b_n, a_n * 0.5f * (1.f - nz) + b_n, a_n * 0.5f * nx,
+                          a_n * 0.5f * ny);
+    }
+    fact_tables<W>(steps, M, sSt, sPos, tid, BT);
+    {
+      const float2 *in = A.psi_in + (A.istride ? run * A.istride : 0);
+      const float pad = exp2f(-0.5f * (float)(W - C.n_in));
+      for (int i = tid; i < DW; i += BT) {
+        const int2 mi = __ldg(&map[i]);
+        const float2 u = flip_sign(in[mi.x & 0x7fffffff], (uint32_t)mi.x & 0x80000000u);
+        psi[i] = make_float2(pad * u.x, pad * u.y);
+      }
+    }
+    __syncthreads();
+
+    int32_t st_code = MBQC_RUN_OK;
+    for (int k = 0; k < M; ++k) {
+      const float4 F = sF[k];
+      const uint2 ss = sSt[k];
+      const bool zstep = (ss.x & kFactZ) != 0u;
+      const int pos = (int)(ss.x & 15u);
+      const bool mq = (ss.x & kFactMq) != 0u, pdead = (ss.x & kFactDead) != 0u;
+      const bool drop_coh = k > 0 && !pdead && mq;
+      // 1. outcome probability (dm_fact_run), term by term in float pairs
+      float p_hi = 0.f, p_lo = 0.f, t_hi = 0.f, t_lo = 0.f, o_hi = 0.f, o_lo = 0.f;
+      const int terms = k == 0 ? D : H;
+      for (int r = tid; r < terms; r += BT) {
+        float v, off = 0.f, tr;
+        if (k == 0) {
+          const float2 u0 = psi[2 * r], u1 = psi[2 * r + 1];
+          const float q00 = u0.x * u0.x + u0.y * u0.y, q11 = u1.x * u1.x + u1.y * u1.y;
+          // x01 = psi0 conj(psi1)
+          off = 2.f * (F.z * (u0.x * u1.x + u0.y * u1.y) - F.w * (u0.y * u1.x - u0.x * u1.y));
+          v = F.x * q00 + F.y * q11;
+          tr = q00 + q11;
+        } else {
+          const uint32_t i0 = ins_bit(r, pos, 0), i1 = ins_bit(r, pos, 1);
+          const float2 q00 = __ldcg(&R[i0 * D + i0]), q11 = __ldcg(&R[i1 * D + i1]);
+          v = F.x * q00.x + F.y * q11.x;
+          if (!drop_coh) {
+            const float2 q01 = __ldcg(&R[i0 * D + i1]);
+            off = 2.f * (F.z * q01.x - F.w * q01.y);
+          }
+          tr = q00.x + q11.x;
+        }
+        two_sum_acc(p_hi, p_lo, drop_coh ? v : v + off, 0.f);
+        two_sum_acc(t_hi, t_lo, tr, 0.f);
+        // prob1 = trace - prob0 term by term
+        two_sum_acc(o_hi, o_lo, drop_coh ? tr_noise * tr - v : tr_noise * tr - v - off, 0.f);
+      }
+      if (k > 0) cluster_arrive();  // this block has read its diagonal
+      float2 prob = block_pair_sum(p_hi, p_lo, sRed, par);
+      float4 G = F;
+      int outcome = 0;
+      bool take1 = false, unprojected = false;
+      if (zstep) {
+        const float2 tot = block_pair_sum(t_hi, t_lo, sRed, par);
+        if (A.flags & MBQC_F_DM_EXPECTATION) {
+          if (g == 0 && A.probs)
+            A.probs[run * A.ostride + k] = 1.0 - ((double)prob.x + (double)prob.y) / ((double)tot.x + (double)tot.y);
+          G = make_float4(1.f, 1.f, 0.f, 0.f);
+          prob = make_float2(1.f, 0.f);
+          outcome = 2;
+          unprojected = true;
+        } else {
+          take1 = !(draw_uniform(A.seed, run, k) * tot.x < prob.x);
+        }
+      } else {
+        take1 = !pair_ge(prob, 1e-4);  // prob0 < 1e-4 (or NaN): outcome 1 (np_simulator_dm.py:335-338)
+      }
+      if (g == 0 && A.probs && !unprojected) A.probs[run * A.ostride + k] = (double)prob.x + (double)prob.y;
+      if (take1) {  // outcome 1 with P1 = I - P0
+        G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
+        prob = block_pair_sum(o_hi, o_lo, sRed, par);
+        outcome = 1;
+      }
+      if (g == 0 && A.outcomes) A.outcomes[run * A.ostride + k] = (int8_t)outcome;
+      const bool bad = !(prob.x > 0.f) || isnan(prob.x) || isinf(prob.x);  // the reference's NaN check
+      if (bad) {  // the same bits, so the same branch, in every thread of the cluster
+        st_code = MBQC_RUN_NAN;
+        if (k > 0) cluster_wait();
+        break;
+      }
+      float inv = __frcp_rn(prob.x);        // correctly rounded 1/hi
+      inv = fmaf(-inv * inv, prob.y, inv);  // 1/(hi + lo) to first order in lo
+      const float g00 = G.x, g11 = G.y, gr = G.z, gi = G.w;
+      if (k == 0) {
+        for (int e = g; e < Cfg::N; e += TT) {
+          const int x = e / D, y = e % D;
+          const float2 u0 = psi[2 * x], u1 = psi[2 * x + 1], v0 = psi[2 * y], v1 = psi[2 * y + 1];
+          // x_ab = psi(x,a) conj(psi(y,b))
+          const float2 x00 = make_float2(u0.x * v0.x + u0.y * v0.y, u0.y * v0.x - u0.x * v0.y);
+          const float2 x11 = make_float2(u1.x * v1.x + u1.y * v1.y, u1.y * v1.x - u1.x * v1.y);
+          const float2 x01 = make_float2(u0.x * v1.x + u0.y * v1.y, u0.y * v1.x - u0.x * v1.y);
+          const float2 x10 = make_float2(u1.x * v0.x + u1.y * v0.y, u1.y * v0.x - u1.x * v0.y);
+          const float sr = g00 * x00.x + g11 * x11.x + gr * (x01.x + x10.x) - gi * (x01.y - x10.y);
+          const float si = g00 * x00.y + g11 * x11.y + gr * (x01.y + x10.y) + gi * (x01.x - x10.x);
+          __stcg(&R[e], make_float2(sr * inv, si * inv));
+        }
+      } else {
+        // 2. one in-place pass over the 2x2 blocks of position pos: at pos 0 a
+        //    block's two columns are one float4 a row, else a unit is the two
+        //    blocks of columns c0, c0 + 1; all loads of U units in flight
+        //    before their stores
+        const uint32_t sgn = ss.y;
+        const float half = pdead ? inv : 0.5f * inv;
+        const float hA = g00 * half, hB = g11 * half, hR = gr * half, hI = gi * half;
+        bool waited = false;
+        if (pos == 0) {
+          constexpr int RSTEP = TT / H, NJ = H / RSTEP, U = NJ >= 4 ? 4 : NJ;
+          static_assert(TT % H == 0 && H % RSTEP == 0 && NJ % U == 0, "rows over the cluster's threads");
+          const uint32_t c = (uint32_t)(g % H), r_first = (uint32_t)(g / H);
+          const uint32_t pc = (__popc((2u * c) & sgn) & 1u) << 31;
+#pragma unroll 1
+          for (int j0 = 0; j0 < NJ; j0 += U) {
+            float4 top[U], bot[U];
+#pragma unroll
+            for (int uu = 0; uu < U; ++uu) {
+              const uint32_t at = (r_first + (uint32_t)(j0 + uu) * RSTEP) * D + c;
+              top[uu] = __ldcg(&R4[at]);
+              bot[uu] = __ldcg(&R4[at + D / 2]);
+            }
+            if (!waited) cluster_wait();
+            waited = true;
+#pragma unroll
+            for (int uu = 0; uu < U; ++uu) {
+              const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP, at = r * D + c;
+              const uint32_t pr = (__popc((2u * r) & sgn) & 1u) << 31;
+              float2 o00, o01, o10, o11;
+              fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(top[uu].x, top[uu].y),
+                           make_float2(top[uu].z, top[uu].w), make_float2(bot[uu].x, bot[uu].y),
+                           make_float2(bot[uu].z, bot[uu].w), pr, pc, o00, o01, o10, o11);
+              __stcg(&R4[at], make_float4(o00.x, o00.y, o01.x, o01.y));
+              __stcg(&R4[at + D / 2], make_float4(o10.x, o10.y, o11.x, o11.y));
+            }
+          }
+        } else {
+          constexpr int HU = H / 2, RSTEP = TT / HU, NJ = H > RSTEP ? H / RSTEP : 1, U = NJ >= 2 ? 2 : NJ;
+          static_assert(TT % HU == 0 && RSTEP <= H && H % RSTEP == 0 && NJ % U == 0, "rows over the cluster's threads");
+          const uint32_t rs = ((uint32_t)D << pos) >> 1;  // row step in float4
+          const uint32_t r_first = (uint32_t)(g / HU);
+          const uint32_t c0 = ins_bit(2u * (uint32_t)(g % HU), pos, 0);  // even
+          const uint32_t pc0 = (__popc(c0 & sgn) & 1u) << 31, pc1 = (__popc((c0 + 1u) & sgn) & 1u) << 31;
+          const uint32_t s0 = c0 >> 1, s1 = (c0 | (1u << pos)) >> 1;
+#pragma unroll 1
+          for (int j0 = 0; j0 < NJ; j0 += U) {
+            float4 q00[U], q01[U], q10[U], q11[U];
+            uint32_t at[U], pr[U];
+#pragma unroll
+            for (int uu = 0; uu < U; ++uu) {
+              const uint32_t r0 = ins_bit(r_first + (uint32_t)(j0 + uu) * RSTEP, pos, 0);
+              at[uu] = (r0 * D) >> 1;
+              pr[uu] = (__popc(r0 & sgn) & 1u) << 31;
+              q00[uu] = __ldcg(&R4[at[uu] + s0]);
+              q01[uu] = __ldcg(&R4[at[uu] + s1]);
+              q10[uu] = __ldcg(&R4[at[uu] + rs + s0]);
+              q11[uu] = __ldcg(&R4[at[uu] + rs + s1]);
+            }
+            if (!waited) cluster_wait();
+            waited = true;
+#pragma unroll
+            for (int uu = 0; uu < U; ++uu) {
+              float2 a00, a01, a10, a11, b00, b01, b10, b11;
+              fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(q00[uu].x, q00[uu].y),
+                           make_float2(q01[uu].x, q01[uu].y), make_float2(q10[uu].x, q10[uu].y),
+                           make_float2(q11[uu].x, q11[uu].y), pr[uu], pc0, a00, a01, a10, a11);
+              fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(q00[uu].z, q00[uu].w),
+                           make_float2(q01[uu].z, q01[uu].w), make_float2(q10[uu].z, q10[uu].w),
+                           make_float2(q11[uu].z, q11[uu].w), pr[uu], pc1, b00, b01, b10, b11);
+              __stcg(&R4[at[uu] + s0], make_float4(a00.x, a00.y, b00.x, b00.y));
+              __stcg(&R4[at[uu] + s1], make_float4(a01.x, a01.y, b01.x, b01.y));
+              __stcg(&R4[at[uu] + rs + s0], make_float4(a10.x, a10.y, b10.x, b10.y));
+              __stcg(&R4[at[uu] + rs + s1], make_float4(a11.x, a11.y, b11.x, b11.y));
+            }
+          }
+        }
+      }
+      cluster_arrive();
+      cluster_wait();
+    }
+
+    // ---- output noise, one output qubit a pass
+    if (st_code == MBQC_RUN_OK && qn != 0.f) {
+      for (int j = 0; j < C.n_out; ++j) {
+        const int pos = sPos[C.out_bits[j]];
+        for (int e = g; e < NB; e += TT) {
+          const uint32_t r = (uint32_t)e / H, c = (uint32_t)e % H;
+          const uint32_t r0 = ins_bit(r, pos, 0) * D, r1 = ins_bit(r, pos, 1) * D;
+          const uint32_t c0 = ins_bit(c, pos, 0), c1 = ins_bit(c, pos, 1);
+          const float2 x00 = __ldcg(&R[r0 + c0]), x01 = __ldcg(&R[r0 + c1]);
+          const float2 x10 = __ldcg(&R[r1 + c0]), x11 = __ldcg(&R[r1 + c1]);
+          const float2 tr = make_float2(x00.x + x11.x, x00.y + x11.y);
+          __stcg(&R[r0 + c0], make_float2(a_n * x00.x + b_n * tr.x, a_n * x00.y + b_n * tr.y));
+          __stcg(&R[r1 + c1], make_float2(a_n * x11.x + b_n * tr.x, a_n * x11.y + b_n * tr.y));
+          __stcg(&R[r0 + c1], make_float2(a_n * x01.x, a_n * x01.y));
+          __stcg(&R[r1 + c0], make_float2(a_n * x10.x, a_n * x10.y));
+        }
+        cluster_arrive();
+        cluster_wait();
+      }
+    }
+    // ---- gather the outputs in the reference order
+    const int n_out = C.n_out, dout = 1 << n_out;
+    int *ridx = reinterpret_cast<int *>(psi);  // psi is no longer needed
+    __syncthreads();
+    for (int y = tid; y < dout; y += BT) {
+      int ri = 0;
+      for (int j = 0; j < n_out; ++j) ri |= ((y >> (n_out - 1 - j)) & 1) << sPos[C.out_bits[j]];
+      ridx[y] = ri;
+    }
+    __syncthreads();
+    float2 *out = A.rho_out + run * A.out_stride;
+    for (int e = g; e < dout * dout; e += TT) {
+      const int yi = e >> n_out, yj = e & (dout - 1);
+      out[e] = st_code == MBQC_RUN_OK ? __ldcg(&R[ridx[yi] * D + ridx[yj]]) : make_float2(NAN, NAN);
+    }
+    if (g == 0 && A.status) A.status[run] = st_code;
+    cluster_arrive();  // the slice and the tables are reused by the cluster's next run
+    cluster_wait();
+  }
 }
 
 // One run per group of TPR threads, 256 / TPR runs per block.
