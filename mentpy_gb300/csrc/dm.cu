@@ -72,6 +72,50 @@ static int launch_dm_fact_cluster(const DmArgs &a, int64_t slots, float2 *ws, cu
   return rc ? rc : check_launch("dm_fwd_fact_ws");
 }
 
+// Windows 9 and 10: the matrix in the cluster's shared memory (dm_fwd_fact_cl)
+// wherever its rows and the step tables fit one block.  Window 10 takes
+// clusters of sixteen blocks, of which the GPU holds few: a batch they cannot
+// all hold at once goes through the workspace (36 steps: 8 runs 472 us in two
+// waves of clusters, 424 us in the workspace; 4 runs 189 and 424 us).
+template <int W>
+static int launch_dm_fact_smem_cluster(const DmArgs &a, int64_t batch, cudaStream_t s, bool &placed) {
+  using Cfg = DmClCfg<W>;
+  const size_t smem = dm_cl_bytes<W>(a.maxm);
+  placed = false;
+  if (smem > (size_t)227 * 1024) return MBQC_OK;
+  auto k = dm_fwd_fact_cl<W>;
+  int rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                      "dm smem attribute");
+  if (rc) return rc;
+  if (Cfg::CS > 8) {
+    rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "dm cluster attribute");
+    if (rc) return rc;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(std::min<int64_t>(batch, 4 * (int64_t)sm_count()) * Cfg::CS));
+  cfg.blockDim = dim3(Cfg::BT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = Cfg::CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (Cfg::CS > 8) {  // sixteen SMs of one GPC: a few clusters at a time
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return MBQC_OK;
+    }
+    if (batch > n) return MBQC_OK;
+  }
+  placed = true;
+  rc = cuda_check(cudaLaunchKernelEx(&cfg, k, a), "dm_fwd_fact_cl cluster launch");
+  return rc ? rc : check_launch("dm_fwd_fact_cl");
+}
+
 // Blocks per run: as many as keep all runs resident at two 512-thread blocks
 // an SM, eight (the portable cluster size) at most and two at least.
 template <int W>
@@ -80,6 +124,11 @@ static int launch_dm_fact_ws(const DmArgs &a, int64_t batch, void *ws, size_t ws
   const int64_t slots = std::min<int64_t>(dm_ws_slots(batch), (int64_t)(ws_bytes / per));
   if (!ws || slots < 1)
     return fail(MBQC_E_INVALID, "dm_forward: window %d needs a workspace of at least %zu bytes", W, per);
+  if constexpr (W <= 10) {
+    bool placed;
+    const int rc = launch_dm_fact_smem_cluster<W>(a, batch, s, placed);
+    if (rc || placed) return rc;
+  }
   float2 *w = static_cast<float2 *>(ws);
   const int64_t room = 2 * (int64_t)sm_count();
   if (slots * 8 <= room) return launch_dm_fact_cluster<W, 8>(a, slots, w, s);

@@ -141,12 +141,24 @@ __device__ __forceinline__ float2 group_sum2(float v, float2 *scratch, int tid, 
   return make_float2(s, lo - (s - hi));
 }
 
-// hi + lo >= t for a pair from group_sum2: decided in float unless hi is
-// within 1e-6 (relative) of t, where the pair is compared in FP64
+// hi + lo >= t for a pair from group_sum2: decided by hi unless it is within
+// 1e-6 (relative) of t, where hi - tf is exact and the remainders decide.  All
+// in float: as an FP64 comparison on that branch the compiler ran it on every
+// thread at every step (two conversions, an add and a compare on a pipe of
+// 1/64 the FP32 rate: ~1,400 cycles a step with 16 warps on an SM).
 __device__ __forceinline__ bool pair_ge(float2 p, double t) {
-  const float tf = (float)t;
-  if (fabsf(p.x - tf) > 1e-6f * tf) return p.x > tf;
-  return (double)p.x + (double)p.y >= t;
+  const float tf = (float)t, tl = (float)(t - (double)tf);
+  const float d = p.x - tf;
+  if (fabsf(d) > 1e-6f * tf) return d > 0.f;
+  return d + (p.y - tl) >= 0.f;  // NaN: false
+}
+
+// A step's recorded probability: prob0 (hi, lo), or for an expectation-mode Z
+// step 1 - prob0 / trace from (prob0, trace).  Kept in the step's functional
+// slot until the run ends, so that the FP64 conversion is off the steps' chain.
+__device__ __forceinline__ double prob_record(float4 v) {
+  const double p = (double)v.x + (double)v.y;
+  return v.z != 0.f ? 1.0 - p / ((double)v.z + (double)v.w) : p;
 }
 
 __device__ __forceinline__ uint32_t ins_bit(uint32_t r, int p, uint32_t b) {

@@ -217,6 +217,7 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
   group_sync(TPR, group);
 
   int32_t st_code = MBQC_RUN_OK;
+  int n_rec = 0;                           // steps with a recorded probability
   const float tr_noise = a_n + 2.f * b_n;  // functional of I after noise folding
   for (int k = 0; k < M; ++k) {
     const float4 F = sF[k];
@@ -256,8 +257,7 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     if (zstep) {
       const float2 tot = group_sum2_db<TPR>(t_re, sRed, tid, group, red_par);
       if (A.flags & MBQC_F_DM_EXPECTATION) {
-        if (tid == 0 && A.probs)
-          A.probs[run * A.ostride + k] = 1.0 - ((double)prob.x + (double)prob.y) / ((double)tot.x + (double)tot.y);
+        if (tid == 0) sF[k] = make_float4(prob.x, prob.y, tot.x, tot.y);
         G = make_float4(1.f, 1.f, 0.f, 0.f);
         prob = make_float2(1.f, 0.f);
         outcome = 2;
@@ -273,12 +273,13 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
       // prob1 = trace - prob0 term by term: the same sums with G
       const float p1 = drop_coh ? (tr_noise * t_re - p_re) : (tr_noise * t_re - p_re - p_off);
       const float2 prob1 = group_sum2_db<TPR>(p1, sRed, tid, group, red_par);
-      if (tid == 0 && A.probs) A.probs[run * A.ostride + k] = (double)prob.x + (double)prob.y;
+      if (tid == 0) sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
       prob = prob1;
       outcome = 1;
-    } else if (tid == 0 && A.probs && !unprojected) {
-      A.probs[run * A.ostride + k] = (double)prob.x + (double)prob.y;
+    } else if (tid == 0 && !unprojected) {
+      sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
     }
+    n_rec = k + 1;
     if (tid == 0 && A.outcomes) A.outcomes[run * A.ostride + k] = (int8_t)outcome;
     if (!(prob.x > 0.f) || isnan(prob.x) || isinf(prob.x)) {  // the reference's NaN check
       st_code = MBQC_RUN_NAN;
@@ -444,6 +445,8 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     ridx[y] = ri;
   }
   group_sync(TPR, group);
+  if (A.probs)
+    for (int k = tid; k < n_rec; k += TPR) A.probs[run * A.ostride + k] = prob_record(sF[k]);
   float2 *out = A.rho_out + run * A.out_stride;
   for (int e = tid; e < dout * dout; e += TPR) {
     const int yi = e >> n_out, yj = e & (dout - 1);
@@ -451,6 +454,379 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
   }
   if (tid == 0 && A.status) A.status[run] = st_code;
   group_sync(TPR, group);  // the slice is reused by the caller's next run
+}
+
+// Windows 9 and 10 with R in the shared memory of a cluster: CS blocks of one
+// run hold D / CS = 32 rows each (64 KB at window 9, eight blocks; 128 KB at
+// window 10, sixteen).  Two row layouts: A deals the rows by their top
+// position bits, so positions 0..4 pair rows of one block; B by their lowest
+// bits, so positions 5.. do.  Steps meet the positions cyclically, so a run
+// stays in a layout for 5 steps, then for n - 5: the last step before a change
+// writes its rows straight to their new owners (distributed shared memory).
+// A step is then: one warp sums the block's diagonal pairs and sends the
+// partial to every block, one cluster barrier, the pass over the block's rows.
+// What bounds it is that chain (cycles a step at window 9: ~1,300 to the
+// barrier's end, 250 the sum, 970 the pass, 1,400 the layout changes' share);
+// the workspace kernel below pays two round trips to the L2 and the slice's
+// traffic through it at every step.  Window 9, 40 steps: 228 us for 1 to 8
+// runs and 325 us for 24 there, 117 and 183 us here; window 10, 36 steps, 4
+// runs: 424 and 189 us.
+template <int W> struct DmClCfg {
+  static constexpr int N = W - 1, LB = 5, OB = N - LB, CS = 1 << OB;  // positions, local and owner row bits
+  static constexpr int D = 1 << N, H = D / 2, RL = 1 << LB;
+  static constexpr int BT = D * RL / 16;  // 16 entries a thread
+  static constexpr int DW = 1 << W;
+};
+
+template <int W> __host__ __device__ constexpr size_t dm_cl_bytes(int maxm) {
+  return (size_t)DmClCfg<W>::D * DmClCfg<W>::RL * 8 + (size_t)DmClCfg<W>::DW * 8 + (size_t)maxm * 24 +
+         2 * 16 * sizeof(float2) + 32;
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <int W>
+__global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_fact_cl(DmArgs A) {
+  namespace cg = cooperative_groups;
+  using Cfg = DmClCfg<W>;
+  constexpr int N = Cfg::N, LB = Cfg::LB, OB = Cfg::OB, CS = Cfg::CS, D = Cfg::D, H = Cfg::H, RL = Cfg::RL,
+                BT = Cfg::BT, DW = Cfg::DW, HU = H / 2;
+  extern __shared__ __align__(16) unsigned char smem_c[];
+  float2 *R = reinterpret_cast<float2 *>(smem_c);
+  float4 *R4 = reinterpret_cast<float4 *>(smem_c);
+  float2 *psi = R + (size_t)D * RL;
+  // step k's functional is sF[k]; its probability is recorded in sF[k - 1],
+  // which every thread has read by then (sF[k] is still being read)
+  float4 *sF = reinterpret_cast<float4 *>(psi + DW) + 1;
+  uint2 *sSt = reinterpret_cast<uint2 *>(sF + A.maxm);
+  float2 *sP = reinterpret_cast<float2 *>(sSt + A.maxm);  // two buffers of a partial per block
+  int8_t *sPos = reinterpret_cast<int8_t *>(sP + 32);
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cl.block_rank();
+  const float qn = f64_to_f32_rn(A.noise);
+  const float a_n = 1.f - (4.f / 3.f) * qn, b_n = (2.f / 3.f) * qn, tr_noise = a_n + 2.f * b_n;
+  int par = 0;
+
+  // row of the matrix that local row l is in layout A / B
+  auto row_of = [&](bool b, uint32_t l) { return b ? (l << OB) | (uint32_t)rank : ((uint32_t)rank << LB) | l; };
+  // the block's partial (warp 0, 16 lanes; float pairs) sent to every block
+  auto send = [&](float2 v) {
+    float hi = v.x, lo = v.y;
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+      const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+      two_sum_acc(hi, lo, oh, ol);
+    }
+    if (tid < CS) *cl.map_shared_rank(sP + par * 16 + rank, tid) = make_float2(hi, lo);
+  };
+  auto collect = [&]() {  // after the cluster barrier: the same bits in every thread
+    const float2 w = sP[par * 16 + (tid & (CS - 1))];
+    par ^= 1;
+    float hi = w.x, lo = w.y;
+#pragma unroll
+    for (int o = CS / 2; o >= 1; o >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+      const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+      two_sum_acc(hi, lo, oh, ol);
+    }
+    const float s = hi + lo;  // renormalise
+    return make_float2(s, lo - (s - hi));
+  };
+
+  cluster_arrive();  // every block of the cluster runs before any writes to another
+  cluster_wait();
+  // every block of a cluster runs the same loops: each barrier is reached by all
+  for (int64_t slot = blockIdx.x / CS; slot < A.B; slot += gridDim.x / CS) {
+    const int ci = A.run_circuit ? A.run_circuit[slot] : 0;
+    const int64_t run = A.run_circuit ? (int64_t)ci : slot;
+    const DevCircuit &C = A.circ[ci];
+    const int M = C.n_steps;
+    const DevStep *steps = A.steps + C.step_off;
+    if (C.w != W || M > A.maxm || M < 1 || C.map_off < 0 || !(steps[M - 1].mask & kDead)) {
+      if (tid == 0 && rank == 0 && A.status) A.status[run] = MBQC_RUN_NAN;  // the host routes such plans elsewhere
+      continue;
+    }
+    const int2 *map = A.maps + C.map_off;
+    const double *ang = A.angles + run * A.astride;
+    for (int k = tid; k < M; k += BT) {
+      const DevStep st = steps[k];
+      const double th = st.aidx >= 0 ? ang[st.aidx] : st.fixed;
+      float nx, ny, nz;
+      bloch(st.plane, th, nx, ny, nz);
+      sF[k] = make_float4(a_n * 0.5f * (1.f + nz) + b_n, a_n * 0.5f * (1.f - nz) + b_n, a_n * 0.5f * nx,
+                          a_n * 0.5f * ny);
+    }
+    fact_tables<W>(steps, M, sSt, sPos, tid, BT);
+    {
+      const float2 *in = A.psi_in + (A.istride ? run * A.istride : 0);
+      const float pad = exp2f(-0.5f * (float)(W - C.n_in));
+      for (int i = tid; i < DW; i += BT) {
+        const int2 mi = __ldg(&map[i]);
+        const float2 u = flip_sign(in[mi.x & 0x7fffffff], (uint32_t)mi.x & 0x80000000u);
+        psi[i] = make_float2(pad * u.x, pad * u.y);
+      }
+    }
+    __syncthreads();
+
+    int32_t st_code = MBQC_RUN_OK;
+    int n_rec = 0;    // steps with a recorded probability
+    bool lb = false;  // the rows' layout: A, or B
+    for (int k = 0; k < M; ++k) {
+      // Outcome probability (what = 0), trace (1) or prob1 (2) of the step
+      // (dm_fact_run): step 0 from the initial window, later from the block's
+      // sixteen diagonal pairs.  Made again where a step needs the trace or
+      // prob1: few do, and nothing of it stays live over the barrier (a spilled
+      // register is an L2 round trip there, the barrier drops the L1).
+      auto partial = [&](int what) {
+        const float4 F = sF[k];
+        const uint2 ss = sSt[k];
+        const int pos = (int)(ss.x & 15u), lp = pos - (lb ? OB : 0);
+        const bool drop_coh = k > 0 && (ss.x & kFactDead) == 0u && (ss.x & kFactMq) != 0u;
+        float2 sum = make_float2(0.f, 0.f);
+        auto add = [&](float v, float off, float tr) {
+          float p;
+          if (what == 0)
+            p = drop_coh ? v : v + off;
+          else if (what == 1)
+            p = tr;
+          else  // prob1 = trace - prob0 term by term
+            p = drop_coh ? tr_noise * tr - v : tr_noise * tr - v - off;
+          two_sum_acc(sum.x, sum.y, p, 0.f);
+        };
+        if (k == 0) {
+          for (int r = rank * 16 + (tid & 15); r < D; r += CS * 16) {
+            const float2 u0 = psi[2 * r], u1 = psi[2 * r + 1];
+            const float q00 = u0.x * u0.x + u0.y * u0.y, q11 = u1.x * u1.x + u1.y * u1.y;
+            // x01 = psi0 conj(psi1)
+            add(F.x * q00 + F.y * q11,
+                2.f * (F.z * (u0.x * u1.x + u0.y * u1.y) - F.w * (u0.y * u1.x - u0.x * u1.y)), q00 + q11);
+          }
+        } else {
+          const uint32_t l0 = ins_bit(tid & 15, lp, 0), l1 = l0 | (1u << lp);
+          const uint32_t i0 = row_of(lb, l0), i1 = row_of(lb, l1);
+          const float2 q00 = R[l0 * D + rsw(i0)], q11 = R[l1 * D + rsw(i1)], q01 = R[l0 * D + rsw(i1)];
+          add(F.x * q00.x + F.y * q11.x, 2.f * (F.z * q01.x - F.w * q01.y), q00.x + q11.x);
+        }
+        return sum;
+      };
+      // the sum over the cluster; only warp 0 has something to publish
+      auto exchange = [&](int what) {
+        if (tid < 32) {
+          send(partial(what));
+          cluster_arrive();
+        } else {
+          cluster_arrive_relaxed();
+        }
+        cluster_wait();
+        return collect();
+      };
+      float2 prob = exchange(0);
+      const float4 F = sF[k];
+      const uint2 ss = sSt[k];
+      const bool zstep = (ss.x & kFactZ) != 0u;
+      const int pos = (int)(ss.x & 15u), lp = pos - (lb ? OB : 0);  // position, local row bit
+      const bool mq = (ss.x & kFactMq) != 0u, pdead = (ss.x & kFactDead) != 0u;
+      float4 G = F;
+      int outcome = 0;
+      bool take1 = false, unprojected = false;
+      const bool writer = tid == 0 && rank == 0;
+      if (zstep) {
+        const float2 tot = exchange(1);
+        if (A.flags & MBQC_F_DM_EXPECTATION) {
+          if (tid == 0) sF[k - 1] = make_float4(prob.x, prob.y, tot.x, tot.y);
+          G = make_float4(1.f, 1.f, 0.f, 0.f);
+          prob = make_float2(1.f, 0.f);
+          outcome = 2;
+          unprojected = true;
+        } else {
+          take1 = !(draw_uniform(A.seed, run, k) * tot.x < prob.x);
+        }
+      } else {
+        take1 = !pair_ge(prob, 1e-4);  // prob0 < 1e-4 (or NaN): outcome 1 (np_simulator_dm.py:335-338)
+      }
+      if (tid == 0 && !unprojected) sF[k - 1] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      n_rec = k + 1;
+      if (take1) {  // outcome 1 with P1 = I - P0
+        G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
+        prob = exchange(2);
+        outcome = 1;
+      }
+      if (writer && A.outcomes) A.outcomes[run * A.ostride + k] = (int8_t)outcome;
+      if (!(prob.x > 0.f) || isnan(prob.x) || isinf(prob.x)) {  // the reference's NaN check
+        st_code = MBQC_RUN_NAN;  // the same bits, so the same branch, in every thread of the cluster
+        break;
+      }
+      float inv = __frcp_rn(prob.x);        // correctly rounded 1/hi
+      inv = fmaf(-inv * inv, prob.y, inv);  // 1/(hi + lo) to first order in lo
+      const float g00 = G.x, g11 = G.y, gr = G.z, gi = G.w;
+      if (k == 0) {
+        for (int e = tid; e < D * RL; e += BT) {
+          const int l = e / D, y = e % D, xr = (int)row_of(false, (uint32_t)l);
+          const float2 u0 = psi[2 * xr], u1 = psi[2 * xr + 1], v0 = psi[2 * y], v1 = psi[2 * y + 1];
+          // x_ab = psi(x,a) conj(psi(y,b))
+          const float2 x00 = make_float2(u0.x * v0.x + u0.y * v0.y, u0.y * v0.x - u0.x * v0.y);
+          const float2 x11 = make_float2(u1.x * v1.x + u1.y * v1.y, u1.y * v1.x - u1.x * v1.y);
+          const float2 x01 = make_float2(u0.x * v1.x + u0.y * v1.y, u0.y * v1.x - u0.x * v1.y);
+          const float2 x10 = make_float2(u1.x * v0.x + u1.y * v0.y, u1.y * v0.x - u1.x * v0.y);
+          const float sr = g00 * x00.x + g11 * x11.x + gr * (x01.x + x10.x) - gi * (x01.y - x10.y);
+          const float si = g00 * x00.y + g11 * x11.y + gr * (x01.y + x10.y) + gi * (x01.x - x10.x);
+          R[l * D + rsw((uint32_t)y)] = make_float2(sr * inv, si * inv);
+        }
+        __syncthreads();
+        continue;
+      }
+      // 2. the pass.  The last step of a layout stores to the rows' new owners,
+      //    once every block has loaded its own
+      const uint32_t sgn = ss.y, rs = ((uint32_t)D << lp) >> 1;  // row step in float4
+      const float half = pdead ? inv : 0.5f * inv;
+      const float hA = g00 * half, hB = g11 * half, hR = gr * half, hI = gi * half;
+      if (pos == 0) {
+        const uint32_t pc = (__popc((2u * (uint32_t)(tid % H)) & sgn) & 1u) << 31;
+        const uint32_t s0 = rsw(2u * (uint32_t)(tid % H)) >> 1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t l = ins_bit((uint32_t)(tid / H + 4 * u), 0, 0), at = ((l * D) >> 1) + s0;
+          const uint32_t pr = (__popc(row_of(lb, l) & sgn) & 1u) << 31;
+          const float4 top = R4[at], bot = R4[at + rs];
+          float2 o00, o01, o10, o11;
+          fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(top.x, top.y), make_float2(top.z, top.w),
+                       make_float2(bot.x, bot.y), make_float2(bot.z, bot.w), pr, pc, o00, o01, o10, o11);
+          R4[at] = make_float4(o00.x, o00.y, o01.x, o01.y);
+          R4[at + rs] = make_float4(o10.x, o10.y, o11.x, o11.y);
+        }
+        __syncthreads();
+        continue;
+      }
+      const uint32_t c0 = ins_bit(2u * (uint32_t)(tid % HU), pos, 0);  // even
+      const uint32_t pc0 = (__popc(c0 & sgn) & 1u) << 31, pc1 = (__popc((c0 + 1u) & sgn) & 1u) << 31;
+      const uint32_t s0 = rsw(c0) >> 1, s1 = rsw(c0 | (1u << pos)) >> 1;
+      // the unit of rows l, l + 2^lp: its outputs in place of its inputs
+      auto unit = [&](uint32_t l, float4 (&x)[4]) {
+        const uint32_t at = (l * D) >> 1;
+        x[0] = R4[at + s0];
+        x[1] = R4[at + s1];
+        x[2] = R4[at + rs + s0];
+        x[3] = R4[at + rs + s1];
+        const uint32_t pr = (__popc(row_of(lb, l) & sgn) & 1u) << 31;
+        float2 a00, a01, a10, a11, b00, b01, b10, b11;
+        fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(x[0].x, x[0].y), make_float2(x[1].x, x[1].y),
+                     make_float2(x[2].x, x[2].y), make_float2(x[3].x, x[3].y), pr, pc0, a00, a01, a10, a11);
+        fact_combine(hA, hB, hR, hI, pdead, mq, make_float2(x[0].z, x[0].w), make_float2(x[1].z, x[1].w),
+                     make_float2(x[2].z, x[2].w), make_float2(x[3].z, x[3].w), pr, pc1, b00, b01, b10, b11);
+        x[0] = make_float4(a00.x, a00.y, b00.x, b00.y);
+        x[1] = make_float4(a01.x, a01.y, b01.x, b01.y);
+        x[2] = make_float4(a10.x, a10.y, b10.x, b10.y);
+        x[3] = make_float4(a11.x, a11.y, b11.x, b11.y);
+      };
+      const uint32_t l0 = ins_bit((uint32_t)(tid / HU), lp, 0), l1 = ins_bit((uint32_t)(tid / HU + 8), lp, 0);
+      if (k + 1 == M || pos != (lb ? N - 1 : LB - 1)) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t l = u ? l1 : l0, at = (l * D) >> 1;
+          float4 x[4];
+          unit(l, x);
+          R4[at + s0] = x[0];
+          R4[at + s1] = x[1];
+          R4[at + rs + s0] = x[2];
+          R4[at + rs + s1] = x[3];
+        }
+        __syncthreads();
+      } else {
+        float4 x[4], y[4];
+        unit(l0, x);
+        unit(l1, y);
+        cluster_arrive_relaxed();
+        cluster_wait();
+        auto row_ptr = [&](uint32_t l) {
+          const uint32_t i = row_of(lb, l), owner = lb ? i >> LB : i & (CS - 1), q = lb ? i & (RL - 1) : i >> OB;
+          return cl.map_shared_rank(R4 + q * (D / 2), (int)owner);
+        };
+        float4 *p = row_ptr(l0), *q = row_ptr(l0 | (1u << lp));
+        p[s0] = x[0];
+        p[s1] = x[1];
+        q[s0] = x[2];
+        q[s1] = x[3];
+        p = row_ptr(l1);
+        q = row_ptr(l1 | (1u << lp));
+        p[s0] = y[0];
+        p[s1] = y[1];
+        q[s0] = y[2];
+        q[s1] = y[3];
+        lb = !lb;
+        cluster_arrive();
+        cluster_wait();
+      }
+    }
+
+    // ---- output noise: the positions this layout pairs, then the others
+    const int n_out = C.n_out, dout = 1 << n_out;
+    if (st_code == MBQC_RUN_OK && qn != 0.f) {
+      for (int half = 0; half < 2; ++half) {
+        for (int j = 0; j < n_out; ++j) {
+          const int pos = sPos[C.out_bits[j]], lp = pos - (lb ? OB : 0);
+          // positions both layouts pair are taken in the first one
+          const bool here = lp >= 0 && lp < LB;
+          const int lq = pos - (lb ? 0 : OB);
+          const bool other = lq >= 0 && lq < LB;
+          if (!here || (half == 1 && other)) continue;
+          for (int e = tid; e < RL / 2 * H; e += BT) {
+            const uint32_t l0 = ins_bit((uint32_t)e / H, lp, 0) * D, l1 = l0 + ((uint32_t)D << lp);
+            const uint32_t c = ins_bit((uint32_t)e % H, pos, 0), c0 = rsw(c), c1 = rsw(c | (1u << pos));
+            const float2 x00 = R[l0 + c0], x01 = R[l0 + c1], x10 = R[l1 + c0], x11 = R[l1 + c1];
+            const float2 tr = make_float2(x00.x + x11.x, x00.y + x11.y);
+            R[l0 + c0] = make_float2(a_n * x00.x + b_n * tr.x, a_n * x00.y + b_n * tr.y);
+            R[l1 + c1] = make_float2(a_n * x11.x + b_n * tr.x, a_n * x11.y + b_n * tr.y);
+            R[l0 + c1] = make_float2(a_n * x01.x, a_n * x01.y);
+            R[l1 + c0] = make_float2(a_n * x10.x, a_n * x10.y);
+          }
+          __syncthreads();
+        }
+        if (half == 0) {  // every row to its owner in the other layout
+          float4 x[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) x[u] = R4[tid + u * BT];
+          cluster_arrive();
+          cluster_wait();
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const uint32_t e = (uint32_t)(tid + u * BT), i = row_of(lb, e / (D / 2));
+            const uint32_t owner = lb ? i >> LB : i & (CS - 1), l = lb ? i & (RL - 1) : i >> OB;
+            cl.map_shared_rank(R4, (int)owner)[l * (D / 2) + e % (D / 2)] = x[u];
+          }
+          lb = !lb;
+          cluster_arrive();
+          cluster_wait();
+        }
+      }
+    }
+    // ---- outputs in the reference order: each block writes the rows it holds
+    int *ridx = reinterpret_cast<int *>(psi), *rinv = ridx + D;  // psi is no longer needed
+    __syncthreads();
+    for (int i = tid; i < D; i += BT) rinv[i] = -1;
+    __syncthreads();
+    for (int y = tid; y < dout; y += BT) {
+      int ri = 0;
+      for (int j = 0; j < n_out; ++j) ri |= ((y >> (n_out - 1 - j)) & 1) << sPos[C.out_bits[j]];
+      ridx[y] = ri;
+      rinv[ri] = y;
+    }
+    __syncthreads();
+    if (rank == 0 && A.probs)
+      for (int k = tid; k < n_rec; k += BT) A.probs[run * A.ostride + k] = prob_record(sF[k - 1]);
+    float2 *out = A.rho_out + run * A.out_stride;
+    for (int e = tid; e < RL << n_out; e += BT) {
+      const int l = e >> n_out, yj = e & (dout - 1), yi = rinv[row_of(lb, (uint32_t)l)];
+      if (yi < 0) continue;
+      out[((int64_t)yi << n_out) + yj] =
+          st_code == MBQC_RUN_OK ? R[l * D + rsw((uint32_t)ridx[yj])] : make_float2(NAN, NAN);
+    }
+    if (tid == 0 && rank == 0 && A.status) A.status[run] = st_code;
+    cluster_arrive();  // the rows and the tables are reused by the cluster's next run; no block
+    cluster_wait();    // leaves while another may still write to it
+  }
 }
 
 // Windows 9..11: R (512 KB to 8 MB) in the workspace, one slice per cluster of
@@ -462,11 +838,8 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
 // overlaps it.  What bounds it is the L2: a step moves the slice in and out
 // once.  One 1024-thread block a run left the rest of the GPU idle and ran at
 // what one SM draws from L2: 24 runs of an 8 x 6 grid (window 9) took
-// 711 us, XXX us with eight blocks a run.
+// 711 us, 325 us with eight blocks a run.
 constexpr int kFactWsThreads = 512;
-
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // Sum of the hi + lo pairs of the block's threads, the same bits in each
 // (two-sum at every addition); scratch double-buffered as in group_sum2_db.
@@ -549,6 +922,7 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
     __syncthreads();
 
     int32_t st_code = MBQC_RUN_OK;
+    int n_rec = 0;  // steps with a recorded probability
     for (int k = 0; k < M; ++k) {
       const float4 F = sF[k];
       const uint2 ss = sSt[k];
@@ -591,8 +965,7 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       if (zstep) {
         const float2 tot = block_pair_sum(t_hi, t_lo, sRed, par);
         if (A.flags & MBQC_F_DM_EXPECTATION) {
-          if (g == 0 && A.probs)
-            A.probs[run * A.ostride + k] = 1.0 - ((double)prob.x + (double)prob.y) / ((double)tot.x + (double)tot.y);
+          if (tid == 0) sF[k] = make_float4(prob.x, prob.y, tot.x, tot.y);
           G = make_float4(1.f, 1.f, 0.f, 0.f);
           prob = make_float2(1.f, 0.f);
           outcome = 2;
@@ -603,7 +976,8 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       } else {
         take1 = !pair_ge(prob, 1e-4);  // prob0 < 1e-4 (or NaN): outcome 1 (np_simulator_dm.py:335-338)
       }
-      if (g == 0 && A.probs && !unprojected) A.probs[run * A.ostride + k] = (double)prob.x + (double)prob.y;
+      if (tid == 0 && !unprojected) sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      n_rec = k + 1;
       if (take1) {  // outcome 1 with P1 = I - P0
         G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
         prob = block_pair_sum(o_hi, o_lo, sRed, par);
@@ -744,6 +1118,8 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       ridx[y] = ri;
     }
     __syncthreads();
+    if (crank == 0 && A.probs)
+      for (int k = tid; k < n_rec; k += BT) A.probs[run * A.ostride + k] = prob_record(sF[k]);
     float2 *out = A.rho_out + run * A.out_stride;
     for (int e = g; e < dout * dout; e += TT) {
       const int yi = e >> n_out, yj = e & (dout - 1);
