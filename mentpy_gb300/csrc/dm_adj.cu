@@ -5,17 +5,20 @@
 
 #include "dispatch.h"
 #include "dm_adj.cuh"
+#include "dm_adj_fact.cuh"
 
 namespace mbqc {
 
 struct DmAdjGeometry {
+  bool fact;  // the factored kernel
   int blocks, maxm, max_a, max_out;
   size_t smem, ws_bytes;
   int64_t slots;
 };
 
-// Workspace: [slots][maxm][4^w] pre-step matrices, then (windows above
-// kDmAdjSmemMaxWindow) [slots][4^w] for the matrix itself.
+// Workspace: [slots][maxm][4^w] pre-step matrices (factored kernel: a quarter
+// of that), then (windows above kDmAdjSmemMaxWindow) [slots][4^w] for the matrix
+// itself.
 template <int W>
 static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g) {
   using Cfg = DmCfg<W>;
@@ -31,7 +34,24 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
   rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, ACfg::BLOCK, g.smem), "occupancy");
   if (rc) return rc;
   if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: kernel does not fit on an SM");
-  const size_t per_slot = ((size_t)maxm + (ACfg::kWs ? 1 : 0)) * Cfg::N * sizeof(float2);
+  size_t per_slot = ((size_t)maxm + (ACfg::kWs ? 1 : 0)) * Cfg::N * sizeof(float2);
+  if constexpr (W >= 3 && W <= 7) {
+    if (g.fact) {
+      auto kf = dm_adj_fact<W>;
+      g.smem = (size_t)ACfg::GROUPS * adj_fact_slice<W>(maxm);
+      rc = cuda_check(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem),
+                      "dm adjoint smem attribute");
+      if (!rc)  // the largest shared-memory carveout: several runs per SM
+        rc = cuda_check(cudaFuncSetAttribute(kf, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                             (int)cudaSharedmemCarveoutMaxShared),
+                        "dm adjoint carveout attribute");
+      if (!rc)
+        rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kf, ACfg::BLOCK, g.smem), "occupancy");
+      if (rc) return rc;
+      if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: kernel does not fit on an SM");
+      per_slot = (size_t)maxm * AdjFactCfg<W>::HIST * sizeof(float4);
+    }
+  }
   int64_t blocks = std::min<int64_t>((batch + ACfg::GROUPS - 1) / ACfg::GROUPS, (int64_t)sm_count() * occ);
   // bound the workspace; fewer runs in flight if needed
   while (blocks > 1 && (size_t)blocks * ACfg::GROUPS * per_slot > ws_cap) blocks = (blocks + 1) / 2;
@@ -44,12 +64,19 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
 
 template <int W>
 static int dm_adj_launch(DmAdjArgs a, const DmAdjGeometry &g, cudaStream_t s) {
+  if constexpr (W >= 3 && W <= 7) {
+    if (g.fact) {
+      dm_adj_fact<W><<<g.blocks, DmAdjCfg<W>::BLOCK, g.smem, s>>>(a);
+      return check_launch("dm_adj_fact");
+    }
+  }
   a.rho_ws = DmAdjCfg<W>::kWs ? a.hist + g.slots * (int64_t)g.maxm * DmCfg<W>::N : nullptr;
   dm_adj_smem<W><<<g.blocks, DmAdjCfg<W>::BLOCK, g.smem, s>>>(a);
   return check_launch("dm_adj_smem");
 }
 
-static int dm_adj_geometry(int w, int64_t batch, int maxm, DmAdjGeometry &g) {
+static int dm_adj_geometry(int w, int64_t batch, int maxm, bool fact, DmAdjGeometry &g) {
+  g.fact = fact;
   // pre-step history: 2 GiB at most in shared-memory windows, 16 GiB above
   const size_t cap = w > kDmAdjSmemMaxWindow ? (size_t)16 << 30 : (size_t)2 << 30;
   switch (w) {
@@ -67,9 +94,12 @@ static int dm_adj_geometry(int w, int64_t batch, int maxm, DmAdjGeometry &g) {
   }
 }
 
+// fact: every circuit of the window ends with a step that shrinks it (the
+// factored kernel's condition).
 static int plan_extents(const mbqc_plan *plan, int window, const int32_t *run_circuit, int &maxm, int &max_in,
-                        int &max_out, int &max_a) {
+                        int &max_out, int &max_a, bool &fact) {
   const PlanView v = view_of(plan);
+  fact = true;
   maxm = 1;
   max_in = max_out = max_a = 0;
   for (int c = 0; c < v.n_circuits; ++c) {
@@ -83,6 +113,7 @@ static int plan_extents(const mbqc_plan *plan, int window, const int32_t *run_ci
     if (hc.has_z)
       return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: circuit %d measures in the Z basis (drawn or unprojected "
                   "outcomes have no adjoint here)", c);
+    if (hc.n_steps < 1 || !(host_steps(plan, c)[hc.n_steps - 1].mask & kDead)) fact = false;
     maxm = std::max(maxm, hc.n_steps);
     max_in = std::max(max_in, hc.n_in);
     max_out = std::max(max_out, hc.n_out);
@@ -103,10 +134,11 @@ int mbqc_dm_adjoint_workspace(const mbqc_plan *plan, int64_t batch, int32_t wind
   *bytes = 0;
   if (batch == 0) return MBQC_OK;
   int maxm, mi, mo, ma;
-  int rc = plan_extents(plan, window, run_circuit, maxm, mi, mo, ma);
+  bool fact;
+  int rc = plan_extents(plan, window, run_circuit, maxm, mi, mo, ma, fact);
   if (rc) return rc;
   DmAdjGeometry g;
-  rc = dm_adj_geometry(window, batch, maxm, g);
+  rc = dm_adj_geometry(window, batch, maxm, fact, g);
   if (rc) return rc;
   *bytes = g.ws_bytes;
   return MBQC_OK;
@@ -124,7 +156,8 @@ int mbqc_dm_adjoint(const mbqc_plan *plan, int64_t batch, int32_t window, const 
   if (!psi_in || !grad_out || !grad_angles) return fail(MBQC_E_INVALID, "dm_adjoint: null buffer");
   if (!(noise >= 0.0 && noise <= 1.0)) return fail(MBQC_E_INVALID, "dm_adjoint: noise %g", noise);
   int maxm, max_in, max_out, max_a;
-  int rc = plan_extents(plan, window, run_circuit, maxm, max_in, max_out, max_a);
+  bool fact;
+  int rc = plan_extents(plan, window, run_circuit, maxm, max_in, max_out, max_a, fact);
   if (rc) return rc;
   if (max_a > 0 && (!angles || angle_stride < max_a || grad_stride < max_a))
     return fail(MBQC_E_INVALID, "dm_adjoint: angle/gradient stride < %d", max_a);
@@ -134,7 +167,7 @@ int mbqc_dm_adjoint(const mbqc_plan *plan, int64_t batch, int32_t window, const 
     return fail(MBQC_E_INVALID, "dm_adjoint: output stride too small");
   if (outcomes && outcome_stride < maxm) return fail(MBQC_E_INVALID, "dm_adjoint: outcome stride too small");
   DmAdjGeometry g;
-  rc = dm_adj_geometry(window, batch, maxm, g);
+  rc = dm_adj_geometry(window, batch, maxm, fact, g);
   if (rc) return rc;
   if (!workspace || workspace_bytes < g.ws_bytes)
     return fail(MBQC_E_INVALID, "dm_adjoint: workspace of %zu bytes, %zu needed", workspace_bytes, g.ws_bytes);

@@ -133,7 +133,7 @@ __device__ __forceinline__ void fact_tables(const DevStep *steps, int M, uint2 *
     }
     sSt[k] = make_uint2(aux, sgn);
   }
-  if (tid < W) sPos[tid] = (int8_t)((M + (tid + W - M % W) % W + W - 2) % (W - 1));
+  if (sPos && tid < W) sPos[tid] = (int8_t)((M + (tid + W - M % W) % W + W - 2) % (W - 1));
 }
 
 // Outputs of one 2x2 block from its entries x_ab (a: row half, b: column
