@@ -34,11 +34,13 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
   rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, ACfg::BLOCK, g.smem), "occupancy");
   if (rc) return rc;
   if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: kernel does not fit on an SM");
+  int groups = ACfg::GROUPS;
   size_t per_slot = ((size_t)maxm + (ACfg::kWs ? 1 : 0)) * Cfg::N * sizeof(float2);
   if constexpr (W >= 3 && W <= 7) {
     if (g.fact) {
       auto kf = dm_adj_fact<W>;
-      g.smem = (size_t)ACfg::GROUPS * adj_fact_slice<W>(maxm);
+      groups = AdjFactCfg<W>::GROUPS;
+      g.smem = (size_t)groups * adj_fact_slice<W>(maxm);
       rc = cuda_check(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem),
                       "dm adjoint smem attribute");
       if (!rc)  // the largest shared-memory carveout: several runs per SM
@@ -46,17 +48,18 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
                                              (int)cudaSharedmemCarveoutMaxShared),
                         "dm adjoint carveout attribute");
       if (!rc)
-        rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kf, ACfg::BLOCK, g.smem), "occupancy");
+        rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kf, groups * AdjFactCfg<W>::TPR, g.smem),
+                        "occupancy");
       if (rc) return rc;
       if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: kernel does not fit on an SM");
       per_slot = (size_t)maxm * AdjFactCfg<W>::HIST * sizeof(float4);
     }
   }
-  int64_t blocks = std::min<int64_t>((batch + ACfg::GROUPS - 1) / ACfg::GROUPS, (int64_t)sm_count() * occ);
+  int64_t blocks = std::min<int64_t>((batch + groups - 1) / groups, (int64_t)sm_count() * occ);
   // bound the workspace; fewer runs in flight if needed
-  while (blocks > 1 && (size_t)blocks * ACfg::GROUPS * per_slot > ws_cap) blocks = (blocks + 1) / 2;
+  while (blocks > 1 && (size_t)blocks * groups * per_slot > ws_cap) blocks = (blocks + 1) / 2;
   g.blocks = (int)std::max<int64_t>(blocks, 1);
-  g.slots = (int64_t)g.blocks * ACfg::GROUPS;
+  g.slots = (int64_t)g.blocks * groups;
   g.ws_bytes = (size_t)g.slots * per_slot;
   g.maxm = maxm;
   return MBQC_OK;
@@ -66,7 +69,7 @@ template <int W>
 static int dm_adj_launch(DmAdjArgs a, const DmAdjGeometry &g, cudaStream_t s) {
   if constexpr (W >= 3 && W <= 7) {
     if (g.fact) {
-      dm_adj_fact<W><<<g.blocks, DmAdjCfg<W>::BLOCK, g.smem, s>>>(a);
+      dm_adj_fact<W><<<g.blocks, AdjFactCfg<W>::GROUPS * AdjFactCfg<W>::TPR, g.smem, s>>>(a);
       return check_launch("dm_adj_fact");
     }
   }

@@ -37,7 +37,8 @@ namespace mbqc {
 template <int W> struct AdjFactCfg {
   static_assert(W >= 3 && W <= 7, "factored adjoint: windows 3..7");
   static constexpr int N = W - 1, D = 1 << N, T = D / 4;
-  static constexpr int TPR = DmCfg<W>::TPR, GROUPS = DmCfg<W>::GROUPS;
+  static constexpr int TPR = DmCfg<W>::TPR;
+  static constexpr int GROUPS = TPR == 32 ? 2 : 1;  // runs per block: small blocks spread a batch over the SMs
   static constexpr int NB = D * D, NI = NB >= TPR ? NB / TPR : 1;  // derivative terms, terms a thread
   static constexpr int RS = TPR / D > 0 ? TPR / D : 1;             // row step between a thread's terms
   static constexpr int HIST = 8 * T * T;                            // float4 a step
@@ -66,7 +67,8 @@ __device__ __forceinline__ float diag_term(float4 G, float q00, float q11, float
 }
 
 template <int W>
-__global__ void __launch_bounds__(256, 3) dm_adj_fact(DmAdjArgs A) {
+__global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512 / (AdjFactCfg<W>::TPR * AdjFactCfg<W>::GROUPS))
+    dm_adj_fact(DmAdjArgs A) {
   using Cfg = AdjFactCfg<W>;
   constexpr int N = Cfg::N, D = Cfg::D, T = Cfg::T, TPR = Cfg::TPR, NB = Cfg::NB, NI = Cfg::NI, RS = Cfg::RS,
                 GROUPS = Cfg::GROUPS, NW = TPR / 32;
@@ -233,35 +235,44 @@ __global__ void __launch_bounds__(256, 3) dm_adj_fact(DmAdjArgs A) {
         const int plo = pa < pb ? pa : pb, phi = pa < pb ? pb : pa;
         const uint32_t rb = ins_bit(ins_bit(tr, plo, 0), phi, 0), cb = ins_bit(ins_bit(tc, plo, 0), phi, 0);
         float4 *h = hist + (int64_t)k * Cfg::HIST;
+        const uint32_t ra = (uint32_t)D << pa, ca = sw(1u << pa), cb2 = sw(1u << pb);
 #pragma unroll
         for (int xr = 0; xr < 2; ++xr)
 #pragma unroll
           for (int xc = 0; xc < 2; ++xc) {
             const uint32_t r0 = rb | ((uint32_t)xr << pb), c0 = cb | ((uint32_t)xc << pb);
-            float2 *p0 = R + r0 * D, *p1 = p0 + (D << pa);
-            const uint32_t s0 = sw(c0), s1 = sw(c0 | (1u << pa));
+            float2 *p0 = R + r0 * D, *p1 = p0 + ra;
+            const uint32_t s0 = sw(cb) ^ (xc ? cb2 : 0u), s1 = s0 ^ ca;
             const float2 y00 = p0[s0], y01 = p0[s1], y10 = p1[s0], y11 = p1[s1];
             if (ss.x & kAdjOff) h[(2 * xr + xc) * (T * T)] = make_float4(y01.x, y01.y, y10.x, y10.y);
             if (ss.x & kAdjPop) h[(4 + 2 * xr + xc) * (T * T)] = make_float4(y00.x, y00.y, y11.x, y11.y);
-            const uint32_t pr = (__popc(r0 & ss.y) & 1u) << 31, pc = (__popc(c0 & ss.y) & 1u) << 31;
-            // the block of slot bits (0, 0), then its copies with the slot's signs
-            auto out = [&](float2 x01, float2 x10, float2 x11) {
-              const float2 f = functional(G, y00, x01, x10, x11);
-              return make_float2(f.x * half, f.y * half);
-            };
-            auto neg = [](float2 v) { return make_float2(-v.x, -v.y); };
-            const float2 o00 = out(y01, y10, y11);
+            // the functional on the block (slot bits 0, 0) and on its copies
+            // with the slot's link signs: the same sums with y01, y10, y11 negated
+            const float tx = __fmul_rn(G.y, y11.x), ty = __fmul_rn(G.y, y11.y);
+            const float ux = y01.x + y10.x, uy = y01.y + y10.y, vx = y01.x - y10.x, vy = y01.y - y10.y;
+            const float px = fmaf(G.x, y00.x, tx), py = fmaf(G.x, y00.y, ty);
+            float2 o00 = make_float2(fmaf(-G.w, vy, fmaf(G.z, ux, px)), fmaf(G.w, vx, fmaf(G.z, uy, py)));
+            o00 = make_float2(o00.x * half, o00.y * half);
             p0[s0] = o00;
             if (pdead) {
               p0[s1] = p1[s0] = p1[s1] = make_float2(0.f, 0.f);
-            } else if (mq) {
-              p0[s1] = flip_sign(out(neg(y01), y10, neg(y11)), pc);
-              p1[s0] = flip_sign(out(y01, neg(y10), neg(y11)), pr);
-              p1[s1] = flip_sign(out(neg(y01), neg(y10), y11), pr ^ pc);
             } else {
-              p0[s1] = flip_sign(o00, pc);
-              p1[s0] = flip_sign(o00, pr);
-              p1[s1] = flip_sign(o00, pr ^ pc);
+              float2 o01 = o00, o10 = o00, o11 = o00;
+              if (mq) {
+                const float mx = fmaf(G.x, y00.x, -tx), my = fmaf(G.x, y00.y, -ty);
+                o11 = make_float2(half * fmaf(G.w, vy, fmaf(-G.z, ux, px)), half * fmaf(-G.w, vx, fmaf(-G.z, uy, py)));
+                o01 = make_float2(half * fmaf(G.w, uy, fmaf(-G.z, vx, mx)), half * fmaf(-G.w, ux, fmaf(-G.z, vy, my)));
+                o10 = make_float2(half * fmaf(-G.w, uy, fmaf(G.z, vx, mx)), half * fmaf(G.w, ux, fmaf(G.z, vy, my)));
+              }
+              if (ss.y) {
+                const uint32_t pr = (__popc(r0 & ss.y) & 1u) << 31, pc = (__popc(c0 & ss.y) & 1u) << 31;
+                o01 = flip_sign(o01, pc);
+                o10 = flip_sign(o10, pr);
+                o11 = flip_sign(o11, pr ^ pc);
+              }
+              p0[s1] = o01;
+              p1[s0] = o10;
+              p1[s1] = o11;
             }
           }
       }
@@ -338,43 +349,78 @@ __global__ void __launch_bounds__(256, 3) dm_adj_fact(DmAdjArgs A) {
       if (tiled) {
         const int plo = pa < pb ? pa : pb, phi = pa < pb ? pb : pa;
         const uint32_t rb = ins_bit(ins_bit(tr, plo, 0), phi, 0), cb = ins_bit(ins_bit(tc, plo, 0), phi, 0);
-        float2 mu[4][4];  // [row][column] over (position a) + 2 (position b)
+        const float4 *hk = hist + (int64_t)k * Cfg::HIST;
+        float4 hv[4];  // the measured qubit's coherences, in flight early
+        if ((ss.x & kAdjOff) && k > 0) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) hv[g] = hk[g * (T * T)];
+        }
+        // row and column i, i = (position a) + 2 (position b)
+        auto row = [&](int i) { return rb | ((uint32_t)(i & 1) << pa) | ((uint32_t)(i >> 1) << pb); };
+        auto col = [&](int j) { return cb | ((uint32_t)(j & 1) << pa) | ((uint32_t)(j >> 1) << pb); };
+        uint32_t rp[4], cp[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          rp[i] = row(i) * D;
+          cp[i] = sw(col(i));
+        }
+        float2 mu[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            mu[i][j] = R[(rb | ((uint32_t)(i & 1) << pa) | ((uint32_t)(i >> 1) << pb)) * D +
-                         sw(cb | ((uint32_t)(j & 1) << pa) | ((uint32_t)(j >> 1) << pb))];
+          for (int j = 0; j < 4; ++j) mu[i][j] = R[rp[i] + cp[j]];
         if (k < M - 1) {
           // Lambda_k from m_{k+1} and step k+1's functional, then mu_k = E^dagger Lambda_k
           float4 G = sF[k + 1];
           if (sOut[k + 1]) G = make_float4(tr_noise - G.x, tr_noise - G.y, -G.z, -G.w);
           const uint2 sn = sSt[k + 1];
           const bool mqn = (sn.x & kFactMq) != 0u, dead = (sn.x & kFactDead) != 0u;
+          if (sn.y) {  // the slot's links to the qubits other than the next measured one
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+              const uint32_t prs = (__popc(row(o) & sn.y) & 1u) << 31, pcs = (__popc(col(o) & sn.y) & 1u) << 31;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                mu[2 + o][j] = flip_sign(mu[2 + o][j], prs);
+                mu[j][2 + o] = flip_sign(mu[j][2 + o], pcs);
+              }
+            }
+          }
+          // Lambda entry of (x, x') from m: conj(G_xx') m, rounded before the
+          // sums as the stored entries were
+          auto lam = [&](int x, int xp, float2 m) {
+            if (x == 0 && xp == 0) return make_float2(__fmul_rn(G.x, m.x), __fmul_rn(G.x, m.y));
+            if (x == 1 && xp == 1) return make_float2(__fmul_rn(G.y, m.x), __fmul_rn(G.y, m.y));
+            const float zx = __fmul_rn(G.z, m.x), wx = __fmul_rn(G.w, m.x);
+            if (x == 0) return make_float2(fmaf(G.w, m.y, zx), fmaf(G.z, m.y, -wx));  // conj(G01) m
+            return make_float2(fmaf(-G.w, m.y, zx), fmaf(G.z, m.y, wx));              // G01 m
+          };
 #pragma unroll
           for (int orr = 0; orr < 2; ++orr)
 #pragma unroll
             for (int oc = 0; oc < 2; ++oc) {
-              const uint32_t prs = (__popc((rb | ((uint32_t)orr << pa)) & sn.y) & 1u) << 31;
-              const uint32_t pcs = (__popc((cb | ((uint32_t)oc << pa)) & sn.y) & 1u) << 31;
-              const float2 m00 = mu[orr][oc], m01 = flip_sign(mu[orr][oc + 2], pcs);
-              const float2 m10 = flip_sign(mu[orr + 2][oc], prs), m11 = flip_sign(mu[orr + 2][oc + 2], prs ^ pcs);
-              // Lambda entry of (x, x') from m: conj(G_xx') m
-              auto lam = [&](int x, int xp, float2 m) {
-                // (rounded before the sums, as the stored entries were)
-                if (x == 0 && xp == 0) return make_float2(__fmul_rn(G.x, m.x), __fmul_rn(G.x, m.y));
-                if (x == 1 && xp == 1) return make_float2(__fmul_rn(G.y, m.x), __fmul_rn(G.y, m.y));
-                const float zx = __fmul_rn(G.z, m.x), wx = __fmul_rn(G.w, m.x);
-                if (x == 0) return make_float2(fmaf(G.w, m.y, zx), fmaf(G.z, m.y, -wx));  // conj(G01) m
-                return make_float2(fmaf(-G.w, m.y, zx), fmaf(G.z, m.y, wx));              // G01 m
-              };
+              const float2 m00 = mu[orr][oc], m01 = mu[orr][oc + 2], m10 = mu[orr + 2][oc], m11 = mu[orr + 2][oc + 2];
+              if (mqn && !dead && G.x == G.y) {
+                // XY, linked slot: the signs (-1)^x on slot row 1 and (-1)^x' on
+                // slot column 1 are additions or subtractions; one product for
+                // the two populations
+                auto add4 = [](float2 a, float2 b, float2 c, float2 d, float sb, float sc, float sd) {
+                  return make_float2(0.5f * (a.x + sb * b.x + sc * c.x + sd * d.x),
+                                     0.5f * (a.y + sb * b.y + sc * c.y + sd * d.y));
+                };
+                const float2 q0 = lam(0, 0, m00), q1 = lam(0, 0, m01), q2 = lam(0, 0, m10), q3 = lam(0, 0, m11);
+                mu[orr][oc] = add4(q0, q1, q2, q3, 1.f, 1.f, 1.f);
+                mu[orr + 2][oc + 2] = add4(q0, q1, q2, q3, -1.f, -1.f, 1.f);
+                mu[orr][oc + 2] = add4(lam(0, 1, m00), lam(0, 1, m01), lam(0, 1, m10), lam(0, 1, m11), -1.f, 1.f, -1.f);
+                mu[orr + 2][oc] = add4(lam(1, 0, m00), lam(1, 0, m01), lam(1, 0, m10), lam(1, 0, m11), 1.f, -1.f, -1.f);
+                continue;
+              }
 #pragma unroll
               for (int x = 0; x < 2; ++x)
 #pragma unroll
                 for (int xp = 0; xp < 2; ++xp) {
                   float2 v = lam(x, xp, m00);
                   if (!dead) {
-                    // the measured qubit's link to the slot: (-1)^{x} on slot row 1, (-1)^{x'} on slot column 1
                     const uint32_t sx = x && mqn ? 0x80000000u : 0u, sxp = xp && mqn ? 0x80000000u : 0u;
                     const float2 l01 = flip_sign(lam(x, xp, m01), sxp), l10 = flip_sign(lam(x, xp, m10), sx);
                     const float2 l11 = flip_sign(lam(x, xp, m11), sx ^ sxp);
@@ -386,75 +432,97 @@ __global__ void __launch_bounds__(256, 3) dm_adj_fact(DmAdjArgs A) {
         }
         // derivative terms Re(conj(mu) dsigma), each to its full-matrix thread
         if (ss.x & kAdjOff) {
-          float4 dG;
-          if (ss.x & kAdjPop) {
-            const DevStep st = steps[k];
-            float dx, dy, dz;
-            dbloch(st.plane, ang[st.aidx], dx, dy, dz);
-            dG = make_float4(a_n * 0.5f * dz, -a_n * 0.5f * dz, a_n * 0.5f * dx, a_n * 0.5f * dy);
-          } else {
-            const float4 F = sF[k];
-            dG = make_float4(0.f, 0.f, -F.w, F.z);  // XY: the functional's quarter turn
-          }
-          if (sOut[k]) dG = make_float4(-dG.x, -dG.y, -dG.z, -dG.w);
           const int h = ((k % W - k) % N + N) % N;  // position -> bit of the full-matrix block index
           const bool mq = (ss.x & kFactMq) != 0u, pdead = (ss.x & kFactDead) != 0u;
-          const float4 *hk = hist + (int64_t)k * Cfg::HIST;
-          auto term = [&](int i, int j, float2 x00, float2 x01, float2 x10, float2 x11) {
-            const float2 d = functional(dG, x00, x01, x10, x11);
-            const uint32_t r = rotl(rb | ((uint32_t)(i & 1) << pa) | ((uint32_t)(i >> 1) << pb), h);
-            const uint32_t c = rotl(cb | ((uint32_t)(j & 1) << pa) | ((uint32_t)(j >> 1) << pb), h);
-            tb[r * D + (N == 6 ? c ^ ((c >> 5) * 10u) ^ ((__popc(r) & 1u) * 21u) : c)] =
-                fmaf(mu[i][j].x, d.x, __fmul_rn(mu[i][j].y, d.y));
+          uint32_t tp[4], tq[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t r = rotl(row(i), h), c = rotl(col(i), h);
+            tp[i] = (r * D) ^ (N == 6 ? (__popc(r) & 1u) * 21u : 0u);
+            tq[i] = N == 6 ? c ^ ((c >> 5) * 10u) : c;
+          }
+          auto term = [&](int i, int j, float2 d) {
+            tb[tp[i] ^ tq[j]] = fmaf(mu[i][j].x, d.x, __fmul_rn(mu[i][j].y, d.y));
           };
+          if (!(ss.x & kAdjPop) && k > 0 && mq && !pdead) {
+            // XY, linked slot: dG = (0, 0, -Im G01, Re G01), the coherences' quarter
+            // turn; the four copies of a block give +-two values
+            const float4 F = sF[k];
+            const float dz = sOut[k] ? F.w : -F.w, dw = sOut[k] ? -F.z : F.z;
 #pragma unroll
-          for (int xr = 0; xr < 2; ++xr)
-#pragma unroll
-            for (int xc = 0; xc < 2; ++xc) {
-              if (k == 0) {
-                // the initial matrix has no slot: each (r, c) has its own block
-#pragma unroll
-                for (int ar = 0; ar < 2; ++ar)
-#pragma unroll
-                  for (int ac = 0; ac < 2; ++ac) {
-                    const uint32_t r = rb | ((uint32_t)ar << pa) | ((uint32_t)xr << pb);
-                    const uint32_t c = cb | ((uint32_t)ac << pa) | ((uint32_t)xc << pb);
-                    term(ar + 2 * xr, ac + 2 * xc, rho0(2 * r, 2 * c), rho0(2 * r, 2 * c + 1),
-                         rho0(2 * r + 1, 2 * c), rho0(2 * r + 1, 2 * c + 1));
-                  }
-                continue;
+            for (int g = 0; g < 4; ++g) {
+              const int xr = g >> 1, xc = g & 1;
+              const float4 v = hv[g];  // y01, y10
+              const float ux = v.x + v.z, uy = v.y + v.w, vx = v.x - v.z, vy = v.y - v.w;
+              float2 d0 = make_float2(fmaf(-dw, vy, __fmul_rn(dz, ux)), fmaf(dw, vx, __fmul_rn(dz, uy)));
+              float2 d1 = make_float2(fmaf(dw, uy, __fmul_rn(-dz, vx)), fmaf(-dw, ux, __fmul_rn(-dz, vy)));
+              float2 d2 = make_float2(-d1.x, -d1.y), d3 = make_float2(-d0.x, -d0.y);
+              if (ss.y) {
+                const uint32_t prs = (__popc(row(2 * xr) & ss.y) & 1u) << 31, pcs = (__popc(col(2 * xc) & ss.y) & 1u) << 31;
+                d1 = flip_sign(d1, pcs);
+                d2 = flip_sign(d2, prs);
+                d3 = flip_sign(d3, prs ^ pcs);
               }
-              const float4 v = hk[(2 * xr + xc) * (T * T)];
-              float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (ss.x & kAdjPop) w = hk[(4 + 2 * xr + xc) * (T * T)];
-              const float2 y01 = make_float2(v.x, v.y), y10 = make_float2(v.z, v.w);
-              const float2 y00 = make_float2(w.x, w.y), y11 = make_float2(w.z, w.w);
-              const uint32_t prs = (__popc((rb | ((uint32_t)xr << pb)) & ss.y) & 1u) << 31;
-              const uint32_t pcs = (__popc((cb | ((uint32_t)xc << pb)) & ss.y) & 1u) << 31;
-              const float2 zero = make_float2(0.f, 0.f);
-#pragma unroll
-              for (int ar = 0; ar < 2; ++ar)
-#pragma unroll
-                for (int ac = 0; ac < 2; ++ac) {
-                  // entries of the block with slot bits (ar, ac)
-                  const uint32_t s = (ar ? prs : 0u) ^ (ac ? pcs : 0u);
-                  const uint32_t sr = ar && mq ? 0x80000000u : 0u, sc = ac && mq ? 0x80000000u : 0u;
-                  if (pdead && (ar || ac))
-                    term(ar + 2 * xr, ac + 2 * xc, zero, zero, zero, zero);
-                  else
-                    term(ar + 2 * xr, ac + 2 * xc, flip_sign(y00, s), flip_sign(y01, s ^ sc),
-                         flip_sign(y10, s ^ sr), flip_sign(y11, s ^ sr ^ sc));
-                }
+              term(2 * xr, 2 * xc, d0);
+              term(2 * xr, 2 * xc + 1, d1);
+              term(2 * xr + 1, 2 * xc, d2);
+              term(2 * xr + 1, 2 * xc + 1, d3);
             }
+          } else {
+            float4 dG;
+            if (ss.x & kAdjPop) {
+              const DevStep st = steps[k];
+              float dx, dy, dz;
+              dbloch(st.plane, ang[st.aidx], dx, dy, dz);
+              dG = make_float4(a_n * 0.5f * dz, -a_n * 0.5f * dz, a_n * 0.5f * dx, a_n * 0.5f * dy);
+            } else {
+              const float4 F = sF[k];
+              dG = make_float4(0.f, 0.f, -F.w, F.z);
+            }
+            if (sOut[k]) dG = make_float4(-dG.x, -dG.y, -dG.z, -dG.w);
+#pragma unroll 1
+            for (int e = 0; e < 16; ++e) {  // rows and columns over (slot, next measured)
+              const int xr = e >> 3, xc = (e >> 2) & 1, ar = (e >> 1) & 1, ac = e & 1;
+              const uint32_t r = rb | ((uint32_t)ar << pa) | ((uint32_t)xr << pb);
+              const uint32_t c = cb | ((uint32_t)ac << pa) | ((uint32_t)xc << pb);
+              float2 x00 = make_float2(0.f, 0.f), x01 = x00, x10 = x00, x11 = x00;
+              if (k == 0) {  // the initial matrix has no slot: each (r, c) has its own block
+                x00 = rho0(2 * r, 2 * c);
+                x01 = rho0(2 * r, 2 * c + 1);
+                x10 = rho0(2 * r + 1, 2 * c);
+                x11 = rho0(2 * r + 1, 2 * c + 1);
+              } else if (!(pdead && (ar || ac))) {
+                const float4 v = hk[(2 * xr + xc) * (T * T)];
+                float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (ss.x & kAdjPop) w = hk[(4 + 2 * xr + xc) * (T * T)];
+                // entries of the block with slot bits (ar, ac)
+                const uint32_t prs = (__popc((rb | ((uint32_t)xr << pb)) & ss.y) & 1u) << 31;
+                const uint32_t pcs = (__popc((cb | ((uint32_t)xc << pb)) & ss.y) & 1u) << 31;
+                const uint32_t s = (ar ? prs : 0u) ^ (ac ? pcs : 0u);
+                const uint32_t sr = ar && mq ? 0x80000000u : 0u, sc = ac && mq ? 0x80000000u : 0u;
+                x00 = flip_sign(make_float2(w.x, w.y), s);
+                x01 = flip_sign(make_float2(v.x, v.y), s ^ sc);
+                x10 = flip_sign(make_float2(v.z, v.w), s ^ sr);
+                x11 = flip_sign(make_float2(w.z, w.w), s ^ sr ^ sc);
+              }
+              const float2 d = functional(dG, x00, x01, x10, x11);
+              float2 m = mu[0][0];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  if (i == ar + 2 * xr && j == ac + 2 * xc) m = mu[i][j];
+              const uint32_t rr = rotl(r, h), cc = rotl(c, h);
+              tb[(rr * D) ^ (N == 6 ? (cc ^ ((cc >> 5) * 10u)) ^ ((__popc(rr) & 1u) * 21u) : cc)] =
+                  fmaf(m.x, d.x, __fmul_rn(m.y, d.y));
+            }
+          }
         }
         // m_k = mu_k / prob_k
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            R[(rb | ((uint32_t)(i & 1) << pa) | ((uint32_t)(i >> 1) << pb)) * D +
-              sw(cb | ((uint32_t)(j & 1) << pa) | ((uint32_t)(j >> 1) << pb))] =
-                make_float2(ck * mu[i][j].x, ck * mu[i][j].y);
+          for (int j = 0; j < 4; ++j) R[rp[i] + cp[j]] = make_float2(ck * mu[i][j].x, ck * mu[i][j].y);
       }
       group_sync(TPR, group);
       // the partial sums of the step before (their warps wrote them before this barrier)
@@ -476,11 +544,13 @@ __global__ void __launch_bounds__(256, 3) dm_adj_fact(DmAdjArgs A) {
       if (ss.x & kAdjOff) {
         float g = 0.f;
         if (NB >= TPR || tid < NB) {
-          const uint32_t c = (uint32_t)tid % D;
+          const uint32_t c = (uint32_t)tid % D, r0 = (uint32_t)tid / D;
+          const uint32_t at = r0 * D + (N == 6 ? c ^ ((c >> 5) * 10u) ^ ((__popc(r0) & 1u) * 21u) : c);
 #pragma unroll
           for (int i = 0; i < NI; ++i) {
-            const uint32_t r = (uint32_t)tid / D + (uint32_t)i * RS;
-            g += tb[r * D + (N == 6 ? c ^ ((c >> 5) * 10u) ^ ((__popc(r) & 1u) * 21u) : c)];
+            constexpr uint32_t step = (uint32_t)RS * D;
+            const uint32_t odd = ((i ^ (i >> 1) ^ (i >> 2) ^ (i >> 3)) & 1) && N == 6 ? 21u : 0u;
+            g += tb[(at ^ odd) + i * step];
           }
         }
         float hi = g, lo = 0.f;
