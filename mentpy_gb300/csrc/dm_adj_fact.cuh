@@ -47,7 +47,7 @@ template <int W> struct AdjFactCfg {
 // shared memory of one run
 template <int W> __host__ __device__ constexpr size_t adj_fact_slice(int maxm) {
   using Cfg = AdjFactCfg<W>;
-  return ((size_t)Cfg::NB * 8 + 2 * (size_t)Cfg::NB * 4 + ((size_t)1 << W) * 8 + (size_t)maxm * 36 + 16 +
+  return ((size_t)Cfg::NB * 8 + 2 * (size_t)Cfg::NB * 4 + ((size_t)1 << W) * 12 + (size_t)maxm * 32 + 16 +
           2 * 8 * sizeof(float2) + 2 * sizeof(float2) + 15) &
          ~(size_t)15;
 }
@@ -81,10 +81,11 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
   float2 *psi = R + NB;
   float *tmp = reinterpret_cast<float *>(psi + (1 << W));  // two buffers of derivative terms
   uint2 *sSt = reinterpret_cast<uint2 *>(tmp + 2 * NB);
-  float2 *sProb = reinterpret_cast<float2 *>(sSt + maxm);
-  float2 *sGr = sProb + maxm;   // two buffers of a partial per warp
-  float2 *sBr = sGr + 2 * 8;    // two broadcast slots
-  int32_t *sOut = reinterpret_cast<int32_t *>(sBr + 2);
+  float2 *sGr = reinterpret_cast<float2 *>(sSt + maxm);  // two buffers of a partial per warp
+  float2 *sBr = sGr + 2 * 8;                             // two broadcast slots
+  float *sInv = reinterpret_cast<float *>(sBr + 2);      // 1 / prob_k
+  int32_t *sOut = reinterpret_cast<int32_t *>(sInv + maxm);
+  int32_t *sMap = sOut + maxm;  // window index -> output index << 8 | storage position of the final matrix, or -1
   const int64_t slot = (int64_t)blockIdx.x * GROUPS + group;
   const DmArgs &F0 = A.f;
   const float qn = f64_to_f32_rn(F0.noise);
@@ -126,7 +127,12 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
     }
   };
 
-  for (int64_t bq = slot; bq < F0.B; bq += (int64_t)gridDim.x * GROUPS) {
+  // runs back and forth over the slots: lists come longest first, so a slot
+  // that began with a long run gets a short one (or none) next
+  const int64_t nslots = (int64_t)gridDim.x * GROUPS;
+  for (int64_t wave = 0; wave * nslots < F0.B; ++wave) {
+    const int64_t bq = wave * nslots + ((wave & 1) ? nslots - 1 - slot : slot);
+    if (bq >= F0.B) continue;
     const int ci = F0.run_circuit ? F0.run_circuit[bq] : 0;
     const int64_t run = F0.run_circuit ? (int64_t)ci : bq;
     const DevCircuit &C = F0.circ[ci];
@@ -211,7 +217,6 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
         outcome = 1;
       }
       if (tid == 0) {
-        sProb[k] = prob;
         sOut[k] = outcome;
         if (F0.outcomes) F0.outcomes[run * F0.ostride + k] = (int8_t)outcome;
       }
@@ -221,6 +226,7 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
       }
       float inv = 1.f / prob.x;
       inv = fmaf(-inv * inv, prob.y, inv);
+      if (tid == 0) sInv[k] = inv;
       const bool dead = k + 1 == M || (sSt[k + 1].x & kFactDead) != 0u;
       const float half = dead ? inv : 0.5f * inv;
       if (k == 0) {
@@ -309,14 +315,19 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
     // output, and Re<Gamma|rho_out>
     const int dout = 1 << C.n_out;
     const float2 *gam = A.grad_out + run * A.gout_stride;
+    for (int i = tid; i < 1 << W; i += TPR) {
+      const int y = __ldg(&map[i]).y;
+      sMap[i] = y >= 0 ? (y << 8) | (int)pos_of((uint32_t)i) : -1;
+    }
+    group_sync(TPR, group);
     float zpart = 0.f;
     for (int e = tid; e < 1 << (2 * W); e += TPR) {
-      const uint32_t i = (uint32_t)e >> W, j = (uint32_t)e & ((1u << W) - 1u);
-      const int yi = __ldg(&map[i]).y, yj = __ldg(&map[j]).y;
-      if (yi >= 0 && yj >= 0) {
-        const float2 x = R[pos_of(i) * D + sw(pos_of(j))], g = gam[yi * dout + yj];
+      const int mi = sMap[e >> W], mj = sMap[e & ((1 << W) - 1)];
+      if ((mi | mj) >= 0) {
+        const int o = (mi >> 8) * dout + (mj >> 8);
+        const float2 x = R[(mi & 255) * D + sw(mj & 255)], g = gam[o];
         zpart += fmaf(g.x, x.x, __fmul_rn(g.y, x.y));
-        if (F0.rho_out) F0.rho_out[run * F0.out_stride + yi * dout + yj] = x;
+        if (F0.rho_out) F0.rho_out[run * F0.out_stride + o] = x;
       }
     }
     const float2 zp = group_sum2<TPR>(zpart, sGr, tid, group);
@@ -325,11 +336,11 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
     // seed Lambda = Gamma - z I on the output subspace
     for (int e = tid; e < NB; e += TPR) {
       const uint32_t r = (uint32_t)e / D, c = (uint32_t)e % D;
-      const int yi = __ldg(&map[win_of(r)]).y, yj = __ldg(&map[win_of(c)]).y;
+      const int mi = sMap[win_of(r)], mj = sMap[win_of(c)];
       float2 l = make_float2(0.f, 0.f);
-      if (yi >= 0 && yj >= 0) {
-        l = gam[yi * dout + yj];
-        if (yi == yj) l.x -= z;
+      if ((mi | mj) >= 0) {
+        l = gam[(mi >> 8) * dout + (mj >> 8)];
+        if (mi == mj) l.x -= z;
       }
       R[r * D + sw(c)] = l;
     }
@@ -341,9 +352,7 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
     // R holds mu_{M-1} (the last step shrinks the window), then m_{k+1}
     for (int k = M - 1; k >= 0; --k) {
       const uint2 ss = sSt[k];
-      const float2 pk = sProb[k];
-      float ck = 1.f / pk.x;
-      ck = fmaf(-ck * ck, pk.y, ck);
+      const float ck = sInv[k];
       const int pa = (k + N - 1) % N, pb = k % N;
       float *tb = tmp + (k & 1) * NB;
       if (tiled) {
@@ -533,12 +542,9 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
           const float2 q = sGr[(kk & 1) * 8 + i];
           two_sum_acc(p.x, p.y, q.x, q.y);
         }
-        const float2 pq = sProb[kk];
-        float cc = 1.f / pq.x;
-        cc = fmaf(-cc * cc, pq.y, cc);
         const float s = p.x + p.y;  // renormalised pair hi + lo, then their sum
         const float gk = s + (p.y - (s - p.x));
-        grad[steps[kk].aidx] = (double)(cc * gk);
+        grad[steps[kk].aidx] = (double)(sInv[kk] * gk);
       };
       if (tid == 0 && k + 1 < M && (sSt[k + 1].x & kAdjOff)) finish(k + 1);
       if (ss.x & kAdjOff) {
