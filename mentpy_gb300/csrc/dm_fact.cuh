@@ -138,6 +138,9 @@ __device__ __forceinline__ void fact_tables(const DevStep *steps, int M, uint2 *
 
 // Outputs of one 2x2 block from its entries x_ab (a: row half, b: column
 // half); hA, hB, hR, hI: the functional with the step's scale folded in.
+// LINKED: the slot has a CZ to the measured qubit (pdead, mq not looked at);
+// SIGNED: pr, pc may be nonzero.
+template <bool LINKED = false, bool SIGNED = true>
 __device__ __forceinline__ void fact_combine(float hA, float hB, float hR, float hI, bool pdead, bool mq, float2 x00,
                                              float2 x01, float2 x10, float2 x11, uint32_t pr, uint32_t pc,
                                              float2 &o00, float2 &o01, float2 &o10, float2 &o11) {
@@ -148,19 +151,131 @@ __device__ __forceinline__ void fact_combine(float hA, float hB, float hR, float
   const float2 u = make_float2(x01.x + x10.x, x01.y + x10.y), v = make_float2(x01.x - x10.x, x01.y - x10.y);
   const float2 sB = make_float2(fmaf(hR, u.x, -hI * v.y), fmaf(hR, u.y, hI * v.x));
   o00 = make_float2(sA.x + sB.x, sA.y + sB.y);
-  if (pdead) {
+  if (!LINKED && pdead) {
     o01 = o10 = o11 = make_float2(0.f, 0.f);
-  } else if (!mq) {
-    o01 = flip_sign(o00, pc);
-    o10 = flip_sign(o00, pr);
-    o11 = flip_sign(o00, pr ^ pc);
-  } else {
+    return;
+  }
+  if (LINKED || mq) {
     // signs (-1)^{a' a + b' b} on the terms: T01 = dA + dB, T10 = dA - dB, T11 = sA - sB
     const float2 dA = make_float2(fmaf(-hB, x11.x, px), fmaf(-hB, x11.y, py));
     const float2 dB = make_float2(fmaf(hI, u.y, -hR * v.x), fmaf(-hI, u.x, -hR * v.y));
-    o01 = flip_sign(make_float2(dA.x + dB.x, dA.y + dB.y), pc);
-    o10 = flip_sign(make_float2(dA.x - dB.x, dA.y - dB.y), pr);
-    o11 = flip_sign(make_float2(sA.x - sB.x, sA.y - sB.y), pr ^ pc);
+    o01 = make_float2(dA.x + dB.x, dA.y + dB.y);
+    o10 = make_float2(dA.x - dB.x, dA.y - dB.y);
+    o11 = make_float2(sA.x - sB.x, sA.y - sB.y);
+  } else {
+    o01 = o10 = o11 = o00;
+  }
+  if (SIGNED) {
+    o01 = flip_sign(o01, pc);
+    o10 = flip_sign(o10, pr);
+    o11 = flip_sign(o11, pr ^ pc);
+  }
+}
+
+// One in-place pass over the 2x2 blocks of position pos.  16-byte
+// shared-memory accesses: at pos 0 a block's two columns are adjacent (one
+// float4 per row); at pos > 0 a unit is the two blocks of columns c0 and c0 + 1
+// (one float4 per row and column half).  A thread keeps one column (pair) for
+// the whole pass and walks rows, so its column index, signs and the
+// row-independent address parts are computed once; all loads of U units before
+// their stores (distinct units never alias).
+template <int W, int TPR, bool LINKED, bool SIGNED>
+__device__ __forceinline__ void fact_pass(float2 *R, int tid, int pos, float hA, float hB, float hR, float hI,
+                                          bool pdead, bool mq, uint32_t sgn) {
+  using Cfg = DmFactCfg<W>;
+  constexpr int D = Cfg::D, H = Cfg::H;
+  auto combine = [&](float2 x00, float2 x01, float2 x10, float2 x11, uint32_t pr, uint32_t pc, float2 &o00,
+                     float2 &o01, float2 &o10, float2 &o11) {
+    fact_combine<LINKED, SIGNED>(hA, hB, hR, hI, pdead, mq, x00, x01, x10, x11, pr, pc, o00, o01, o10, o11);
+  };
+  auto sign = [&](uint32_t i) { return SIGNED ? (__popc(i & sgn) & 1u) << 31 : 0u; };
+  float4 *R4 = reinterpret_cast<float4 *>(R);
+  if (pos == 0) {
+    // H columns of blocks; thread tid: column tid % H, rows tid / H + j * (TPR / H)
+    constexpr int CPT = H < TPR ? H : TPR;  // threads per row of blocks
+    constexpr int RSTEP = TPR / CPT, NJ = (H + RSTEP - 1) / RSTEP;
+    constexpr int U = NJ >= 4 ? 4 : NJ;
+    constexpr bool ALL = NJ * RSTEP == H;  // every row index is in range
+    const uint32_t c = (uint32_t)(tid % CPT), r_first = (uint32_t)(tid / CPT);
+    for (int cc = (int)c; cc < H; cc += CPT) {  // one iteration unless H > TPR
+      const uint32_t pc = sign(2u * (uint32_t)cc);
+      const uint32_t ccs = rsw(2u * (uint32_t)cc) >> 1;  // the column pair's float4 slot in its row
+      for (int j0 = 0; j0 < NJ; j0 += U) {
+        float4 top[U], bot[U];
+        uint32_t at[U], pr[U];
+#pragma unroll
+        for (int uu = 0; uu < U; ++uu) {
+          const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
+          if (ALL || r < (uint32_t)H) {
+            at[uu] = r * D + ccs;  // float4 index of (row 2r, columns 2c, 2c + 1)
+            pr[uu] = sign(2u * r);
+            top[uu] = R4[at[uu]];
+            bot[uu] = R4[at[uu] + D / 2];
+          }
+        }
+#pragma unroll
+        for (int uu = 0; uu < U; ++uu) {
+          const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
+          if (ALL || r < (uint32_t)H) {
+            float2 o00, o01, o10, o11;
+            combine(make_float2(top[uu].x, top[uu].y), make_float2(top[uu].z, top[uu].w),
+                    make_float2(bot[uu].x, bot[uu].y), make_float2(bot[uu].z, bot[uu].w), pr[uu], pc, o00, o01,
+                    o10, o11);
+            R4[at[uu]] = make_float4(o00.x, o00.y, o01.x, o01.y);
+            R4[at[uu] + D / 2] = make_float4(o10.x, o10.y, o11.x, o11.y);
+          }
+        }
+      }
+    }
+  } else if constexpr (W >= 3) {  // window 2 has position 0 only
+    // H/2 column pairs; thread tid: pair tid % HU, rows tid / HU + j * (TPR / HU)
+    constexpr int HU = H / 2;
+    constexpr int CPT = HU < TPR ? HU : TPR;
+    constexpr int RSTEP = TPR / CPT, NJ = (H + RSTEP - 1) / RSTEP;
+    constexpr int U = NJ >= 2 ? 2 : NJ;
+    constexpr bool ALL = NJ * RSTEP == H;
+    const uint32_t rs = ((uint32_t)D << pos) >> 1;  // row step in float4
+    const uint32_t r_first = (uint32_t)(tid / CPT);
+    for (int cp = tid % CPT; cp < HU; cp += CPT) {  // one iteration unless HU > TPR
+      const uint32_t c0 = ins_bit(2u * (uint32_t)cp, pos, 0);  // even
+      const uint32_t pc0 = sign(c0), pc1 = sign(c0 + 1u);
+      // float4 slots of the column pairs (c0, c0 + 1) and (c0 + 2^pos, c0 + 2^pos + 1) in a row
+      const uint32_t s0 = rsw(c0) >> 1, s1 = rsw(c0 | (1u << pos)) >> 1;
+      for (int j0 = 0; j0 < NJ; j0 += U) {
+        float4 q00[U], q01[U], q10[U], q11[U];
+        uint32_t at[U], pr[U];
+#pragma unroll
+        for (int uu = 0; uu < U; ++uu) {
+          const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
+          if (ALL || r < (uint32_t)H) {
+            const uint32_t r0 = ins_bit(r, pos, 0);
+            at[uu] = (r0 * D) >> 1;  // float4 index of row r0
+            pr[uu] = sign(r0);
+            q00[uu] = R4[at[uu] + s0];
+            q01[uu] = R4[at[uu] + s1];
+            q10[uu] = R4[at[uu] + rs + s0];
+            q11[uu] = R4[at[uu] + rs + s1];
+          }
+        }
+#pragma unroll
+        for (int uu = 0; uu < U; ++uu) {
+          const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
+          if (ALL || r < (uint32_t)H) {
+            float2 a00, a01, a10, a11, b00, b01, b10, b11;
+            combine(make_float2(q00[uu].x, q00[uu].y), make_float2(q01[uu].x, q01[uu].y),
+                    make_float2(q10[uu].x, q10[uu].y), make_float2(q11[uu].x, q11[uu].y), pr[uu], pc0, a00, a01,
+                    a10, a11);
+            combine(make_float2(q00[uu].z, q00[uu].w), make_float2(q01[uu].z, q01[uu].w),
+                    make_float2(q10[uu].z, q10[uu].w), make_float2(q11[uu].z, q11[uu].w), pr[uu], pc1, b00, b01,
+                    b10, b11);
+            R4[at[uu] + s0] = make_float4(a00.x, a00.y, b00.x, b00.y);
+            R4[at[uu] + s1] = make_float4(a01.x, a01.y, b01.x, b01.y);
+            R4[at[uu] + rs + s0] = make_float4(a10.x, a10.y, b10.x, b10.y);
+            R4[at[uu] + rs + s1] = make_float4(a11.x, a11.y, b11.x, b11.y);
+          }
+        }
+      }
+    }
   }
 }
 
@@ -225,37 +340,73 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     const bool zstep = (ss.x & kFactZ) != 0u;
     const int pos = (int)(ss.x & 15u);
     const bool mq = (ss.x & kFactMq) != 0u, pdead = (ss.x & kFactDead) != 0u;
-    // 1. outcome probability: trace of the contraction (diagonal blocks)
-    //    step 0: from |psi_0> over bit 0; later: from R over position pos
+    // 1. outcome probability (what = 0): trace of the contraction (diagonal
+    //    blocks), step 0 from |psi_0> over bit 0, later from R over position pos
     //    (with a |+> slot entangled to the measured qubit, the coherences of
-    //    the measured qubit drop out of the trace)
-    float p_re = 0.f, p_off = 0.f, t_re = 0.f;  // sums of G00 x00 + G11 x11, of 2 Re(G01 x01), of the trace
-    if (k == 0) {
-      for (int r = tid; r < DW / 2; r += TPR) {
-        const float2 u0 = psi[2 * r], u1 = psi[2 * r + 1];
-        const float q00 = u0.x * u0.x + u0.y * u0.y, q11 = u1.x * u1.x + u1.y * u1.y;
-        p_re += F.x * q00 + F.y * q11;
-        // x01 = psi0 conj(psi1)
-        p_off += 2.f * (F.z * (u0.x * u1.x + u0.y * u1.y) - F.w * (u0.y * u1.x - u0.x * u1.y));
-        t_re += q00 + q11;
-      }
-    } else {
-      for (int r = tid; r < H; r += TPR) {
-        const uint32_t i0 = ins_bit(r, pos, 0), i1 = ins_bit(r, pos, 1);
-        const float2 q00 = R[i0 * D + rsw(i0)], q11 = R[i1 * D + rsw(i1)], q01 = R[i0 * D + rsw(i1)];
-        p_re += F.x * q00.x + F.y * q11.x;
-        p_off += 2.f * (F.z * q01.x - F.w * q01.y);
-        t_re += q00.x + q11.x;
-      }
-    }
+    //    the measured qubit drop out of the trace).  what = 1: the trace, 2:
+    //    prob1 = trace - prob0 term by term.  One warp reads and sums the
+    //    diagonal; the barrier that hands the sum on also says that it was read.
     const bool drop_coh = k > 0 && !pdead && mq;
-    float2 prob = group_sum2_db<TPR>(drop_coh ? p_re : p_re + p_off, sRed, tid, group, red_par);
+    auto diagonal = [&](int what) -> float2 {
+      if (k == 0) {
+        float p_re = 0.f, p_off = 0.f, t_re = 0.f;  // sums of G00 x00 + G11 x11, of 2 Re(G01 x01), of the trace
+        for (int r = tid; r < DW / 2; r += TPR) {
+          const float2 u0 = psi[2 * r], u1 = psi[2 * r + 1];
+          const float q00 = u0.x * u0.x + u0.y * u0.y, q11 = u1.x * u1.x + u1.y * u1.y;
+          p_re += F.x * q00 + F.y * q11;
+          // x01 = psi0 conj(psi1)
+          p_off += 2.f * (F.z * (u0.x * u1.x + u0.y * u1.y) - F.w * (u0.y * u1.x - u0.x * u1.y));
+          t_re += q00 + q11;
+        }
+        return group_sum2_db<TPR>(what == 0 ? p_re + p_off : what == 1 ? t_re : tr_noise * t_re - p_re - p_off, sRed,
+                                  tid, group, red_par);
+      }
+      constexpr int L = H < 32 ? H : 32;  // lanes with a term of their own (the others repeat them)
+      float hi = 0.f, lo = 0.f;
+      if (tid < 32) {
+#pragma unroll
+        for (int r = tid & (L - 1), n = 0; n < H / L; r += L, ++n) {
+          const uint32_t i0 = ins_bit(r, pos, 0), i1 = i0 | (1u << pos);
+          const float2 q00 = R[i0 * D + rsw(i0)], q11 = R[i1 * D + rsw(i1)];
+          const float p_re = F.x * q00.x + F.y * q11.x, t_re = q00.x + q11.x;
+          float v;
+          if (what == 1) {
+            v = t_re;
+          } else if (drop_coh) {
+            v = what == 0 ? p_re : tr_noise * t_re - p_re;
+          } else {
+            const float2 q01 = R[i0 * D + rsw(i1)];
+            const float p_off = 2.f * (F.z * q01.x - F.w * q01.y);
+            v = what == 0 ? p_re + p_off : tr_noise * t_re - p_re - p_off;
+          }
+          two_sum_acc(hi, lo, v, 0.f);
+        }
+#pragma unroll
+        for (int o = L / 2; o >= 1; o >>= 1) {
+          const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+          const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+          two_sum_acc(hi, lo, oh, ol);
+        }
+        const float sum = hi + lo;  // renormalise
+        lo = lo - (sum - hi);
+        hi = sum;
+      }
+      if constexpr (TPR > 32) {
+        float2 *buf = sRed + red_par * 32;
+        red_par ^= 1;
+        if (tid == 0) *buf = make_float2(hi, lo);
+        group_sync(TPR, group);
+        return *buf;
+      }
+      return make_float2(hi, lo);
+    };
+    float2 prob = diagonal(0);
     float4 G = F;
     int outcome = 0;
     bool take1 = false;
     bool unprojected = false;
     if (zstep) {
-      const float2 tot = group_sum2_db<TPR>(t_re, sRed, tid, group, red_par);
+      const float2 tot = diagonal(1);
       if (A.flags & MBQC_F_DM_EXPECTATION) {
         if (tid == 0) sF[k] = make_float4(prob.x, prob.y, tot.x, tot.y);
         G = make_float4(1.f, 1.f, 0.f, 0.f);
@@ -270,9 +421,7 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     }
     if (take1) {  // outcome 1 with P1 = I - P0
       G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
-      // prob1 = trace - prob0 term by term: the same sums with G
-      const float p1 = drop_coh ? (tr_noise * t_re - p_re) : (tr_noise * t_re - p_re - p_off);
-      const float2 prob1 = group_sum2_db<TPR>(p1, sRed, tid, group, red_par);
+      const float2 prob1 = diagonal(2);
       if (tid == 0) sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
       prob = prob1;
       outcome = 1;
@@ -310,106 +459,21 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     // probability sum above follows each thread's reads (a warp-sized group
     // syncs here)
     if constexpr (TPR == 32) group_sync(TPR, group);
-    // 2. one in-place pass over the 2x2 blocks of position pos, the scale
-    //    folded into the functional.  16-byte shared-memory accesses: at pos
-    //    0 a block's two columns are adjacent (one float4 per row); at pos > 0
-    //    a unit is the two blocks of columns c0 and c0 + 1 (one float4 per
-    //    row and column half).  A thread keeps one column (pair) for the
-    //    whole pass and walks rows, so its column index, signs and the
-    //    row-independent address parts are computed once; all loads of U
-    //    units before their stores (distinct units never alias).
+    // 2. the pass, the scale folded into the functional.  Slots of circuits
+    //    with a causal flow are linked to the measured qubit, and on wires to no
+    //    other: those passes are straight-line code without sign operations
+    //    (the general one spent ~460 of its 770 warp instructions a step beside
+    //    the arithmetic)
     const uint32_t sgn = ss.y;
     const float half = pdead ? inv : 0.5f * inv;
     const float hA = g00 * half, hB = g11 * half, hR = gr * half, hI = gi * half;
-    auto combine = [&](float2 x00, float2 x01, float2 x10, float2 x11, uint32_t pr, uint32_t pc, float2 &o00,
-                       float2 &o01, float2 &o10, float2 &o11) {
-      fact_combine(hA, hB, hR, hI, pdead, mq, x00, x01, x10, x11, pr, pc, o00, o01, o10, o11);
-    };
-    float4 *R4 = reinterpret_cast<float4 *>(R);
-    if (pos == 0) {
-      // H columns of blocks; thread tid: column tid % H, rows tid / H + j * (TPR / H)
-      constexpr int CPT = H < TPR ? H : TPR;  // threads per row of blocks
-      constexpr int RSTEP = TPR / CPT, NJ = (H + RSTEP - 1) / RSTEP;
-      constexpr int U = NJ >= 4 ? 4 : NJ;
-      const uint32_t c = (uint32_t)(tid % CPT), r_first = (uint32_t)(tid / CPT);
-      for (int cc = (int)c; cc < H; cc += CPT) {  // one iteration unless H > TPR
-        const uint32_t pc = (__popc((2u * (uint32_t)cc) & sgn) & 1u) << 31;
-        const uint32_t ccs = rsw(2u * (uint32_t)cc) >> 1;  // the column pair's float4 slot in its row
-        for (int j0 = 0; j0 < NJ; j0 += U) {
-          float4 top[U], bot[U];
-          uint32_t at[U], pr[U];
-#pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
-            if (r < (uint32_t)H) {
-              at[uu] = r * D + ccs;  // float4 index of (row 2r, columns 2c, 2c + 1)
-              pr[uu] = (__popc((2u * r) & sgn) & 1u) << 31;
-              top[uu] = R4[at[uu]];
-              bot[uu] = R4[at[uu] + D / 2];
-            }
-          }
-#pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
-            if (r < (uint32_t)H) {
-              float2 o00, o01, o10, o11;
-              combine(make_float2(top[uu].x, top[uu].y), make_float2(top[uu].z, top[uu].w),
-                      make_float2(bot[uu].x, bot[uu].y), make_float2(bot[uu].z, bot[uu].w), pr[uu], pc, o00, o01,
-                      o10, o11);
-              R4[at[uu]] = make_float4(o00.x, o00.y, o01.x, o01.y);
-              R4[at[uu] + D / 2] = make_float4(o10.x, o10.y, o11.x, o11.y);
-            }
-          }
-        }
-      }
-    } else if constexpr (W >= 3) {  // window 2 has position 0 only
-      // H/2 column pairs; thread tid: pair tid % HU, rows tid / HU + j * (TPR / HU)
-      constexpr int HU = H / 2;
-      constexpr int CPT = HU < TPR ? HU : TPR;
-      constexpr int RSTEP = TPR / CPT, NJ = (H + RSTEP - 1) / RSTEP;
-      constexpr int U = NJ >= 2 ? 2 : NJ;
-      const uint32_t rs = ((uint32_t)D << pos) >> 1;  // row step in float4
-      const uint32_t r_first = (uint32_t)(tid / CPT);
-      for (int cp = tid % CPT; cp < HU; cp += CPT) {  // one iteration unless HU > TPR
-        const uint32_t c0 = ins_bit(2u * (uint32_t)cp, pos, 0);  // even
-        const uint32_t pc0 = (__popc(c0 & sgn) & 1u) << 31, pc1 = (__popc((c0 + 1u) & sgn) & 1u) << 31;
-        // float4 slots of the column pairs (c0, c0 + 1) and (c0 + 2^pos, c0 + 2^pos + 1) in a row
-        const uint32_t s0 = rsw(c0) >> 1, s1 = rsw(c0 | (1u << pos)) >> 1;
-        for (int j0 = 0; j0 < NJ; j0 += U) {
-          float4 q00[U], q01[U], q10[U], q11[U];
-          uint32_t at[U], pr[U];
-#pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
-            if (r < (uint32_t)H) {
-              const uint32_t r0 = ins_bit(r, pos, 0);
-              at[uu] = (r0 * D) >> 1;  // float4 index of row r0
-              pr[uu] = (__popc(r0 & sgn) & 1u) << 31;
-              q00[uu] = R4[at[uu] + s0];
-              q01[uu] = R4[at[uu] + s1];
-              q10[uu] = R4[at[uu] + rs + s0];
-              q11[uu] = R4[at[uu] + rs + s1];
-            }
-          }
-#pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const uint32_t r = r_first + (uint32_t)(j0 + uu) * RSTEP;
-            if (r < (uint32_t)H) {
-              float2 a00, a01, a10, a11, b00, b01, b10, b11;
-              combine(make_float2(q00[uu].x, q00[uu].y), make_float2(q01[uu].x, q01[uu].y),
-                      make_float2(q10[uu].x, q10[uu].y), make_float2(q11[uu].x, q11[uu].y), pr[uu], pc0, a00, a01,
-                      a10, a11);
-              combine(make_float2(q00[uu].z, q00[uu].w), make_float2(q01[uu].z, q01[uu].w),
-                      make_float2(q10[uu].z, q10[uu].w), make_float2(q11[uu].z, q11[uu].w), pr[uu], pc1, b00, b01,
-                      b10, b11);
-              R4[at[uu] + s0] = make_float4(a00.x, a00.y, b00.x, b00.y);
-              R4[at[uu] + s1] = make_float4(a01.x, a01.y, b01.x, b01.y);
-              R4[at[uu] + rs + s0] = make_float4(a10.x, a10.y, b10.x, b10.y);
-              R4[at[uu] + rs + s1] = make_float4(a11.x, a11.y, b11.x, b11.y);
-            }
-          }
-        }
-      }
+    if (mq && !pdead) {
+      if (sgn == 0u)
+        fact_pass<W, TPR, true, false>(R, tid, pos, hA, hB, hR, hI, pdead, mq, sgn);
+      else
+        fact_pass<W, TPR, true, true>(R, tid, pos, hA, hB, hR, hI, pdead, mq, sgn);
+    } else {
+      fact_pass<W, TPR, false, true>(R, tid, pos, hA, hB, hR, hI, pdead, mq, sgn);
     }
     group_sync(TPR, group);
   }
