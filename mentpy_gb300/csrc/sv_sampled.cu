@@ -10,7 +10,8 @@
 // outcomes (up to a global phase).
 //
 // A group of threads owns one run: a warp for windows <= 10 (four runs per
-// block), the whole block for windows 11..20 (256, 512 or 1024 threads).  The
+// block, sv_sampled_warp), the whole block for windows 11..20 (256, 512 or 1024
+// threads, sv_sampled).  The
 // window sits in shared memory up to w = 14 (128 KB) and in a caller
 // workspace (one 2^w slot per block, the block looping over runs) from 15.
 // Batches smaller than the GPU at w >= 15 share each run among a cluster of
@@ -84,14 +85,6 @@ __device__ __forceinline__ uint32_t insert_bit(uint32_t r, int p, uint32_t b) {
   return ((r >> p) << (p + 1)) | (b << p) | (r & ((1u << p) - 1u));
 }
 
-template <int TPR>
-__device__ __forceinline__ void group_barrier() {
-  if constexpr (TPR == 32)
-    __syncwarp();
-  else
-    __syncthreads();
-}
-
 // Sum of three per-thread values over the group, the same bits in every
 // thread (a butterfly, then the warps' partials in a fixed order).
 template <int TPR>
@@ -121,26 +114,17 @@ __device__ __forceinline__ void group_sum3(float &a, float &b, float &c, float *
   }
 }
 
-// the end of a step or a run: the group's barrier, or the cluster's
-template <int TPR, int CS>
-__device__ __forceinline__ void sampled_barrier() {
-  if constexpr (CS > 1)
-    run_barrier<CS>();
-  else
-    group_barrier<TPR>();
-}
-
 template <int W, int CS>
 __global__ void __launch_bounds__(SampledCfg<W>::kBlock) sv_sampled(SampledArgs a) {
   using Cfg = SampledCfg<W>;
   constexpr int D = 1 << W, TPR = Cfg::TPR;
-  static_assert(CS == 1 || (Cfg::kWs && TPR > 32), "clusters share a run only with the window in the workspace");
+  static_assert(TPR > 32, "windows 11 and up: the block owns the run");
+  static_assert(CS == 1 || Cfg::kWs, "clusters share a run only with the window in the workspace");
   constexpr int QS = D / 2 / CS, DS = D / CS;  // this block's pairs / window entries of a pass
   __shared__ float cred[8];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
-  const int tid = TPR == 32 ? lane : (int)threadIdx.x;
-  const int G = blockDim.x / TPR, g = threadIdx.x / TPR;
+  const int tid = (int)threadIdx.x;
   const int M = a.M, FW = (M + 31) >> 5;
   int crank = 0, cid = blockIdx.x, ncl = gridDim.x, cpar = 0;
   if constexpr (CS > 1) {
@@ -149,14 +133,13 @@ __global__ void __launch_bounds__(SampledCfg<W>::kBlock) sv_sampled(SampledArgs 
     ncl = gridDim.x / CS;
   }
   const int q_lo = crank * QS, i_lo = crank * DS;
-  unsigned char *base = smem_raw + (size_t)g * a.group_bytes;
+  unsigned char *base = smem_raw;
   float2 *s = Cfg::kWs ? a.ws + (size_t)cid * D : reinterpret_cast<float2 *>(base);
   uint32_t *fx = reinterpret_cast<uint32_t *>(base + (Cfg::kWs ? 0 : (size_t)D * sizeof(float2)));
   uint32_t *fz = fx + FW;
   float *red = reinterpret_cast<float *>(fz + FW);
 
-  // G == 1 whenever TPR > 32, so the block-wide barriers see the same trip count
-  for (int64_t run = (int64_t)cid * G + g; run < a.B; run += (int64_t)ncl * G) {
+  for (int64_t run = cid; run < a.B; run += ncl) {
     for (int i = tid; i < 2 * FW; i += TPR) fx[i] = 0u;
     const float2 *in = a.psi_in + (a.istride ? run * a.istride : 0);
     for (int i = i_lo + tid; i < i_lo + DS; i += TPR) {
@@ -168,7 +151,7 @@ __global__ void __launch_bounds__(SampledCfg<W>::kBlock) sv_sampled(SampledArgs 
                          init_parity((uint32_t)i, a.init_cz, W) << 31);
       }
     }
-    sampled_barrier<TPR, CS>();
+    run_barrier<CS>();
 
     uint32_t xo = 0, zo = 0;  // pending X / Z on the outputs
     int32_t code = MBQC_RUN_OK;
@@ -240,7 +223,7 @@ __global__ void __launch_bounds__(SampledCfg<W>::kBlock) sv_sampled(SampledArgs 
         zo ^= a.z_out[k];
       }
       if (tid == 0 && crank == 0 && a.outcomes) a.outcomes[run * a.ostride + k] = (int8_t)m;
-      sampled_barrier<TPR, CS>();
+      run_barrier<CS>();
     }
     const int dout = 1 << a.n_out;
     float2 *out = a.psi_out + run * dout;
@@ -253,7 +236,150 @@ __global__ void __launch_bounds__(SampledCfg<W>::kBlock) sv_sampled(SampledArgs 
       out[yy] = flip_sign(v, (uint32_t)(__popc(yy & zo) & 1u) << 31);  // then Z signs
     }
     if (tid == 0 && crank == 0 && a.status) a.status[run] = code;
-    sampled_barrier<TPR, CS>();  // the next run overwrites the window and the frame
+    run_barrier<CS>();  // the next run overwrites the window and the frame
+  }
+}
+
+// Windows <= 10: a warp per run.  The step's chain is what bounds it (66 steps
+// in turn, each a sum over the warp, a draw and an update), so only what depends
+// on the previous step is on it: the pairs stay in registers between the weight
+// sums and the update, and a lane makes, for one of the next 32 steps, the
+// coefficient, the uniform draw and the byproduct targets; a step takes them by
+// shuffle.  Outcomes leave 32 at a time.  500 runs of many_wires 6x12 (w = 7, 66
+// steps): 56.2 us with the block kernel's code on one warp (which read the
+// window twice a step and met the byproduct lists and two 64-bit hashes on the
+// chain), 39.5 us (host-bound).  The sums are taken in that code's order: the same draws.
+template <int W>
+__global__ void __launch_bounds__(128) sv_sampled_warp(SampledArgs a) {
+  constexpr int D = 1 << W, QS = D / 2, NIT = QS > 32 ? QS / 32 : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31;
+  const int G = blockDim.x / 32, g = threadIdx.x / 32;
+  const int M = a.M, FW = (M + 31) >> 5;
+  unsigned char *base = smem_raw + (size_t)g * a.group_bytes;
+  float2 *s = reinterpret_cast<float2 *>(base);
+  uint32_t *fx = reinterpret_cast<uint32_t *>(base + (size_t)D * sizeof(float2));
+  uint32_t *fz = fx + FW;
+  const bool live = QS >= 32 || lane < QS;
+
+  for (int64_t run = (int64_t)blockIdx.x * G + g; run < a.B; run += (int64_t)gridDim.x * G) {
+    for (int i = lane; i < 2 * FW; i += 32) fx[i] = 0u;
+    const float2 *in = a.psi_in + (a.istride ? run * a.istride : 0);
+    for (int i = lane; i < D; i += 32) {
+      const int2 m = a.map[i];
+      s[i] = flip_sign(in[m.x & 0x7fffffff], (uint32_t)m.x & 0x80000000u);
+    }
+    __syncwarp();
+
+    uint32_t xo = 0, zo = 0;  // pending X / Z on the outputs
+    int32_t code = MBQC_RUN_OK;
+    float2 creg = make_float2(0.f, 0.f);  // this lane's step of the current 32
+    uint32_t mreg = 0u, xoreg = 0u, zoreg = 0u, wx = 0u, wz = 0u;
+    int xsreg = -1, zbreg = 0, znreg = 0, zi0 = -1, zi1 = -1, oreg = 0;
+    float ureg = 0.f;
+    int p = 0;
+    for (int k = 0; k < M; ++k, p = p + 1 == W ? 0 : p + 1) {
+      const int kl = k & 31;
+      if (kl == 0) {
+        if (k + lane < M) {
+          const int kk = k + lane;
+          const DevStep st = a.steps[kk];
+          const double th = st.aidx >= 0 ? a.angles[run * a.astride + st.aidx] : st.fixed;
+          float2 ph;
+          sv_coef(st.plane, th, false, creg, ph);
+          mreg = st.mask;
+          const uint64_t h = sm64(a.seed ^ sm64(((uint64_t)run << 20) ^ (uint64_t)kk));
+          ureg = (float)(h >> 40) * 5.9604644775390625e-08f;
+          xsreg = a.x_step[kk];
+          zbreg = a.z_off[kk];
+          znreg = a.z_off[kk + 1] - zbreg;
+          zi0 = znreg > 0 ? a.z_idx[zbreg] : -1;
+          zi1 = znreg > 1 ? a.z_idx[zbreg + 1] : -1;
+          xoreg = a.x_out[kk];
+          zoreg = a.z_out[kk];
+        }
+        __syncwarp();
+        wx = fx[k >> 5];
+        wz = fz[k >> 5];
+      }
+      float2 c = make_float2(__shfl_sync(0xffffffffu, creg.x, kl), __shfl_sync(0xffffffffu, creg.y, kl));
+      const uint32_t mask = __shfl_sync(0xffffffffu, mreg, kl);
+      const float u01 = __shfl_sync(0xffffffffu, ureg, kl);
+      const bool dead = (mask & kDead) != 0u;
+      if ((wx >> kl) & 1u) c.y = -c.y;                    // X: angle -> -angle
+      if ((wz >> kl) & 1u) c = make_float2(-c.x, -c.y);  // Z: angle -> angle + pi
+      // branch weights
+      float2 u[NIT], v[NIT];
+      float sr = 0.f, si = 0.f, t = 0.f;
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) {
+        u[n] = v[n] = make_float2(0.f, 0.f);
+        if (live) {
+          const uint32_t i0 = insert_bit((uint32_t)(lane + 32 * n), p, 0u);
+          u[n] = s[i0];
+          v[n] = s[i0 | (1u << p)];
+        }
+        sr += u[n].x * v[n].x + u[n].y * v[n].y;
+        si += u[n].x * v[n].y - u[n].y * v[n].x;
+        t += u[n].x * u[n].x + u[n].y * u[n].y + v[n].x * v[n].x + v[n].y * v[n].y;
+      }
+      group_sum3<32>(sr, si, t, nullptr);
+      const float re = c.x * sr - c.y * si;  // Re(c S)
+      const float n0 = t + 2.f * re, n1 = t - 2.f * re;
+      const int m = (u01 * (n0 + n1) >= n0) ? 1 : 0;
+      const float nm = m ? n1 : n0;
+      if (!(nm > 0.f) || isnan(nm) || isinf(nm)) {  // the same value in every lane
+        code = isnan(nm) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM;
+        if (a.outcomes && lane < kl) a.outcomes[run * a.ostride + (k - kl) + lane] = (int8_t)oreg;
+        break;
+      }
+      const float gn = rsqrtf(dead ? nm : 2.f * nm);
+      const float2 ce = m ? make_float2(-c.x, -c.y) : c;
+      if (live) {
+#pragma unroll
+        for (int n = 0; n < NIT; ++n) {
+          const uint32_t i0 = insert_bit((uint32_t)(lane + 32 * n), p, 0u), i1 = i0 | (1u << p);
+          const float2 phi = make_float2(gn * (u[n].x + ce.x * v[n].x - ce.y * v[n].y),
+                                         gn * (u[n].y + ce.x * v[n].y + ce.y * v[n].x));
+          s[i0] = phi;
+          s[i1] = dead ? make_float2(0.f, 0.f) : flip_sign(phi, (uint32_t)(__popc(i1 & mask) & 1u) << 31);
+        }
+      }
+      if (m) {  // byproducts of outcome 1 go to later steps only (checked on the host; skipped here otherwise)
+        const int xt = __shfl_sync(0xffffffffu, xsreg, kl);
+        const int zn = __shfl_sync(0xffffffffu, znreg, kl), zb = __shfl_sync(0xffffffffu, zbreg, kl);
+        const int z0 = __shfl_sync(0xffffffffu, zi0, kl), z1 = __shfl_sync(0xffffffffu, zi1, kl);
+        xo ^= __shfl_sync(0xffffffffu, xoreg, kl);
+        zo ^= __shfl_sync(0xffffffffu, zoreg, kl);
+        // a step of these 32: in the lanes' words; a later one: lane 0 in the bitset
+        auto flip = [&](uint32_t *f, uint32_t &w, int st) {
+          if (st <= k || st >= M) return;
+          if ((st >> 5) == (k >> 5))
+            w ^= 1u << (st & 31);
+          else if (lane == 0)
+            f[st >> 5] ^= 1u << (st & 31);
+        };
+        flip(fx, wx, xt);
+        if (zn > 0) flip(fz, wz, z0);
+        if (zn > 1) flip(fz, wz, z1);
+        for (int j = 2; j < zn; ++j) flip(fz, wz, a.z_idx[zb + j]);
+      }
+      if (lane == kl) oreg = m;
+      if (a.outcomes && (kl == 31 || k + 1 == M) && lane <= kl)
+        a.outcomes[run * a.ostride + (k - kl) + lane] = (int8_t)oreg;
+      __syncwarp();
+    }
+    const int dout = 1 << a.n_out;
+    float2 *out = a.psi_out + run * dout;
+    for (int i = lane; i < D; i += 32) {
+      const int y = a.map[i].y;
+      if (y < 0) continue;
+      const uint32_t yy = (uint32_t)y ^ xo;  // X on the outputs permutes the index
+      const float2 w = code == MBQC_RUN_OK ? s[i] : make_float2(NAN, NAN);
+      out[yy] = flip_sign(w, (uint32_t)(__popc(yy & zo) & 1u) << 31);  // then Z signs
+    }
+    if (lane == 0 && a.status) a.status[run] = code;
+    __syncwarp();  // the next run overwrites the window and the frame
   }
 }
 
@@ -292,6 +418,14 @@ static int sampled_cluster_launch(const SampledArgs &a, int runs, size_t smem, c
 }
 
 template <int W>
+static auto sampled_kernel() {
+  if constexpr (SampledCfg<W>::TPR == 32)
+    return &sv_sampled_warp<W>;
+  else
+    return &sv_sampled<W, 1>;
+}
+
+template <int W>
 static int launch_sampled(SampledArgs a, size_t ws_bytes, cudaStream_t s) {
   using Cfg = SampledCfg<W>;
   const int fw = (a.M + 31) >> 5;
@@ -324,7 +458,7 @@ static int launch_sampled(SampledArgs a, size_t ws_bytes, cudaStream_t s) {
   if (blocks > 0x7fffffff / 4) blocks = 0x7fffffff / 4;  // the blocks loop over the remaining runs
   if (cs == 4) return sampled_cluster_launch<W, 4>(a, (int)blocks, G * gb, s);
   if (cs == 2) return sampled_cluster_launch<W, 2>(a, (int)blocks, G * gb, s);
-  auto k = sv_sampled<W, 1>;
+  auto k = sampled_kernel<W>();
   rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(G * gb)),
                   "sampled smem attribute");
   if (rc) return rc;
