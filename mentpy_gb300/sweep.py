@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .plan import WindowPlan, compile_plan
+from .plan import PLANE_CODES, WindowPlan, compile_plan
 
 
 _TUNED = {}  # (window, steps, n_in, n_out, batch bucket) -> fastest register-kernel variant
@@ -34,8 +34,10 @@ def gpu_hold(us: float = 2000.0) -> None:
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> ctypes.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    # the current stream's handle without building a Stream object (~3 us)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
@@ -70,6 +72,9 @@ def as_device(x, dtype, device) -> torch.Tensor:
     (lazy conjugate / negative views are materialised: the kernels read raw
     memory)."""
     if isinstance(x, torch.Tensor):
+        if (x.dtype == dtype and x.device == device and x.is_contiguous() and not x.is_neg()
+                and not (x.is_complex() and x.is_conj())):
+            return x  # the usual case: nothing to convert
         t = x.to(device=device, dtype=dtype)
         if t.is_complex():
             t = t.resolve_conj()
@@ -351,14 +356,30 @@ class StatevectorSweep:
 
     # ------------------------------------------------------------ adjoint
     def _workspace(self, runs: int) -> torch.Tensor:
-        f64 = 1 if self.dtype == torch.complex128 else 0
-        n = ctypes.c_size_t()
-        _native.check(_native.lib().mbqc_sv_adjoint_workspace(self.dplan.handle, runs, f64, ctypes.byref(n)))
+        need = getattr(self, "_ws_need", None)  # (runs, bytes) of the last call
+        if need is None or need[0] != runs:
+            f64 = 1 if self.dtype == torch.complex128 else 0
+            n = ctypes.c_size_t()
+            _native.check(_native.lib().mbqc_sv_adjoint_workspace(self.dplan.handle, runs, f64, ctypes.byref(n)))
+            need = self._ws_need = (runs, n.value)
         ws = getattr(self, "_ws", None)
-        if ws is None or ws.numel() < n.value:
-            ws = torch.empty(max(n.value, 16), dtype=torch.uint8, device=self.device)
+        if ws is None or ws.numel() < need[1]:
+            ws = torch.empty(max(need[1], 16), dtype=torch.uint8, device=self.device)
             self._ws = ws
         return ws
+
+    def _every_angle_written(self) -> bool:
+        """Whether the adjoint writes the gradient of every angle: the register
+        kernels (windows up to 8 in XY, X and Y) always do, the block-per-run
+        kernels write the angles that some step uses."""
+        v = getattr(self, "_all_written", None)
+        if v is None:
+            p = self.plan
+            planes = np.asarray(p.step_plane)
+            v = (p.window <= 8 and not (planes > PLANE_CODES["Y"]).any()) or (
+                len(set(np.asarray(p.step_angle).tolist()) - {-1}) == self.n_angles)
+            self._all_written = v
+        return v
 
     def adjoint(self, angles, inputs, grad_out, *, status: Optional[torch.Tensor] = None, stream=None):
         """dL/dangles [B, A] (float64) for dL = Re sum conj(grad_out) dz, where
@@ -374,13 +395,14 @@ class StatevectorSweep:
         g = as_device(grad_out, self.dtype, self.device)
         if g.shape != (B, 2 ** self.n_out):
             raise ValueError(f"grad_out must have shape {(B, 2 ** self.n_out)}")
-        # zeros: the block-per-run kernels (windows above 8, XZ / YZ plans)
-        # write only the angles that some step uses, and an angle no step
-        # uses (a trainable node that is never measured) has derivative 0
-        grad = torch.zeros((B, self.n_angles), dtype=torch.float64, device=self.device)
+        # an angle no step uses (a trainable node that is never measured) has
+        # derivative 0: filled in where the kernel does not write it
+        written = self._every_angle_written()
+        make = torch.empty if written else torch.zeros
+        grad = make((B, self.n_angles), dtype=torch.float64, device=self.device)
         if B == 0:
             return grad
-        if stream is not None:
+        if stream is not None and not written:
             stream.wait_stream(torch.cuda.current_stream(self.device))  # the zeros before the kernel
         ws = self._workspace(B)
         fn = _native.lib().mbqc_sv_adjoint if self.dtype == torch.complex64 else _native.lib().mbqc_sv_adjoint_f64
