@@ -82,6 +82,13 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
     else if (runs * 2 <= sms)
       g.wg.cluster = 2;
   }
+  // the rest of a block's shared memory holds what it can of its slice of the
+  // window; at one 512-thread block an SM (its registers) that costs no occupancy
+  g.wg.res = 0;
+  if (hc.w > 14) {
+    g.wg.res = wide_adj_resident(hc.w, hc.n_steps, g.gen, g.wg.cluster, (size_t)optin - 1024);
+    g.smem += (size_t)g.wg.res * 8192;
+  }
   int64_t blocks = g.wg.cluster > 1 ? (int64_t)sm_count() / g.wg.cluster : (int64_t)sm_count() * occ;
   if (runs < blocks) blocks = runs;
   const int64_t cap = (int64_t)(kWideAdjMaxWorkspace / ((size_t)slot * 8));

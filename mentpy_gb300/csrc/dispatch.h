@@ -69,6 +69,7 @@ struct WideAdjGeom {
   uint32_t out_mask;
   int64_t slot_elems;  // complex64 elements of one run slot of the workspace
   int cluster;         // blocks sharing a run (1, 2 or 4; windows >= 15 only)
+  int res;             // 1,024-entry pieces of a block's slice of the window in its shared memory (windows >= 15)
 };
 constexpr int kWideAdjMaxWindow = 20;
 constexpr size_t kWideAdjMaxWorkspace = (size_t)16 << 30;
@@ -76,6 +77,7 @@ constexpr size_t kWideAdjMaxWorkspace = (size_t)16 << 30;
 int launch_sv_adj_wide(const SvAdjArgs &a, const WideAdjGeom &g, const AdjLaunch &l, cudaStream_t s, bool gen);
 int wide_adj_threads(int w);
 size_t wide_adj_smem(int w, int M, bool gen);
+int wide_adj_resident(int w, int M, bool gen, int cluster, size_t limit);
 
 int sm_count();
 
