@@ -39,7 +39,7 @@ struct AdjGeometry {
 
 // Windows 9..20: one block per run slot (a cluster of 2 or 4 blocks for
 // windows above 14 when the batch leaves SMs idle); each slot holds the
-// pre-step half-state of every step (and the window itself above w = 14), and
+// history of every step (and the window itself above w = 14), and
 // the slot count is capped by the blocks resident on the GPU and by
 // kWideAdjMaxWorkspace.
 static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGeometry &g) {
@@ -49,6 +49,7 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
                  : fail(MBQC_E_UNSUPPORTED, "FP64 adjoint: window %d > %d", hc.w, kAdjMaxWindow);
   if (hc.w > kWideAdjMaxWindow)
     return fail(MBQC_E_UNSUPPORTED, "adjoint: window %d > %d", hc.w, kWideAdjMaxWindow);
+  g.gen = g.gen || hc.n_steps == 0;  // no step: nothing of the window is a copy
   g.wide = true;
   g.rpw = 1;
   g.periods = 0;
@@ -66,11 +67,12 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
   SvAdjArgs dummy{};
   dummy.W = hc.w;
   g.wg.cluster = 1;
+  g.wg.res = 0;
   rc = launch_sv_adj_wide(dummy, g.wg, q, nullptr, g.gen);
   if (rc) return rc;
   if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "adjoint: kernel does not fit on an SM");
   const int64_t D = (int64_t)1 << hc.w;
-  const int64_t slot = (hc.w > 14 ? D : 0) + (int64_t)hc.n_steps * (g.gen ? D : D / 2);
+  const int64_t slot = (hc.w > 14 ? D : 0) + (g.gen ? hc.n_steps * D : (hc.n_steps + 1) * (D / 4));
   // a batch smaller than the GPU: runs of a window in the workspace are
   // shared by a cluster of 2 or 4 blocks (one block per SM), so that more SMs
   // work on them; blocks below counts run slots (clusters)
@@ -84,7 +86,6 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
   }
   // the rest of a block's shared memory holds what it can of its slice of the
   // window; at one 512-thread block an SM (its registers) that costs no occupancy
-  g.wg.res = 0;
   if (hc.w > 14) {
     g.wg.res = wide_adj_resident(hc.w, hc.n_steps, g.gen, g.wg.cluster, (size_t)optin - 1024);
     g.smem += (size_t)g.wg.res * 8192;

@@ -11,10 +11,10 @@
 //   lambda_{k-1}[r, 0] = alpha_k mu[r],  lambda_{k-1}[r, 1] = alpha_k conj(c_k) mu[r].
 //
 // The window does not fit in registers here, so the block keeps it in shared
-// memory (w <= 14) or in its workspace slot (w >= 15).  The forward pass writes the pre-step
-// half-state u_{k-1}[., 1] of every step to the slot's history (2^(w-1)
-// complex64 per step) and the backward pass reads it back: one forward, one
-// backward, no recompute.  The grid is persistent (a workspace slot per
+// memory (w <= 14) or in its workspace slot (w >= 15).  The forward pass writes
+// what it needs of the pre-step half-state u_{k-1}[., 1] of every step to the
+// slot's history and the backward pass reads it back: one forward, one backward,
+// no recompute.  The grid is persistent (a workspace slot per
 // block); the slot count is capped so the workspace stays within
 // kWideAdjMaxWorkspace.  Block sums (norms, <z|g>, the gradient terms) are a
 // butterfly per warp, then the warps' partials in a fixed order, so every
@@ -334,53 +334,79 @@ __global__ void __launch_bounds__(WideAdjCfg<W>::TPR) sv_adj_wide_gen(SvAdjArgs 
   }
 }
 
-// XY, X and Y plans, windows 9..20.  A block's TPR threads of the chain's sums
-// are its BT = TPR / 2 threads, each two of them: a thread takes the pairs q and
-// q + 1 (q even) of every TPR, so the window and the history move in 16-byte
-// accesses and an address, a sign parity and a residency test serve two pairs.
+// XY, X and Y plans, windows 9..20.  After step k the window is phi_k and its
+// signed copy on the entering qubit's bit (or zero), so only phi_k's N = 2^(w-1)
+// amplitudes are kept: index q = the window index without bit p_k = k mod w.
+// Step k reads phi_{k-1}: a (measured bit 0) and b (1) give the two halves
+//   phi_k[entered bit 0] = a + c b,   phi_k[entered bit 1] = s (a + s' c b),
+// s the sign of the entered qubit's CZs, s' = -1 where one of them is with the
+// measured qubit: a pair of slots that differ in bit p - 1 of q, in place.  At
+// p = 0 (the removed bit moves from w - 1 to 0) the slots move: that step reads
+// the window and writes its scratch copy, the next reads that and writes back.
+// The history of a step is b alone (N / 2); lambda is kept the same way
+// (lambda[., 1] = conj(c) lambda[., 0]): pairs on bit p, w - 1 the step that moves.
 //
-// What bounds it at w = 17 (64 runs of the 16 x 10 grid, a cluster of two blocks
-// a run) is the traffic between the L2 and the SMs, ~6 TB/s:
-//   * two forward steps a pass where both pair entries of the block's slice: the
-//     window moves once for both, one barrier.  The second step takes no scale
-//     of its own (scales are exact powers of two: the results keep their bits);
-//     the last step's norm is a result, so that step is a pass of its own;
-//   * what fits of the slice stays in the block's shared memory (at(): 27 of 64
-//     pieces of 1,024 entries), the rest in the slot.  Steps on the top bits of
-//     a shared run pair entries of two blocks through distributed shared memory;
-//   * the gradient's FP64 products are made for all steps at the run's end.
-// One pair a thread and step at a time, the window of w >= 15 in the slot, against
-// this (10 columns): w = 17, 64 runs 5.91 -> 4.98 ms; w = 15, 60 runs 1.37 -> 0.87;
-// w = 12, 512 runs 1.09 -> 0.60; w = 10, 1,024 runs 0.35 -> 0.21 ms.
-// The sums keep that kernel's order (its threads' pairs by n, a warp's lanes as
-// a butterfly, the warps in turn, the cluster's blocks in turn): the same bits.
-template <int W, int CS> struct WideVecCfg {
-  static constexpr int D = 1 << W;
-  static constexpr int TPR = W <= 9 ? 128 : (W == 10 ? 256 : (W == 11 ? 512 : 1024));
-  static constexpr int BT = TPR / 2, VW = TPR / 32;
+// What bounds it at w = 17 (64 runs of the 16 x 10 grid, two blocks a run) is
+// issue at four warps a scheduler: 53 % of the slots, DRAM at a quarter of its
+// rate (the history).  Keeping both halves it was the traffic between the L2 and
+// the SMs: w = 17, 64 runs 4.98 -> 2.76 ms; w = 15, 256 runs 2.80 -> 2.02; w = 19,
+// 32 runs of 18 x 6 9.44 -> 4.72 ms.  The block keeps its slice of the window in shared memory as far as it
+// fits (RES: all of it); the forward pass takes up to three steps at a time on
+// pairs inside the slice; a step on the bits that join slices pairs entries of
+// two blocks through distributed shared memory.
+//
+// The gradient's sums are those of TPR = 2 BT threads, thread v taking the q =
+// v mod TPR in turn.  A backward step on a bit below log2 TPR gives a thread two
+// of those (insert_bit(tid, p) and its partner); a step above it updates lambda
+// first and then sums over q in order (tid: v = 2 tid and 2 tid + 1).
+template <int W, int CS> struct WideHalfCfg {
+  static constexpr int D = 1 << W, N = D / 2, NS = N / CS;
+  static constexpr int LT = W <= 9 ? 7 : (W == 10 ? 8 : (W == 11 ? 9 : 10));
+  static constexpr int TPR = 1 << LT, BT = TPR / 2, VW = TPR / 32;
   static constexpr bool kWs = W > 14;
-  static constexpr int QS = D / 2 / CS, DS = D / CS, NIT = QS / TPR;
-  static constexpr int U = kWs ? (NIT < 4 ? NIT : 4) : 2;  // items in flight
   static constexpr int LOGCS = CS == 4 ? 2 : (CS == 2 ? 1 : 0);
-  static constexpr int MINB = kWs ? 1 : 1024 / BT;
-  static_assert(W >= 9 && QS % TPR == 0 && NIT % U == 0 && NIT >= 2, "pairs per thread");
+  static constexpr int SB = W - 1 - LOGCS;  // index bits of a block's slice
+  static constexpr int FMAX = SB - LT + 1 < 3 ? SB - LT + 1 : 3;
+  static constexpr int MINB = W >= 14 ? 1 : 1024 / BT;
+  static constexpr int U = W >= 14 ? 4 : 2;  // items whose loads are issued together
+  static_assert(W >= 9 && SB >= LT + 1, "entries per thread");
   static_assert(CS == 1 || kWs, "clusters share a run only with the window in the workspace");
 };
 
-// Sum of NV values of 2 BT virtual threads (v[j][0], v[j][1]: those of 2 t and
-// 2 t + 1), in the order of block_sum over TPR threads.
+// Sum of NV values of 2 BT virtual threads, in the order of block_sum over them:
+// thread tid holds those of insert_bit(tid, p) (v[j][0]) and its partner on bit p.
 template <int VW, int NV>
-__device__ __forceinline__ void block_sum_vec(const float (&v)[NV][2], float (&out)[NV], float *red, int &par) {
+__device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&out)[NV], float *red, int &par, int p) {
   float *r = red + par * (VW * 4);
+  const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (p < 5) {
+    const int top = threadIdx.x >> 4;
 #pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    float a = v[j][0], b = v[j][1];
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
+    for (int j = 0; j < NV; ++j) {
+      float a = v[j][0], b = v[j][1];
+      for (int o = 16; o > (1 << p); o >>= 1) {  // bits above p sit one lane bit lower
+        a += __shfl_xor_sync(0xffffffffu, a, o >> 1);
+        b += __shfl_xor_sync(0xffffffffu, b, o >> 1);
+      }
+      a += b;
+      for (int o = (1 << p) >> 1; o >= 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if ((lane & 15) == 0) r[top * 4 + j] = a;
     }
-    if ((threadIdx.x & 15) == 0) r[(threadIdx.x >> 4) * 4 + j] = a + b;
+  } else {
+    const int w0 = (int)wide_insert_bit((uint32_t)wq, p - 5);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      float a = v[j][0], b = v[j][1];
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if (lane == 0) {
+        r[w0 * 4 + j] = a;
+        r[(w0 | (1 << (p - 5))) * 4 + j] = b;
+      }
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -393,17 +419,22 @@ __device__ __forceinline__ void block_sum_vec(const float (&v)[NV][2], float (&o
   par ^= 1;
 }
 
-template <int W, int CS>
-__global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::MINB))
+__device__ __forceinline__ uint32_t wide_remove_bit(uint32_t q, int p) {
+  return ((q >> (p + 1)) << p) | (q & ((1u << p) - 1u));
+}
+__device__ __forceinline__ uint32_t sign_of(uint32_t v, uint32_t mask) { return (uint32_t)__popc(v & mask) << 31; }
+
+template <int W, int CS, bool RES>
+__global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>::MINB))
     sv_adj_wide(SvAdjArgs A, WideAdjGeom G) {
-  using Cfg = WideVecCfg<W, CS>;
-  constexpr int D = Cfg::D, TPR = Cfg::TPR, BT = Cfg::BT, VW = Cfg::VW, H2 = D / 2, QS = Cfg::QS, DS = Cfg::DS,
-                NIT = Cfg::NIT, U = Cfg::U, LOGCS = Cfg::LOGCS;
+  using Cfg = WideHalfCfg<W, CS>;
+  constexpr int N = Cfg::N, NS = Cfg::NS, TPR = Cfg::TPR, BT = Cfg::BT, VW = Cfg::VW, LT = Cfg::LT, SB = Cfg::SB,
+                FMAX = Cfg::FMAX;
   __shared__ float cred[8];
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const int M = A.M, NA = A.n_angles;
-  size_t off = Cfg::kWs ? 0 : wide_al((size_t)D * 8);
+  size_t off = Cfg::kWs ? 0 : wide_al((size_t)2 * N * 8);
   float2 *s_coef = reinterpret_cast<float2 *>(smem + off);
   off += wide_al((size_t)M * 8);
   uint32_t *s_mask = reinterpret_cast<uint32_t *>(smem + off);
@@ -421,23 +452,28 @@ __global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::M
     cid = blockIdx.x / CS;
     ncl = gridDim.x / CS;
   }
-  const uint32_t q_lo = (uint32_t)crank * QS, i_lo = (uint32_t)crank * DS;
+  const uint32_t q_lo = (uint32_t)crank * NS, h_lo = q_lo / 2;  // this block's entries, its pairs
   float2 *slot = reinterpret_cast<float2 *>(A.ckpt) + (size_t)cid * G.slot_elems;
-  float2 *hist = slot + (Cfg::kWs ? D : 0);
+  float2 *hist = slot + (Cfg::kWs ? 2 * N : 0);  // step 0: N entries; step k: N / 2 at (k + 1) N / 2
   float2 *swin = reinterpret_cast<float2 *>(smem + (Cfg::kWs ? off : 0));
-  float2 *gown = slot + i_lo;
+  float2 *scratch = (Cfg::kWs ? slot : swin) + N;
+  float2 *gown = slot + q_lo;
   const uint32_t res = (uint32_t)G.res;
-  auto at = [&](uint32_t i) -> float4 * {  // entries i, i + 1 (i even) of this block's slice
-    const uint32_t local = i & (DS - 1);
-    if constexpr (!Cfg::kWs) return reinterpret_cast<float4 *>(swin + local);
-    return reinterpret_cast<float4 *>(((local >> 10) < res ? swin : gown) + local);
+  auto home = [&](uint32_t q) -> float2 * {  // an entry of this block's slice
+    const uint32_t local = q & (NS - 1);
+    if constexpr (RES) return swin + local;
+    return ((local >> 10) < res ? swin : gown) + local;
   };
-  auto at_any = [&](uint32_t i) -> float4 * {  // of any block's
-    if constexpr (CS == 1) return at(i);
-    const uint32_t local = i & (DS - 1);
-    if ((local >> 10) >= res) return reinterpret_cast<float4 *>(slot + i);
-    return reinterpret_cast<float4 *>(cooperative_groups::this_cluster().map_shared_rank(swin, (int)(i / DS)) + local);
+  auto any = [&](uint32_t q) -> float2 * {  // of any block's
+    if constexpr (CS == 1) return home(q);
+    const uint32_t local = q & (NS - 1);
+    if (!RES && (local >> 10) >= res) return slot + q;
+    return cooperative_groups::this_cluster().map_shared_rank(swin, (int)(q / NS)) + local;
   };
+  auto scr = [&](uint32_t q) -> float2 * { return scratch + q; };
+  auto hist_of = [&](int k) -> float2 * { return hist + (size_t)(k ? k + 1 : 0) * (N / 2); };
+  using One = std::integral_constant<int, 1>;
+  using Max = std::integral_constant<int, FMAX>;
   using Yes = std::true_type;
   using No = std::false_type;
 
@@ -450,16 +486,22 @@ __global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::M
   const int n_in = A.n_in, n_out = A.n_out;
   const int64_t dout = (int64_t)1 << n_out;
   int par = 0;
-  auto phi_of = [](float2 u0, float2 u1, float2 c, float al) {
-    return make_float2(al * (u0.x + c.x * u1.x - c.y * u1.y), al * (u0.y + c.x * u1.y + c.y * u1.x));
+  auto phi_of = [](float2 a, float2 b, float2 c) {
+    return make_float2(fmaf(-c.y, b.y, fmaf(c.x, b.x, a.x)), fmaf(c.y, b.x, fmaf(c.x, b.y, a.y)));
   };
-  auto other = [](float2 v, uint32_t odd, bool dead) {  // the entering qubit's half
-    return dead ? make_float2(0.f, 0.f) : flip_sign(v, odd << 31);
+  auto times = [](float s, float2 v) { return make_float2(s * v.x, s * v.y); };
+  auto norm2 = [](float2 v) { return v.x * v.x + v.y * v.y; };
+  auto conj_mul = [](float2 c, float2 m) {
+    return make_float2(fmaf(c.y, m.y, __fmul_rn(c.x, m.x)), fmaf(c.x, m.y, -__fmul_rn(c.y, m.x)));
   };
-  auto parity = [](uint32_t v) { return (uint32_t)__popc(v) & 1u; };
-  auto lo2 = [](float4 v) { return make_float2(v.x, v.y); };
-  auto hi2 = [](float4 v) { return make_float2(v.z, v.w); };
-  auto join = [](float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); };
+  auto plus = [](float2 a, float2 b, uint32_t s) {
+    const float2 m = flip_sign(b, s);
+    return make_float2(a.x + m.x, a.y + m.y);
+  };
+  auto add_t = [](float (&t)[2][2], int z, float2 m, float2 h) {  // conj(mu) u
+    t[0][z] += fmaf(m.x, h.x, __fmul_rn(m.y, h.y));
+    t[1][z] += fmaf(m.x, h.y, -__fmul_rn(m.y, h.x));
+  };
 
   for (int64_t run = cid; run < A.B; run += ncl) {
     const int64_t vrow = fid ? run / A.J : run;
@@ -470,157 +512,175 @@ __global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::M
       float2 c, ph;
       sv_coef(st.plane, th, false, c, ph);
       s_coef[k] = c;
+      s_expo[k] = 0;
     }
-    // ---- initial window: input on its bits, |+> elsewhere, the CZ layer's signs
     const float2 *in = reinterpret_cast<const float2 *>(A.psi_in) +
                        irow * (fid ? ((int64_t)1 << n_in) : A.istride);
+    // ---- norm of the first window (input on its bits, |+> elsewhere)
     float nrm;
     {
       float nv[1][2] = {{0.f, 0.f}}, sum[1];
-      for (uint32_t i = i_lo + 2 * tid; i < i_lo + DS; i += TPR) {
-        float2 v[2];
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          v[z] = flip_sign(in[gather_bits(i + z, G.in_bits, n_in)], init_parity(i + z, G.init_cz, W) << 31);
-          nv[0][z] += v[z].x * v[z].x + v[z].y * v[z].y;
-        }
-        *at(i) = join(v[0], v[1]);
-      }
-      block_sum_vec<VW, 1>(nv, sum, red, par);
+      for (uint32_t x = (uint32_t)(crank * BT + tid); x < (1u << n_in); x += CS * BT) nv[0][0] += norm2(in[x]);
+      block_sum_pair<VW, 1>(nv, sum, red, par, 0);
       cluster_sum<CS, 1>(sum, cred, cpar);
-      nrm = sum[0];
+      nrm = sum[0] * RealBits<float>::pow2(W - n_in);
     }
 
-    // ---- forward, keeping every step's pre-step half-state
-    for (int k = 0; k < M; ++k) {
+    // ---- forward
+    bool moved = false;  // the window is in its scratch copy
+    {  // step 0: from the input and the CZ layer's signs
       const int e = renorm_exponent<float>(nrm);
       const float al = RealBits<float>::pow2(-e);
-      const float2 c = s_coef[k];
-      const uint32_t mask = s_mask[k];
-      const bool dead = (mask & kDead) != 0u;
-      const int p = k % W;
-      float4 *hk = reinterpret_cast<float4 *>(hist + (size_t)k * H2);
+      const float2 c = times(al, s_coef[0]);
+      if (tid == 0) s_expo[0] = e;
       float acc[1][2] = {{0.f, 0.f}}, sum[1];
-      if (tid == 0) s_expo[k] = e;
-      if (p + 1 < W - LOGCS && k + 2 < M) {
-        if (tid == 0) s_expo[k + 1] = 0;
-        const float2 c2 = s_coef[k + 1];
-        const uint32_t mask2 = s_mask[k + 1];
-        const bool dead2 = (mask2 & kDead) != 0u;
-        float4 *hk2 = hk + H2 / 2;
-        constexpr int U2 = NIT / 2 < U ? NIT / 2 : U;
-        auto pass = [&](auto p0) {  // p0: bit 0 is measured, quads are 4 consecutive entries
-          for (int b = 0; b < NIT / 2; b += U2) {
-            float4 x[U2][4];
+      for (uint32_t q = q_lo + tid; q < q_lo + NS; q += BT) {
+        float2 v[2];
 #pragma unroll
-            for (int j = 0; j < U2; ++j) {
-              const uint32_t r = q_lo / 2 + 2 * tid + (uint32_t)(b + j) * TPR;
-              const uint32_t i = p0.value ? 4 * r : wide_insert_bit(wide_insert_bit(r, p), p + 1);
-#pragma unroll
-              for (int z = 0; z < 4; ++z) x[j][z] = *at(p0.value ? i + 2 * z : i | ((uint32_t)z << p));
-            }
-#pragma unroll
-            for (int j = 0; j < U2; ++j) {
-              const uint32_t r = q_lo / 2 + 2 * tid + (uint32_t)(b + j) * TPR;
-              const uint32_t i = p0.value ? 4 * r : wide_insert_bit(wide_insert_bit(r, p), p + 1);
-              float2 v[2][4];  // quads r, r + 1: entries (bit p) + 2 (bit p + 1)
-#pragma unroll
-              for (int z = 0; z < 4; ++z) {
-                v[0][z] = p0.value ? ((z & 1) ? hi2(x[j][z >> 1]) : lo2(x[j][z >> 1])) : lo2(x[j][z]);
-                v[1][z] = p0.value ? ((z & 1) ? hi2(x[j][2 + (z >> 1)]) : lo2(x[j][2 + (z >> 1)])) : hi2(x[j][z]);
-              }
-              const uint32_t h = (p0.value ? 2 * r : wide_insert_bit(r, p)) >> 1, hs = (1u << p) >> 1;
-              if (p0.value) {
-                hk[h] = join(v[0][1], v[0][3]);
-                hk[h + 1] = join(v[1][1], v[1][3]);
-              } else {
-                hk[h] = join(v[0][1], v[1][1]);
-                hk[h + hs] = join(v[0][3], v[1][3]);
-              }
-              // sign parities of the entries, those of quad r + 1 one index bit away
-              const uint32_t nb = p0.value ? 4u : 1u;
-              const uint32_t s1 = parity((i | (1u << p)) & mask), s3 = parity((i | (3u << p)) & mask);
-              const uint32_t t2 = parity((i | (2u << p)) & mask2), t3 = parity((i | (3u << p)) & mask2);
-              const uint32_t d1 = parity(nb & mask), d2 = parity(nb & mask2);
-#pragma unroll
-              for (int z = 0; z < 2; ++z) {
-                v[z][0] = phi_of(v[z][0], v[z][1], c, al);
-                v[z][2] = phi_of(v[z][2], v[z][3], c, al);
-                v[z][1] = other(v[z][0], s1 ^ (z ? d1 : 0u), dead);
-                v[z][3] = other(v[z][2], s3 ^ (z ? d1 : 0u), dead);
-              }
-              if (p0.value) {
-                hk2[h] = join(v[0][2], v[0][3]);
-                hk2[h + 1] = join(v[1][2], v[1][3]);
-              } else {
-                hk2[h] = join(v[0][2], v[1][2]);
-                hk2[h + hs] = join(v[0][3], v[1][3]);
-              }
-#pragma unroll
-              for (int z = 0; z < 2; ++z) {
-                v[z][0] = phi_of(v[z][0], v[z][2], c2, 1.f);
-                v[z][1] = phi_of(v[z][1], v[z][3], c2, 1.f);
-                v[z][2] = other(v[z][0], t2 ^ (z ? d2 : 0u), dead2);
-                v[z][3] = other(v[z][1], t3 ^ (z ? d2 : 0u), dead2);
-                acc[0][z] += v[z][0].x * v[z][0].x + v[z][0].y * v[z][0].y;
-                acc[0][z] += v[z][1].x * v[z][1].x + v[z][1].y * v[z][1].y;
-              }
-#pragma unroll
-              for (int z = 0; z < 4; ++z)
-                *at(p0.value ? i + 2 * z : i | ((uint32_t)z << p)) =
-                    p0.value ? join(v[z >> 1][2 * (z & 1)], v[z >> 1][2 * (z & 1) + 1]) : join(v[0][z], v[1][z]);
-            }
-          }
-        };
-        if (p == 0)
-          pass(Yes{});
-        else
-          pass(No{});
-        block_sum_vec<VW, 1>(acc, sum, red, par);
-        cluster_sum<CS, 1>(sum, cred, cpar);
-        nrm = dead2 ? sum[0] : 2.f * sum[0];
-        ++k;
-        continue;
+        for (uint32_t z = 0; z < 2; ++z)
+          v[z] = flip_sign(in[gather_bits(2 * q + z, G.in_bits, n_in)], init_parity(2 * q + z, G.init_cz, W) << 31);
+        hist[q] = v[1];
+        const float2 o = phi_of(times(al, v[0]), v[1], c);
+        acc[0][0] += norm2(o);
+        *home(q) = o;
       }
-      auto pass = [&](auto p0, auto &&ent) {
-        for (int b = 0; b < NIT; b += U) {
-          float4 x[U], y[U];  // U items loaded before any is written back
+      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
+      cluster_sum<CS, 1>(sum, cred, cpar);
+      nrm = (s_mask[0] & kDead) ? sum[0] : 2.f * sum[0];
+    }
+    // F steps from step k on (p >= 1): the slots' bits p - 1 .. p + F - 2
+    auto fwd = [&](auto fc, auto &&src, auto &&dst, int k, float al, float (&acc)[1][2]) {
+      constexpr int F = decltype(fc)::value, Z = 1 << F, U = F == 1 ? 4 : 2;
+      constexpr int CNT = NS / Z / BT, UU = CNT < U ? CNT : U;
+      const int b = k % W - 1;
+      const uint32_t low = (1u << b) - 1u;
+      float2 c[F], c1[F];
+      uint32_t m[F], sg[F], zt[F];
+      bool dead[F];
+      const uint32_t r0 = (uint32_t)crank * (NS / Z) + tid;
 #pragma unroll
-          for (int j = 0; j < U; ++j) {
-            const uint32_t q = q_lo + 2 * tid + (uint32_t)(b + j) * TPR;
-            const uint32_t i0 = wide_insert_bit(q, p);
-            x[j] = *ent(i0);
-            y[j] = *ent(p0.value ? i0 + 2 : i0 | (1u << p));
+      for (int f = 0; f < F; ++f) {
+        m[f] = s_mask[k + f - 1];
+        dead[f] = (m[f] & kDead) != 0u;
+        c[f] = s_coef[k + f];
+        if (f == 0) c[f] = times(al, c[f]);
+        c1[f] = flip_sign(c[f], ((m[f] >> (b + f + 1)) & 1u) << 31);
+        const uint32_t ib = ((r0 >> b) << (b + F + 1)) | (r0 & low) | (1u << (b + f));
+        sg[f] = (uint32_t)__popc(ib & m[f]) & 1u;
+        zt[f] = 0;
+#pragma unroll
+        for (int z = 0; z < Z; ++z)
+          zt[f] |= ((uint32_t)__popc((((uint32_t)((z & ((1 << f) - 1)) | ((z >> (f + 1)) << (f + 2)))) << b) & m[f]) & 1u)
+                   << z;
+      }
+      for (int n = 0; n < CNT; n += UU) {
+        float2 x[UU][Z];
+#pragma unroll
+        for (int j = 0; j < UU; ++j) {
+          const uint32_t r = r0 + (uint32_t)(n + j) * BT;
+          const uint32_t s = ((r >> b) << (b + F)) | (r & low);
+#pragma unroll
+          for (int z = 0; z < Z; ++z) x[j][z] = *src(s | ((uint32_t)z << b));
+        }
+#pragma unroll
+        for (int j = 0; j < UU; ++j) {
+          const uint32_t rn = (uint32_t)(n + j) * BT, r = r0 + rn;
+          const uint32_t s = ((r >> b) << (b + F)) | (r & low);
+          const uint32_t hx = ((r >> b) << (b + F - 1)) | (r & low);
+          const uint32_t ibn = ((rn >> b) << (b + F + 1)) | (rn & low);
+#pragma unroll
+          for (int f = 0; f < F; ++f) {
+            float2 *hk = hist_of(k + f) + hx;
+            const uint32_t zs = zt[f] ^ (0u - (sg[f] ^ ((uint32_t)__popc(ibn & m[f]) & 1u)));
+#pragma unroll
+            for (int z = 0; z < Z; ++z) {
+              if ((z >> f) & 1) continue;
+              const float2 bb = x[j][z | (1 << f)];
+              const float2 aa = f == 0 ? times(al, x[j][z]) : x[j][z];
+              hk[(uint32_t)((z & ((1 << f) - 1)) | ((z >> (f + 1)) << f)) << b] = bb;
+              x[j][z] = phi_of(aa, bb, c[f]);
+              const float2 o1 = flip_sign(phi_of(aa, bb, c1[f]), (zs >> z) << 31);
+              x[j][z | (1 << f)] = dead[f] ? make_float2(0.f, 0.f) : o1;
+            }
           }
 #pragma unroll
-          for (int j = 0; j < U; ++j) {
-            const uint32_t q = q_lo + 2 * tid + (uint32_t)(b + j) * TPR;
-            const uint32_t i0 = wide_insert_bit(q, p);
-            const float2 ua = lo2(x[j]), va = p0.value ? hi2(x[j]) : lo2(y[j]);
-            const float2 ub = p0.value ? lo2(y[j]) : hi2(x[j]), vb = hi2(y[j]);
-            hk[q >> 1] = join(va, vb);
-            const uint32_t s1 = parity((i0 | (1u << p)) & mask), d1 = parity((p0.value ? 2u : 1u) & mask);
-            const float2 pa = phi_of(ua, va, c, al), pb = phi_of(ub, vb, c, al);
-            const float2 oa = other(pa, s1, dead), ob = other(pb, s1 ^ d1, dead);
-            *ent(i0) = p0.value ? join(pa, oa) : join(pa, pb);
-            *ent(p0.value ? i0 + 2 : i0 | (1u << p)) = p0.value ? join(pb, ob) : join(oa, ob);
-            acc[0][0] += pa.x * pa.x + pa.y * pa.y;
-            acc[0][1] += pb.x * pb.x + pb.y * pb.y;
+          for (int z = 0; z < Z; ++z) {
+            acc[0][0] += norm2(x[j][z]);
+            *dst(s | ((uint32_t)z << b)) = x[j][z];
           }
         }
-      };
-      if (p == 0)
-        pass(Yes{}, at);
-      else if (CS > 1 && p >= W - LOGCS)
-        pass(No{}, at_any);
-      else
-        pass(No{}, at);
-      block_sum_vec<VW, 1>(acc, sum, red, par);
+      }
+    };
+    for (int k = 1; k < M;) {
+      const int e = renorm_exponent<float>(nrm);
+      const float al = RealBits<float>::pow2(-e);
+      const int p = k % W;
+      if (tid == 0) s_expo[k] = e;
+      float acc[1][2] = {{0.f, 0.f}}, sum[1];
+      int f = 1;
+      if (p == 0) {
+        const uint32_t mask = s_mask[k - 1];
+        const bool dead = (mask & kDead) != 0u;
+        const float2 c = times(al, s_coef[k]), c1 = flip_sign(c, (mask & 1u) << 31);
+        float2 *hk = hist_of(k);
+        for (uint32_t m = h_lo + tid; m < h_lo + NS / 2; m += BT) {
+          const float2 aa = times(al, *home(2 * m)), bb = *home(2 * m + 1);
+          hk[m] = bb;
+          const float2 o0 = phi_of(aa, bb, c);
+          float2 o1 = flip_sign(phi_of(aa, bb, c1), sign_of((2 * m) | (1u << (W - 1)), mask));
+          if (dead) o1 = make_float2(0.f, 0.f);
+          *scr(m) = o0;
+          *scr(m | (N / 2)) = o1;
+          acc[0][0] += norm2(o0) + norm2(o1);
+        }
+        moved = true;
+      } else if (CS > 1 && p - 1 >= SB) {
+        fwd(One{}, any, any, k, al, acc);
+      } else {
+        if (p - 1 + FMAX <= SB && k + FMAX <= M) f = FMAX;
+        if (f == FMAX) {
+          if (moved)
+            fwd(Max{}, scr, home, k, al, acc);
+          else
+            fwd(Max{}, home, home, k, al, acc);
+        } else {
+          if (moved)
+            fwd(One{}, scr, home, k, al, acc);
+          else
+            fwd(One{}, home, home, k, al, acc);
+        }
+        moved = false;
+      }
+      k += f;
+      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
       cluster_sum<CS, 1>(sum, cred, cpar);
-      nrm = dead ? sum[0] : 2.f * sum[0];
+      nrm = (s_mask[k - 1] & kDead) ? sum[0] : 2.f * sum[0];
     }
+    auto now = [&](uint32_t q) -> float2 * {
+      if (moved) return scr(q);
+      return any(q);
+    };
 
     // ---- output and the seed lambda_M = dL/du_M
+    const int pl = (M - 1) % W;
+    const uint32_t mask_l = s_mask[M - 1];
+    const bool dead_l = (mask_l & kDead) != 0u;
+    auto out_of = [&](uint32_t i) {  // u_M
+      const float2 v = *now(wide_remove_bit(i, pl));
+      if (!((i >> pl) & 1u)) return v;
+      return dead_l ? make_float2(0.f, 0.f) : flip_sign(v, sign_of(i, mask_l));
+    };
+    {  // the last norm is a result: its sums in order
+      float acc[1][2] = {{0.f, 0.f}}, sum[1];
+      for (uint32_t q = q_lo + 2 * tid; q < q_lo + NS; q += TPR) {
+        const float2 v0 = *now(q), v1 = *now(q + 1);
+        acc[0][0] += norm2(v0);
+        acc[0][1] += norm2(v1);
+      }
+      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
+      cluster_sum<CS, 1>(sum, cred, cpar);
+      nrm = dead_l ? sum[0] : 2.f * sum[0];
+    }
     const bool ok = RealBits<float>::finite_pos(nrm);
     float inv = 0.f;
     if (ok) {
@@ -634,141 +694,260 @@ __global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::M
       run_barrier<CS>();  // the next run overwrites the coefficients
       continue;
     }
-    float loss_term = 0.f;
-    if (fid) {
-      const float2 *tg = reinterpret_cast<const float2 *>(A.targets) + irow * dout;
-      float pv[2][2] = {}, ps[2];  // <t|u_M>
-      for (uint32_t i = i_lo + 2 * tid; i < i_lo + DS; i += TPR) {
-        const float4 w = *at(i);
+    const float2 *row = reinterpret_cast<const float2 *>(fid ? A.targets : A.grad_out) + (fid ? irow : run) * dout;
+    float loss_term = 0.f, w0, w1, w2, w3;  // the seed's factors
+    {
+      float pv[2][2] = {}, ps[2];  // <t|u_M>, or Re <u_M|g>
+      for (uint32_t i = 2 * q_lo + 2 * tid; i < 2 * q_lo + 2 * NS; i += TPR) {
 #pragma unroll
-        for (int z = 0; z < 2; ++z) {
+        for (uint32_t z = 0; z < 2; ++z) {
           if ((i + z) & ~G.out_mask) continue;
-          const float2 t = tg[gather_bits(i + z, G.out_bits, n_out)], a = z ? hi2(w) : lo2(w);
-          pv[0][z] += t.x * a.x + t.y * a.y;
-          pv[1][z] += t.x * a.y - t.y * a.x;
+          const float2 t = row[gather_bits(i + z, G.out_bits, n_out)], a = out_of(i + z);
+          if (fid) {
+            pv[0][z] += t.x * a.x + t.y * a.y;
+            pv[1][z] += t.x * a.y - t.y * a.x;
+          } else {
+            pv[0][z] += a.x * t.x + a.y * t.y;
+          }
         }
       }
-      block_sum_vec<VW, 2>(pv, ps, red, par);
+      block_sum_pair<VW, 2>(pv, ps, red, par, 0);
       cluster_sum<CS, 2>(ps, cred, cpar);
-      const float ar = ps[0] * inv, ai = ps[1] * inv;
-      const float F = ar * ar + ai * ai;
-      const float wJ = 1.f / (float)A.J;
-      loss_term = (1.f - F) * wJ;
-      // lambda = (2/J)(F z - a t) / |u_M|
-      const float k2 = 2.f * wJ * inv, fz = F * inv;
-      for (uint32_t i = i_lo + 2 * tid; i < i_lo + DS; i += TPR) {
-        const float4 w = *at(i);
-        float2 l[2];
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          l[z] = make_float2(0.f, 0.f);
-          if (!((i + z) & ~G.out_mask)) {
-            const float2 t = tg[gather_bits(i + z, G.out_bits, n_out)], a = z ? hi2(w) : lo2(w);
-            l[z] = make_float2(k2 * (fz * a.x - (ar * t.x - ai * t.y)), k2 * (fz * a.y - (ar * t.y + ai * t.x)));
-          }
-        }
-        *at(i) = join(l[0], l[1]);
-      }
-    } else {
-      const float2 *go = reinterpret_cast<const float2 *>(A.grad_out) + run * dout;
-      float zv[1][2] = {{0.f, 0.f}}, zs[1];  // Re <u_M|g>
-      for (uint32_t i = i_lo + 2 * tid; i < i_lo + DS; i += TPR) {
-        const float4 w = *at(i);
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          if ((i + z) & ~G.out_mask) continue;
-          const float2 g = go[gather_bits(i + z, G.out_bits, n_out)], a = z ? hi2(w) : lo2(w);
-          zv[0][z] += a.x * g.x + a.y * g.y;
-        }
-      }
-      block_sum_vec<VW, 1>(zv, zs, red, par);
-      cluster_sum<CS, 1>(zs, cred, cpar);
-      const float zgi = zs[0] * inv * inv;
-      for (uint32_t i = i_lo + 2 * tid; i < i_lo + DS; i += TPR) {
-        const float4 w = *at(i);
-        float2 l[2];
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          l[z] = make_float2(0.f, 0.f);
-          if (!((i + z) & ~G.out_mask)) {
-            const float2 g = go[gather_bits(i + z, G.out_bits, n_out)], a = z ? hi2(w) : lo2(w);
-            l[z] = make_float2(inv * (g.x - zgi * a.x), inv * (g.y - zgi * a.y));
-          }
-        }
-        *at(i) = join(l[0], l[1]);
+      if (fid) {
+        w0 = ps[0] * inv;
+        w1 = ps[1] * inv;
+        const float F = w0 * w0 + w1 * w1;
+        const float wJ = 1.f / (float)A.J;
+        loss_term = (1.f - F) * wJ;
+        w2 = 2.f * wJ * inv;
+        w3 = F * inv;
+      } else {
+        w0 = w1 = w2 = 0.f;
+        w3 = ps[0] * inv * inv;
       }
     }
-    run_barrier<CS>();
+    auto seed_of = [&](uint32_t i, float2 a) {
+      if (i & ~G.out_mask) return make_float2(0.f, 0.f);
+      const float2 t = row[gather_bits(i, G.out_bits, n_out)];
+      if (fid)  // lambda = (2/J)(F z - a t) / |u_M|
+        return make_float2(w2 * (w3 * a.x - (w0 * t.x - w1 * t.y)), w2 * (w3 * a.y - (w0 * t.y + w1 * t.x)));
+      return make_float2(inv * (t.x - w3 * a.x), inv * (t.y - w3 * a.y));
+    };
 
     // ---- backward
-    for (int k = M - 1; k >= 0; --k) {
+    // u_{k-1}[., 1] at q: the history's b, or its signed copy
+    auto hist_at = [&](int k, uint32_t q) {
+      if (k == 0) return hist[q];
+      const int p = k % W, pp = p ? p - 1 : W - 2;
+      const uint32_t mask = s_mask[k - 1];
+      const float2 h = hist_of(k)[wide_remove_bit(q, pp)];
+      if (!((q >> pp) & 1u)) return h;
+      if (mask & kDead) return make_float2(0.f, 0.f);
+      return flip_sign(h, sign_of(wide_insert_bit(q, p) | (1u << p), mask));
+    };
+    auto prefetch = [&](int k) {  // the block's part of a history
+      const char *h = reinterpret_cast<const char *>(hist_of(k) + h_lo);
+      for (uint32_t o = tid * 128u; o < (uint32_t)NS * 4u; o += BT * 128u)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(h + o));
+    };
+    // lambda_k's other half, mu_k and lambda_{k-1} = al mu_k of a pair
+    auto pair_back = [&](float2 a, float2 b, float2 cn, float al, bool dead, uint32_t s0, uint32_t s1, float2 &m0,
+                         float2 &m1) {
+      const float2 ca = conj_mul(cn, a);
+      if (dead) {
+        m0 = times(al, a);
+        m1 = times(al, ca);
+      } else {
+        m0 = times(al, plus(a, b, s0));
+        m1 = times(al, plus(ca, conj_mul(cn, b), s1));
+      }
+    };
+    auto finish = [&](int k, const float (&t)[2][2], int p) {
+      float ts[2];
+      block_sum_pair<VW, 2>(t, ts, red, par, p);
+      cluster_sum<CS, 2>(ts, cred, cpar);
+      // kept in the history this step has finished with
+      if (tid == 0 && crank == 0) hist_of(k)[0] = make_float2(ts[0], ts[1]);
+    };
+    {  // the last step, from the seed
+      const int k = M - 1;
       const float al = RealBits<float>::pow2(-s_expo[k]);
-      const float2 c = s_coef[k];
+      float t[2][2] = {};
+      for (uint32_t q = q_lo + 2 * tid; q < q_lo + NS; q += TPR) {
+        float2 m[2];
+#pragma unroll
+        for (uint32_t z = 0; z < 2; ++z) {
+          const uint32_t i0 = wide_insert_bit(q + z, pl), i1 = i0 | (1u << pl);
+          const float2 v = *now(q + z);
+          m[z] = seed_of(i0, v);
+          if (!dead_l) {
+            const uint32_t s1 = sign_of(i1, mask_l);
+            m[z] = plus(m[z], seed_of(i1, flip_sign(v, s1)), s1);
+          }
+          m[z] = times(al, m[z]);
+          add_t(t, z, m[z], hist_at(k, q + z));
+        }
+        *home(q) = m[0];
+        *home(q + 1) = m[1];
+      }
+      if (k > 1) prefetch(k - 1);
+      finish(k, t, 0);
+    }
+    moved = false;
+    // lambda of step k, pairs on bit p (below w - 1), the sums to follow
+    auto bwd = [&](auto &&src, auto &&dst, int k, float al, float2 cn, uint32_t mask) {
+      constexpr int CNT = NS / 2 / BT, U = CNT < Cfg::U ? CNT : Cfg::U;
+      const int p = k % W;
+      const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid;
+      const bool dead = (mask & kDead) != 0u;
+      const uint32_t z1 = ((mask >> (p + 1)) & 1u) << 31;
+      const uint32_t st = sign_of(((r0 >> p) << (p + 2)) | (r0 & low) | (1u << p), mask);
+      for (int n = 0; n < CNT; n += U) {
+        float2 x[U], y[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          const uint32_t q0 = wide_insert_bit(r0 + (uint32_t)(n + j) * BT, p);
+          x[j] = *src(q0);
+          y[j] = *src(q0 | (1u << p));
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          const uint32_t rn = (uint32_t)(n + j) * BT, q0 = wide_insert_bit(r0 + rn, p);
+          const uint32_t s0 = st ^ sign_of(((rn >> p) << (p + 2)) | (rn & low), mask);
+          float2 m0, m1;
+          pair_back(x[j], y[j], cn, al, dead, s0, s0 ^ z1, m0, m1);
+          *dst(q0) = m0;
+          *dst(q0 | (1u << p)) = m1;
+        }
+      }
+    };
+    for (int k = M - 2; k >= 0; --k) {
+      const float al = RealBits<float>::pow2(-s_expo[k]);
+      const float2 cn = s_coef[k + 1];
       const uint32_t mask = s_mask[k];
       const bool dead = (mask & kDead) != 0u;
       const int p = k % W;
-      float4 *hk = reinterpret_cast<float4 *>(hist + (size_t)k * H2);
-      float t[2][2] = {}, ts[2];  // sum conj(mu) u[., 1]
-      auto pass = [&](auto p0, auto &&ent) {
-        for (int b = 0; b < NIT; b += U) {
-          float4 x[U], y[U], hh[U];  // U items and their history loaded before any is written back
+      float t[2][2] = {};
+      if (k > 1) prefetch(k - 1);
+      if (p == W - 1) {  // the slots move
+        for (uint32_t m = h_lo + tid; m < h_lo + NS / 2; m += BT) {
+          const float2 a = *any(m), b = *any(m | (N / 2));
+          const float2 h0 = hist_at(k, 2 * m), h1 = hist_at(k, 2 * m + 1);
+          const uint32_t s0 = sign_of((2 * m) | (1u << (W - 1)), mask);
+          float2 m0, m1;
+          pair_back(a, b, cn, al, dead, s0, s0 ^ ((mask & 1u) << 31), m0, m1);
+          add_t(t, 0, m0, h0);
+          add_t(t, 1, m1, h1);
+          *scr(2 * m) = m0;
+          *scr(2 * m + 1) = m1;
+        }
+        moved = true;
+        finish(k, t, 0);
+      } else if (p < LT) {
+        auto direct = [&](auto first) {
+          constexpr int CNT = NS / 2 / BT, U = CNT < Cfg::U ? CNT : Cfg::U;
+          const int pp = p ? p - 1 : W - 2;
+          const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid;
+          const uint32_t z1 = ((mask >> (p + 1)) & 1u) << 31;
+          const uint32_t it = ((r0 >> p) << (p + 2)) | (r0 & low) | (1u << p);
+          const uint32_t st = sign_of(it, mask);
+          const float2 *hk = hist_of(k);
+          const uint32_t hm = first.value ? 0u : s_mask[k - 1];
+          const uint32_t hz = ((hm >> (p + 1)) & 1u) << 31;
+          const uint32_t ht = sign_of(it, hm);
+          const bool gone = (hm & kDead) != 0u;
+          for (int n = 0; n < CNT; n += U) {
+            float2 x[U], y[U], h0[U], h1[U];
 #pragma unroll
-          for (int j = 0; j < U; ++j) {
-            const uint32_t q = q_lo + 2 * tid + (uint32_t)(b + j) * TPR;
-            const uint32_t i0 = wide_insert_bit(q, p);
-            hh[j] = hk[q >> 1];
-            x[j] = *ent(i0);
-            y[j] = *ent(p0.value ? i0 + 2 : i0 | (1u << p));
-          }
-#pragma unroll
-          for (int j = 0; j < U; ++j) {
-            const uint32_t q = q_lo + 2 * tid + (uint32_t)(b + j) * TPR;
-            const uint32_t i0 = wide_insert_bit(q, p);
-            const uint32_t s1 = parity((i0 | (1u << p)) & mask), d1 = parity((p0.value ? 2u : 1u) & mask);
-            float2 l0[2], l1[2];
-            l0[0] = lo2(x[j]);
-            l1[0] = p0.value ? hi2(x[j]) : lo2(y[j]);
-            l0[1] = p0.value ? lo2(y[j]) : hi2(x[j]);
-            l1[1] = hi2(y[j]);
-#pragma unroll
-            for (int z = 0; z < 2; ++z) {
-              float2 mu = l0[z];
-              if (!dead) {
-                const float2 m1 = flip_sign(l1[z], (s1 ^ (z ? d1 : 0u)) << 31);
-                mu.x += m1.x;
-                mu.y += m1.y;
-              }
-              const float2 h = z ? hi2(hh[j]) : lo2(hh[j]);
-              t[0][z] += fmaf(mu.x, h.x, __fmul_rn(mu.y, h.y));
-              t[1][z] += fmaf(mu.x, h.y, -__fmul_rn(mu.y, h.x));
-              l0[z] = make_float2(al * mu.x, al * mu.y);
-              l1[z] = make_float2(al * fmaf(c.y, mu.y, __fmul_rn(c.x, mu.x)),  // conj(c) mu
-                                  al * fmaf(c.x, mu.y, -__fmul_rn(c.y, mu.x)));
+            for (int j = 0; j < U; ++j) {
+              const uint32_t q0 = wide_insert_bit(r0 + (uint32_t)(n + j) * BT, p), q1 = q0 | (1u << p);
+              h0[j] = hk[first.value ? q0 : wide_remove_bit(q0, pp)];
+              h1[j] = hk[first.value ? q1 : wide_remove_bit(q1, pp)];
+              x[j] = *home(q0);
+              y[j] = *home(q1);
             }
-            *ent(i0) = p0.value ? join(l0[0], l1[0]) : join(l0[0], l0[1]);
-            *ent(p0.value ? i0 + 2 : i0 | (1u << p)) = p0.value ? join(l0[1], l1[1]) : join(l1[0], l1[1]);
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+              const uint32_t rn = (uint32_t)(n + j) * BT, q0 = wide_insert_bit(r0 + rn, p);
+              const uint32_t in_ = ((rn >> p) << (p + 2)) | (rn & low);
+              const uint32_t s0 = st ^ sign_of(in_, mask);
+              float2 m0, m1;
+              pair_back(x[j], y[j], cn, al, dead, s0, s0 ^ z1, m0, m1);
+              if (!first.value && ((q0 >> pp) & 1u)) {
+                const uint32_t g0 = ht ^ sign_of(in_, hm);
+                h0[j] = gone ? make_float2(0.f, 0.f) : flip_sign(h0[j], g0);
+                h1[j] = gone ? make_float2(0.f, 0.f) : flip_sign(h1[j], g0 ^ hz);
+              }
+              add_t(t, 0, m0, h0[j]);
+              add_t(t, 1, m1, h1[j]);
+              *home(q0) = m0;
+              *home(q0 | (1u << p)) = m1;
+            }
+          }
+        };
+        if (k == 0)
+          direct(Yes{});
+        else
+          direct(No{});
+        finish(k, t, p);
+      } else {
+        bool joined = false;
+        if constexpr (CS > 1) {
+          if (p >= SB) {  // after the slots moved (p = w - 2), always
+            joined = true;
+            if (moved)
+              bwd(scr, any, k, al, cn, mask);
+            else
+              bwd(any, any, k, al, cn, mask);
+            run_barrier<CS>();
           }
         }
-      };
-      if (p == 0)
-        pass(Yes{}, at);
-      else if (CS > 1 && p >= W - LOGCS)
-        pass(No{}, at_any);
-      else
-        pass(No{}, at);
-      block_sum_vec<VW, 2>(t, ts, red, par);
-      cluster_sum<CS, 2>(ts, cred, cpar);
-      // kept in the history this step has finished with
-      if (tid == 0 && crank == 0) hist[(size_t)k * H2] = make_float2(ts[0], ts[1]);
+        if (!joined) {
+          if (CS == 1 && moved)
+            bwd(scr, home, k, al, cn, mask);
+          else
+            bwd(home, home, k, al, cn, mask);
+          __syncthreads();
+        }
+        moved = false;
+        constexpr int CNT = NS / TPR, U = CNT < Cfg::U ? CNT : Cfg::U;
+        const int pp = p - 1;  // >= 1
+        const uint32_t hm = s_mask[k - 1], r0 = q_lo + 2 * tid;
+        const uint32_t hz = (hm & 1u) << 31;
+        const bool gone = (hm & kDead) != 0u;
+        const uint32_t ht = sign_of(wide_insert_bit(r0, p) | (1u << p), hm);
+        const float4 *hk = reinterpret_cast<const float4 *>(hist_of(k));
+        for (int n = 0; n < CNT; n += U) {
+          float4 x[U], h[U];
+#pragma unroll
+          for (int j = 0; j < U; ++j) {
+            const uint32_t q = r0 + (uint32_t)(n + j) * TPR;
+            h[j] = hk[wide_remove_bit(q, pp) >> 1];
+            x[j] = *reinterpret_cast<const float4 *>(home(q));
+          }
+#pragma unroll
+          for (int j = 0; j < U; ++j) {
+            const uint32_t qn = (uint32_t)(n + j) * TPR, q = r0 + qn;
+            float2 h0 = make_float2(h[j].x, h[j].y), h1 = make_float2(h[j].z, h[j].w);
+            if ((q >> pp) & 1u) {
+              const uint32_t g0 = ht ^ sign_of(wide_insert_bit(qn, p), hm);
+              h0 = gone ? make_float2(0.f, 0.f) : flip_sign(h0, g0);
+              h1 = gone ? make_float2(0.f, 0.f) : flip_sign(h1, g0 ^ hz);
+            }
+            add_t(t, 0, make_float2(x[j].x, x[j].y), h0);
+            add_t(t, 1, make_float2(x[j].z, x[j].w), h1);
+          }
+        }
+        finish(k, t, 0);
+      }
     }
     if (crank == 0) {
       __syncthreads();
       for (int k = tid; k < M; k += BT) {
         const int ai = s_aidx[k];
         if (ai < 0) continue;
-        const float al = RealBits<float>::pow2(-s_expo[k]);
-        const float2 c = s_coef[k], t01 = hist[(size_t)k * H2];
-        const double g = (double)al * ((double)c.x * t01.y + (double)c.y * t01.x);  // alpha Im(c t)
+        const float2 c = s_coef[k], t01 = hist_of(k)[0];  // scaled by alpha_k
+        const double g = (double)c.x * t01.y + (double)c.y * t01.x;  // alpha Im(c t)
         if (fid)
           atomicAdd(&A.grad[vrow * NA + ai], g);
         else
@@ -788,7 +967,7 @@ __global__ void __launch_bounds__((WideVecCfg<W, CS>::BT), (WideVecCfg<W, CS>::M
 int wide_adj_resident(int w, int M, bool gen, int cluster, size_t limit) {
   if (w <= 14 || gen) return 0;
   const size_t base = wide_smem_bytes(w, M, gen) + 64;
-  const size_t pieces = ((size_t)1 << (w - 10)) / (size_t)cluster;
+  const size_t pieces = ((size_t)1 << (w - 11)) / (size_t)cluster;
   const size_t room = limit > base ? (limit - base) / 8192 : 0;
   return (int)(pieces < room ? pieces : room);
 }
@@ -826,15 +1005,27 @@ static int wide_launch(K k, const SvAdjArgs &a, const WideAdjGeom &g, const AdjL
   return check_launch("sv_adj_wide");
 }
 
+template <int W, int CS>
+static int wide_half(const SvAdjArgs &a, const WideAdjGeom &g, const AdjLaunch &l, cudaStream_t s) {
+  using Cfg = WideHalfCfg<W, CS>;
+  if constexpr (!Cfg::kWs) {
+    return wide_launch(sv_adj_wide<W, CS, true>, a, g, l, Cfg::BT, CS, s);
+  } else {
+    if constexpr (Cfg::NS <= 16384)
+      if (g.res == Cfg::NS / 1024) return wide_launch(sv_adj_wide<W, CS, true>, a, g, l, Cfg::BT, CS, s);
+    return wide_launch(sv_adj_wide<W, CS, false>, a, g, l, Cfg::BT, CS, s);
+  }
+}
+
 template <int W>
 static int wide_pick(const SvAdjArgs &a, const WideAdjGeom &g, const AdjLaunch &l, cudaStream_t s, bool gen) {
   if (gen) return wide_launch(sv_adj_wide_gen<W>, a, g, l, WideAdjCfg<W>::TPR, 1, s);
   if constexpr (W >= 9) {
     if constexpr (WideAdjCfg<W>::kWs) {
-      if (g.cluster == 4) return wide_launch(sv_adj_wide<W, 4>, a, g, l, WideVecCfg<W, 4>::BT, 4, s);
-      if (g.cluster == 2) return wide_launch(sv_adj_wide<W, 2>, a, g, l, WideVecCfg<W, 2>::BT, 2, s);
+      if (g.cluster == 4) return wide_half<W, 4>(a, g, l, s);
+      if (g.cluster == 2) return wide_half<W, 2>(a, g, l, s);
     }
-    return wide_launch(sv_adj_wide<W, 1>, a, g, l, WideVecCfg<W, 1>::BT, 1, s);
+    return wide_half<W, 1>(a, g, l, s);
   }
   return fail(MBQC_E_UNSUPPORTED, "adjoint: window %d takes the register kernel", W);
 }
