@@ -72,7 +72,6 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
   if (rc) return rc;
   if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "adjoint: kernel does not fit on an SM");
   const int64_t D = (int64_t)1 << hc.w;
-  const int64_t slot = (hc.w > 14 ? D : 0) + (g.gen ? hc.n_steps * D : (hc.n_steps + 1) * (D / 4));
   // a batch smaller than the GPU: runs of a window in the workspace are
   // shared by a cluster of 2 or 4 blocks (one block per SM), so that more SMs
   // work on them; blocks below counts run slots (clusters)
@@ -90,6 +89,10 @@ static int adj_geometry_wide(const DevCircuit &hc, int64_t runs, bool f64, AdjGe
     g.wg.res = wide_adj_resident(hc.w, hc.n_steps, g.gen, g.wg.cluster, (size_t)optin - 1024);
     g.smem += (size_t)g.wg.res * 8192;
   }
+  // the window and its scratch copy, the steps' history, their warp sums
+  const int64_t slot = (hc.w > 14 ? D : 0) + (g.gen ? hc.n_steps * D
+                                                    : (hc.n_steps + 1) * (D / 4) +
+                                                          (int64_t)hc.n_steps * g.wg.cluster * (wide_adj_threads(hc.w) / 32));
   int64_t blocks = g.wg.cluster > 1 ? (int64_t)sm_count() / g.wg.cluster : (int64_t)sm_count() * occ;
   if (runs < blocks) blocks = runs;
   const int64_t cap = (int64_t)(kWideAdjMaxWorkspace / ((size_t)slot * 8));

@@ -346,19 +346,24 @@ __global__ void __launch_bounds__(WideAdjCfg<W>::TPR) sv_adj_wide_gen(SvAdjArgs 
 // The history of a step is b alone (N / 2); lambda is kept the same way
 // (lambda[., 1] = conj(c) lambda[., 0]): pairs on bit p, w - 1 the step that moves.
 //
-// What bounds it at w = 17 (64 runs of the 16 x 10 grid, two blocks a run) is
-// issue at four warps a scheduler: 53 % of the slots, DRAM at a quarter of its
-// rate (the history).  Keeping both halves it was the traffic between the L2 and
-// the SMs: w = 17, 64 runs 4.98 -> 2.76 ms; w = 15, 256 runs 2.80 -> 2.02; w = 19,
-// 32 runs of 18 x 6 9.44 -> 4.72 ms.  The block keeps its slice of the window in shared memory as far as it
-// fits (RES: all of it); the forward pass takes up to three steps at a time on
-// pairs inside the slice; a step on the bits that join slices pairs entries of
-// two blocks through distributed shared memory.
-//
-// The gradient's sums are those of TPR = 2 BT threads, thread v taking the q =
-// v mod TPR in turn.  A backward step on a bit below log2 TPR gives a thread two
-// of those (insert_bit(tid, p) and its partner); a step above it updates lambda
-// first and then sums over q in order (tid: v = 2 tid and 2 tid + 1).
+// What bounds it at w = 17 (64 runs of the 16 x 10 grid, two blocks a run, 2.41 ms)
+// is latency at four warps a scheduler: a forward pass of three steps 13 us, a
+// backward step 8.6 us on a low bit, 6.2 us in order, 11 to 13 us where it takes
+// two passes or joins slices; the history's DRAM floor is 2.5 us a step.
+//   * What fits of the block's slice stays in its shared memory (RES: all of it).
+//     Entries are placed so that lanes which leave out low bits miss each other's
+//     banks (wide_place), indices are split into a thread's part and a uniform one.
+//   * The forward pass takes three steps at a time on pairs inside the slice (p = 1:
+//     the slots of an item are neighbours and move as 16 bytes).
+//   * The gradient's sums are those of TPR = 2 BT threads, thread v taking the q = v
+//     mod TPR in turn.  A backward step on a bit below log2 TPR gives a thread two
+//     of those (insert_bit(tid, p) and its partner); on the three bits above, the
+//     pairs are 2, 4 and 8 apart in one thread's order and a group of them is held;
+//     above that, and on bits that join slices, lambda is updated first and summed
+//     over q in order afterwards.  Only the warps' sums are made per step.
+// Both halves kept, one or two steps a pass: w = 17, 64 runs 4.98 ms; w = 15, 256
+// runs 2.80 -> 1.77; w = 12, 512 runs 0.60 -> 0.52; w = 19, 32 runs of 18 x 6 9.44 ->
+// 4.32 ms.  Loading the history a batch ahead was slower (2.64 ms).
 template <int W, int CS> struct WideHalfCfg {
   static constexpr int D = 1 << W, N = D / 2, NS = N / CS;
   static constexpr int LT = W <= 9 ? 7 : (W == 10 ? 8 : (W == 11 ? 9 : 10));
@@ -373,11 +378,11 @@ template <int W, int CS> struct WideHalfCfg {
   static_assert(CS == 1 || kWs, "clusters share a run only with the window in the workspace");
 };
 
-// Sum of NV values of 2 BT virtual threads, in the order of block_sum over them:
-// thread tid holds those of insert_bit(tid, p) (v[j][0]) and its partner on bit p.
-template <int VW, int NV>
-__device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&out)[NV], float *red, int &par, int p) {
-  float *r = red + par * (VW * 4);
+// Warp sums of NV values of 2 BT virtual threads, in the order of block_sum over
+// them: thread tid holds those of insert_bit(tid, p) (v[j][0]) and its partner on
+// bit p; put(j, virtual warp, sum).
+template <int NV, typename Put>
+__device__ __forceinline__ void warp_sums_pair(const float (&v)[NV][2], int p, Put put) {
   const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (p < 5) {
     const int top = threadIdx.x >> 4;
@@ -390,7 +395,7 @@ __device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&
       }
       a += b;
       for (int o = (1 << p) >> 1; o >= 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if ((lane & 15) == 0) r[top * 4 + j] = a;
+      if ((lane & 15) == 0) put(j, top, a);
     }
   } else {
     const int w0 = (int)wide_insert_bit((uint32_t)wq, p - 5);
@@ -403,11 +408,17 @@ __device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&
         b += __shfl_xor_sync(0xffffffffu, b, o);
       }
       if (lane == 0) {
-        r[w0 * 4 + j] = a;
-        r[(w0 | (1 << (p - 5))) * 4 + j] = b;
+        put(j, w0, a);
+        put(j, w0 | (1 << (p - 5)), b);
       }
     }
   }
+}
+
+template <int VW, int NV>
+__device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&out)[NV], float *red, int &par) {
+  float *r = red + par * (VW * 4);
+  warp_sums_pair<NV>(v, 0, [&](int j, int w, float a) { r[w * 4 + j] = a; });
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
@@ -422,6 +433,13 @@ __device__ __forceinline__ void block_sum_pair(const float (&v)[NV][2], float (&
 __device__ __forceinline__ uint32_t wide_remove_bit(uint32_t q, int p) {
   return ((q >> (p + 1)) << p) | (q & ((1u << p) - 1u));
 }
+// Place of an entry in its slice: bits 4..6 folded into 1..3, so that accesses of
+// 8 bytes whose lanes leave out a bit below 4, or three bits from 0 or 3 on, find
+// 16 different banks.  Linear, and 16-byte pairs stay together.
+__device__ __forceinline__ uint32_t wide_place(uint32_t e) {
+  return e ^ ((e >> 3) & 12u) ^ (((e >> 4) & 1u) * 14u);
+}
+__device__ __forceinline__ float sign_f(float v, uint32_t s) { return __uint_as_float(__float_as_uint(v) ^ s); }
 __device__ __forceinline__ uint32_t sign_of(uint32_t v, uint32_t mask) { return (uint32_t)__popc(v & mask) << 31; }
 
 template <int W, int CS, bool RES>
@@ -455,19 +473,28 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
   const uint32_t q_lo = (uint32_t)crank * NS, h_lo = q_lo / 2;  // this block's entries, its pairs
   float2 *slot = reinterpret_cast<float2 *>(A.ckpt) + (size_t)cid * G.slot_elems;
   float2 *hist = slot + (Cfg::kWs ? 2 * N : 0);  // step 0: N entries; step k: N / 2 at (k + 1) N / 2
+  float2 *part = hist + (size_t)(M + 1) * (N / 2);  // [step][rank][warp]
   float2 *swin = reinterpret_cast<float2 *>(smem + (Cfg::kWs ? off : 0));
   float2 *scratch = (Cfg::kWs ? slot : swin) + N;
   float2 *gown = slot + q_lo;
   const uint32_t res = (uint32_t)G.res;
   auto home = [&](uint32_t q) -> float2 * {  // an entry of this block's slice
-    const uint32_t local = q & (NS - 1);
+    const uint32_t local = wide_place(q & (NS - 1));
     if constexpr (RES) return swin + local;
     return ((local >> 10) < res ? swin : gown) + local;
   };
+  auto home_at = [&](uint32_t local) -> float2 * {  // by its place
+    if constexpr (RES) return swin + local;
+    return ((local >> 10) < res ? swin : gown) + local;
+  };
+  auto slice_at = [&](uint32_t qn) -> float2 * {  // the slice holding the piece of 1,024 from qn on
+    if constexpr (RES) return swin;
+    return (qn >> 10) < res ? swin : gown;
+  };
   auto any = [&](uint32_t q) -> float2 * {  // of any block's
     if constexpr (CS == 1) return home(q);
-    const uint32_t local = q & (NS - 1);
-    if (!RES && (local >> 10) >= res) return slot + q;
+    const uint32_t local = wide_place(q & (NS - 1));
+    if (!RES && (local >> 10) >= res) return slot + (q & ~(uint32_t)(NS - 1)) + local;
     return cooperative_groups::this_cluster().map_shared_rank(swin, (int)(q / NS)) + local;
   };
   auto scr = [&](uint32_t q) -> float2 * { return scratch + q; };
@@ -491,6 +518,7 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
   };
   auto times = [](float s, float2 v) { return make_float2(s * v.x, s * v.y); };
   auto norm2 = [](float2 v) { return v.x * v.x + v.y * v.y; };
+  auto add_norm = [](float &s, float2 v) { s = fmaf(v.x, v.x, fmaf(v.y, v.y, s)); };  // for a scale alone
   auto conj_mul = [](float2 c, float2 m) {
     return make_float2(fmaf(c.y, m.y, __fmul_rn(c.x, m.x)), fmaf(c.x, m.y, -__fmul_rn(c.y, m.x)));
   };
@@ -501,6 +529,10 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
   auto add_t = [](float (&t)[2][2], int z, float2 m, float2 h) {  // conj(mu) u
     t[0][z] += fmaf(m.x, h.x, __fmul_rn(m.y, h.y));
     t[1][z] += fmaf(m.x, h.y, -__fmul_rn(m.y, h.x));
+  };
+  auto add_ts = [](float (&t)[2][2], int z, float2 m, float2 h, float s) {  // u = s h, s = 1, -1 or 0
+    t[0][z] = fmaf(s, fmaf(m.x, h.x, __fmul_rn(m.y, h.y)), t[0][z]);
+    t[1][z] = fmaf(s, fmaf(m.x, h.y, -__fmul_rn(m.y, h.x)), t[1][z]);
   };
 
   for (int64_t run = cid; run < A.B; run += ncl) {
@@ -521,7 +553,7 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
     {
       float nv[1][2] = {{0.f, 0.f}}, sum[1];
       for (uint32_t x = (uint32_t)(crank * BT + tid); x < (1u << n_in); x += CS * BT) nv[0][0] += norm2(in[x]);
-      block_sum_pair<VW, 1>(nv, sum, red, par, 0);
+      block_sum_pair<VW, 1>(nv, sum, red, par);
       cluster_sum<CS, 1>(sum, cred, cpar);
       nrm = sum[0] * RealBits<float>::pow2(W - n_in);
     }
@@ -534,34 +566,67 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
       const float2 c = times(al, s_coef[0]);
       if (tid == 0) s_expo[0] = e;
       float acc[1][2] = {{0.f, 0.f}}, sum[1];
-      for (uint32_t q = q_lo + tid; q < q_lo + NS; q += BT) {
+      // input index and CZ sign of i = t ^ n (no bit in common): x(t) ^ x(n) and
+      // Q(t) ^ Q(n) ^ |n & a(t)| ^ |t & a(n)|, a(v) the couplings of v's bits; the
+      // part of the next 32 n is made by the lanes
+      auto couplings = [&](uint32_t v) {
+        uint32_t a = 0;
+        for (int q = 0; q < W; ++q) a ^= (0u - ((v >> q) & 1u)) & G.init_cz[q];
+        return a;
+      };
+      uint32_t xt[2], at[2], qt[2], xn = 0, an = 0;
+#pragma unroll
+      for (uint32_t z = 0; z < 2; ++z) {
+        const uint32_t i = 2 * (q_lo + tid) + z;
+        xt[z] = (uint32_t)gather_bits(i, G.in_bits, n_in);
+        at[z] = couplings(i);
+        qt[z] = init_parity(i, G.init_cz, W);
+      }
+      for (uint32_t n = 0; n < NS / BT; ++n) {
+        const uint32_t q = q_lo + tid + n * BT, in2 = 2 * n * BT;
+        if ((n & 31u) == 0) {
+          const uint32_t i = 2 * (n + (tid & 31)) * BT;
+          xn = (uint32_t)gather_bits(i, G.in_bits, n_in) | (init_parity(i, G.init_cz, W) << 31);
+          an = couplings(i);
+        }
+        const uint32_t xj = __shfl_sync(0xffffffffu, xn, n & 31), aj = __shfl_sync(0xffffffffu, an, n & 31);
         float2 v[2];
 #pragma unroll
-        for (uint32_t z = 0; z < 2; ++z)
-          v[z] = flip_sign(in[gather_bits(2 * q + z, G.in_bits, n_in)], init_parity(2 * q + z, G.init_cz, W) << 31);
+        for (uint32_t z = 0; z < 2; ++z) {
+          const uint32_t odd = qt[z] ^ (xj >> 31) ^ (uint32_t)__popc(in2 & at[z]) ^
+                               (uint32_t)__popc((2 * (q_lo + tid) + z) & aj);
+          v[z] = flip_sign(in[xt[z] ^ (xj & 0x7fffffffu)], odd << 31);
+        }
         hist[q] = v[1];
         const float2 o = phi_of(times(al, v[0]), v[1], c);
         acc[0][0] += norm2(o);
         *home(q) = o;
       }
-      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
+      block_sum_pair<VW, 1>(acc, sum, red, par);
       cluster_sum<CS, 1>(sum, cred, cpar);
       nrm = (s_mask[0] & kDead) ? sum[0] : 2.f * sum[0];
     }
     // F steps from step k on (p >= 1): the slots' bits p - 1 .. p + F - 2
-    auto fwd = [&](auto fc, auto &&src, auto &&dst, int k, float al, float (&acc)[1][2]) {
+    // (p1: p = 1, the slots of an item are neighbours; sc: read from the scratch
+    // copy; jn: the pair joins two slices)
+    auto fwd = [&](auto fc, auto p1, auto sc, auto jn, int k, float al, float (&acc)[1][2]) {
       constexpr int F = decltype(fc)::value, Z = 1 << F, U = F == 1 ? 4 : 2;
       constexpr int CNT = NS / Z / BT, UU = CNT < U ? CNT : U;
-      const int b = k % W - 1;
+      constexpr bool B0 = p1.value && F > 1;
+      const int b = B0 ? 0 : k % W - 1;
       const uint32_t low = (1u << b) - 1u;
       float2 c[F], c1[F];
       uint32_t m[F], sg[F], zt[F];
-      bool dead[F];
+      uint32_t keep[F];
+      float2 *hk[F];
+      // index maps are bitwise: the thread's part once, the rest uniform
       const uint32_t r0 = (uint32_t)crank * (NS / Z) + tid;
+      const uint32_t s0 = ((r0 >> b) << (b + F)) | (r0 & low), l0 = wide_place(s0 & (NS - 1));
 #pragma unroll
       for (int f = 0; f < F; ++f) {
         m[f] = s_mask[k + f - 1];
-        dead[f] = (m[f] & kDead) != 0u;
+        keep[f] = (m[f] & kDead) ? 0u : ~0u;
+        hk[f] = hist_of(k + f) + (((r0 >> b) << (b + F - 1)) | (r0 & low));
         c[f] = s_coef[k + f];
         if (f == 0) c[f] = times(al, c[f]);
         c1[f] = flip_sign(c[f], ((m[f] >> (b + f + 1)) & 1u) << 31);
@@ -577,36 +642,66 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         float2 x[UU][Z];
 #pragma unroll
         for (int j = 0; j < UU; ++j) {
-          const uint32_t r = r0 + (uint32_t)(n + j) * BT;
-          const uint32_t s = ((r >> b) << (b + F)) | (r & low);
+          const uint32_t rn = (uint32_t)(n + j) * BT;
+          const uint32_t sn = ((rn >> b) << (b + F)) | (rn & low);
 #pragma unroll
-          for (int z = 0; z < Z; ++z) x[j][z] = *src(s | ((uint32_t)z << b));
+          for (int z = 0; z < Z; ++z) {
+            const uint32_t zb = sn | ((uint32_t)z << b);
+            if constexpr (B0) {
+              if (z & 1) continue;
+              const float4 v = *reinterpret_cast<const float4 *>(sc.value ? scr(s0 | zb) : home_at(l0 ^ wide_place(zb)));
+              x[j][z] = make_float2(v.x, v.y);
+              x[j][z | 1] = make_float2(v.z, v.w);
+            } else if constexpr (sc.value)
+              x[j][z] = *scr(s0 | zb);
+            else if constexpr (jn.value)
+              x[j][z] = *any(s0 | zb);
+            else
+              x[j][z] = *home_at(l0 ^ wide_place(zb));
+          }
         }
 #pragma unroll
         for (int j = 0; j < UU; ++j) {
-          const uint32_t rn = (uint32_t)(n + j) * BT, r = r0 + rn;
-          const uint32_t s = ((r >> b) << (b + F)) | (r & low);
-          const uint32_t hx = ((r >> b) << (b + F - 1)) | (r & low);
+          const uint32_t rn = (uint32_t)(n + j) * BT;
+          const uint32_t sn = ((rn >> b) << (b + F)) | (rn & low);
+          const uint32_t hn = ((rn >> b) << (b + F - 1)) | (rn & low);
           const uint32_t ibn = ((rn >> b) << (b + F + 1)) | (rn & low);
 #pragma unroll
           for (int f = 0; f < F; ++f) {
-            float2 *hk = hist_of(k + f) + hx;
             const uint32_t zs = zt[f] ^ (0u - (sg[f] ^ ((uint32_t)__popc(ibn & m[f]) & 1u)));
+            float2 hv[Z / 2];
 #pragma unroll
             for (int z = 0; z < Z; ++z) {
               if ((z >> f) & 1) continue;
+              const int hz = (z & ((1 << f) - 1)) | ((z >> (f + 1)) << f);
               const float2 bb = x[j][z | (1 << f)];
               const float2 aa = f == 0 ? times(al, x[j][z]) : x[j][z];
-              hk[(uint32_t)((z & ((1 << f) - 1)) | ((z >> (f + 1)) << f)) << b] = bb;
+              if constexpr (B0)
+                hv[hz] = bb;
+              else
+                hk[f][hn | ((uint32_t)hz << b)] = bb;
               x[j][z] = phi_of(aa, bb, c[f]);
-              const float2 o1 = flip_sign(phi_of(aa, bb, c1[f]), (zs >> z) << 31);
-              x[j][z | (1 << f)] = dead[f] ? make_float2(0.f, 0.f) : o1;
+              x[j][z | (1 << f)] = keep_flip(phi_of(aa, bb, c1[f]), keep[f], (zs << (31 - z)) & (keep[f] & 0x80000000u));
+            }
+            if constexpr (B0) {
+#pragma unroll
+              for (int z = 0; z < Z / 2; z += 2)
+                *reinterpret_cast<float4 *>(hk[f] + (hn | (uint32_t)z)) =
+                    make_float4(hv[z].x, hv[z].y, hv[z + 1].x, hv[z + 1].y);
             }
           }
 #pragma unroll
           for (int z = 0; z < Z; ++z) {
-            acc[0][0] += norm2(x[j][z]);
-            *dst(s | ((uint32_t)z << b)) = x[j][z];
+            add_norm(acc[0][0], x[j][z]);
+            const uint32_t zb = sn | ((uint32_t)z << b);
+            if constexpr (B0) {
+              if (z & 1) continue;
+              *reinterpret_cast<float4 *>(home_at(l0 ^ wide_place(zb))) =
+                  make_float4(x[j][z].x, x[j][z].y, x[j][z | 1].x, x[j][z | 1].y);
+            } else if constexpr (jn.value)
+              *any(s0 | zb) = x[j][z];
+            else
+              *home_at(l0 ^ wide_place(zb)) = x[j][z];
           }
         }
       }
@@ -624,7 +719,8 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         const float2 c = times(al, s_coef[k]), c1 = flip_sign(c, (mask & 1u) << 31);
         float2 *hk = hist_of(k);
         for (uint32_t m = h_lo + tid; m < h_lo + NS / 2; m += BT) {
-          const float2 aa = times(al, *home(2 * m)), bb = *home(2 * m + 1);
+          const float4 v = *reinterpret_cast<const float4 *>(home(2 * m));
+          const float2 aa = times(al, make_float2(v.x, v.y)), bb = make_float2(v.z, v.w);
           hk[m] = bb;
           const float2 o0 = phi_of(aa, bb, c);
           float2 o1 = flip_sign(phi_of(aa, bb, c1), sign_of((2 * m) | (1u << (W - 1)), mask));
@@ -635,24 +731,26 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         }
         moved = true;
       } else if (CS > 1 && p - 1 >= SB) {
-        fwd(One{}, any, any, k, al, acc);
+        fwd(One{}, No{}, No{}, Yes{}, k, al, acc);
       } else {
         if (p - 1 + FMAX <= SB && k + FMAX <= M) f = FMAX;
         if (f == FMAX) {
-          if (moved)
-            fwd(Max{}, scr, home, k, al, acc);
+          if (moved)  // p = 1
+            fwd(Max{}, Yes{}, Yes{}, No{}, k, al, acc);
+          else if (p == 1)
+            fwd(Max{}, Yes{}, No{}, No{}, k, al, acc);
           else
-            fwd(Max{}, home, home, k, al, acc);
+            fwd(Max{}, No{}, No{}, No{}, k, al, acc);
         } else {
           if (moved)
-            fwd(One{}, scr, home, k, al, acc);
+            fwd(One{}, Yes{}, Yes{}, No{}, k, al, acc);
           else
-            fwd(One{}, home, home, k, al, acc);
+            fwd(One{}, No{}, No{}, No{}, k, al, acc);
         }
         moved = false;
       }
       k += f;
-      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
+      block_sum_pair<VW, 1>(acc, sum, red, par);
       cluster_sum<CS, 1>(sum, cred, cpar);
       nrm = (s_mask[k - 1] & kDead) ? sum[0] : 2.f * sum[0];
     }
@@ -677,7 +775,7 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         acc[0][0] += norm2(v0);
         acc[0][1] += norm2(v1);
       }
-      block_sum_pair<VW, 1>(acc, sum, red, par, 0);
+      block_sum_pair<VW, 1>(acc, sum, red, par);
       cluster_sum<CS, 1>(sum, cred, cpar);
       nrm = dead_l ? sum[0] : 2.f * sum[0];
     }
@@ -698,11 +796,16 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
     float loss_term = 0.f, w0, w1, w2, w3;  // the seed's factors
     {
       float pv[2][2] = {}, ps[2];  // <t|u_M>, or Re <u_M|g>
-      for (uint32_t i = 2 * q_lo + 2 * tid; i < 2 * q_lo + 2 * NS; i += TPR) {
+      const uint32_t i0 = 2 * q_lo + 2 * tid;
+      const uint32_t ot[2] = {(uint32_t)gather_bits(i0, G.out_bits, n_out), (uint32_t)gather_bits(i0 + 1, G.out_bits, n_out)};
+      uint32_t on = 0;
+      for (uint32_t n = 0; n < 2 * NS / TPR; ++n) {  // the output index by halves, as the input's
+        if ((n & 31u) == 0) on = (uint32_t)gather_bits((n + (tid & 31)) * TPR, G.out_bits, n_out);
+        const uint32_t oj = __shfl_sync(0xffffffffu, on, n & 31), i = i0 + n * TPR;
 #pragma unroll
         for (uint32_t z = 0; z < 2; ++z) {
           if ((i + z) & ~G.out_mask) continue;
-          const float2 t = row[gather_bits(i + z, G.out_bits, n_out)], a = out_of(i + z);
+          const float2 t = row[ot[z] ^ oj], a = out_of(i + z);
           if (fid) {
             pv[0][z] += t.x * a.x + t.y * a.y;
             pv[1][z] += t.x * a.y - t.y * a.x;
@@ -711,7 +814,7 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
           }
         }
       }
-      block_sum_pair<VW, 2>(pv, ps, red, par, 0);
+      block_sum_pair<VW, 2>(pv, ps, red, par);
       cluster_sum<CS, 2>(ps, cred, cpar);
       if (fid) {
         w0 = ps[0] * inv;
@@ -726,9 +829,9 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         w3 = ps[0] * inv * inv;
       }
     }
-    auto seed_of = [&](uint32_t i, float2 a) {
+    auto seed_of = [&](uint32_t i, uint32_t o, float2 a) {  // i, its output index
       if (i & ~G.out_mask) return make_float2(0.f, 0.f);
-      const float2 t = row[gather_bits(i, G.out_bits, n_out)];
+      const float2 t = row[o];
       if (fid)  // lambda = (2/J)(F z - a t) / |u_M|
         return make_float2(w2 * (w3 * a.x - (w0 * t.x - w1 * t.y)), w2 * (w3 * a.y - (w0 * t.y + w1 * t.x)));
       return make_float2(inv * (t.x - w3 * a.x), inv * (t.y - w3 * a.y));
@@ -750,39 +853,52 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
       for (uint32_t o = tid * 128u; o < (uint32_t)NS * 4u; o += BT * 128u)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(h + o));
     };
-    // lambda_k's other half, mu_k and lambda_{k-1} = al mu_k of a pair
-    auto pair_back = [&](float2 a, float2 b, float2 cn, float al, bool dead, uint32_t s0, uint32_t s1, float2 &m0,
-                         float2 &m1) {
-      const float2 ca = conj_mul(cn, a);
-      if (dead) {
-        m0 = times(al, a);
-        m1 = times(al, ca);
-      } else {
-        m0 = times(al, plus(a, b, s0));
-        m1 = times(al, plus(ca, conj_mul(cn, b), s1));
+    // mu_k and lambda_{k-1} = al mu_k of a pair of lambda_k (a and b, and their
+    // copies conj(cn) a, conj(cn) b): al and the signs ride on the factors, exact
+    auto pair_back = [&](float2 a, float2 b, float2 cn, float2 acn, float al, bool dead, uint32_t s0, uint32_t s1,
+                         float2 &m0, float2 &m1) {
+      m0 = times(al, a);
+      m1 = conj_mul(acn, a);
+      if (!dead) {
+        const float2 cb = conj_mul(cn, b);
+        const float f0 = sign_f(al, s0), f1 = sign_f(al, s1);
+        m0 = make_float2(fmaf(f0, b.x, m0.x), fmaf(f0, b.y, m0.y));
+        m1 = make_float2(fmaf(f1, cb.x, m1.x), fmaf(f1, cb.y, m1.y));
       }
     };
-    auto finish = [&](int k, const float (&t)[2][2], int p) {
-      float ts[2];
-      block_sum_pair<VW, 2>(t, ts, red, par, p);
-      cluster_sum<CS, 2>(ts, cred, cpar);
-      // kept in the history this step has finished with
-      if (tid == 0 && crank == 0) hist_of(k)[0] = make_float2(ts[0], ts[1]);
+    // the warps' sums of a step's gradient terms, added up at the run's end; the
+    // barrier orders the window (all: between the cluster's blocks as well)
+    auto finish = [&](int k, const float (&t)[2][2], int p, bool all) {
+      float *pk = reinterpret_cast<float *>(part + ((size_t)k * CS + crank) * VW);
+      warp_sums_pair<2>(t, p, [&](int j, int w, float a) { pk[2 * w + j] = a; });
+      if (CS > 1 && all)
+        run_barrier<CS>();
+      else
+        __syncthreads();
     };
     {  // the last step, from the seed
       const int k = M - 1;
       const float al = RealBits<float>::pow2(-s_expo[k]);
       float t[2][2] = {};
-      for (uint32_t q = q_lo + 2 * tid; q < q_lo + NS; q += TPR) {
+      uint32_t ot[2], on = 0;
+#pragma unroll
+      for (uint32_t z = 0; z < 2; ++z)
+        ot[z] = (uint32_t)gather_bits(wide_insert_bit(q_lo + 2 * tid + z, pl), G.out_bits, n_out);
+      const uint32_t op = (uint32_t)gather_bits(1u << pl, G.out_bits, n_out);
+      for (uint32_t n = 0; n < NS / TPR; ++n) {
+        const uint32_t q = q_lo + 2 * tid + n * TPR;
+        if ((n & 31u) == 0)
+          on = (uint32_t)gather_bits(wide_insert_bit((n + (tid & 31)) * TPR, pl), G.out_bits, n_out);
+        const uint32_t oj = __shfl_sync(0xffffffffu, on, n & 31);
         float2 m[2];
 #pragma unroll
         for (uint32_t z = 0; z < 2; ++z) {
           const uint32_t i0 = wide_insert_bit(q + z, pl), i1 = i0 | (1u << pl);
           const float2 v = *now(q + z);
-          m[z] = seed_of(i0, v);
+          m[z] = seed_of(i0, ot[z] ^ oj, v);
           if (!dead_l) {
             const uint32_t s1 = sign_of(i1, mask_l);
-            m[z] = plus(m[z], seed_of(i1, flip_sign(v, s1)), s1);
+            m[z] = plus(m[z], seed_of(i1, ot[z] ^ oj ^ op, flip_sign(v, s1)), s1);
           }
           m[z] = times(al, m[z]);
           add_t(t, z, m[z], hist_at(k, q + z));
@@ -791,14 +907,14 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         *home(q + 1) = m[1];
       }
       if (k > 1) prefetch(k - 1);
-      finish(k, t, 0);
+      finish(k, t, 0, true);
     }
     moved = false;
     // lambda of step k, pairs on bit p (below w - 1), the sums to follow
-    auto bwd = [&](auto &&src, auto &&dst, int k, float al, float2 cn, uint32_t mask) {
+    auto bwd = [&](auto &&src, auto &&dst, int k, float al, float2 cn, float2 acn, uint32_t mask) {
       constexpr int CNT = NS / 2 / BT, U = CNT < Cfg::U ? CNT : Cfg::U;
       const int p = k % W;
-      const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid;
+      const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid, qt = wide_insert_bit(r0, p);
       const bool dead = (mask & kDead) != 0u;
       const uint32_t z1 = ((mask >> (p + 1)) & 1u) << 31;
       const uint32_t st = sign_of(((r0 >> p) << (p + 2)) | (r0 & low) | (1u << p), mask);
@@ -806,16 +922,16 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         float2 x[U], y[U];
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-          const uint32_t q0 = wide_insert_bit(r0 + (uint32_t)(n + j) * BT, p);
+          const uint32_t q0 = qt | wide_insert_bit((uint32_t)(n + j) * BT, p);
           x[j] = *src(q0);
           y[j] = *src(q0 | (1u << p));
         }
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-          const uint32_t rn = (uint32_t)(n + j) * BT, q0 = wide_insert_bit(r0 + rn, p);
+          const uint32_t rn = (uint32_t)(n + j) * BT, q0 = qt | wide_insert_bit(rn, p);
           const uint32_t s0 = st ^ sign_of(((rn >> p) << (p + 2)) | (rn & low), mask);
           float2 m0, m1;
-          pair_back(x[j], y[j], cn, al, dead, s0, s0 ^ z1, m0, m1);
+          pair_back(x[j], y[j], cn, acn, al, dead, s0, s0 ^ z1, m0, m1);
           *dst(q0) = m0;
           *dst(q0 | (1u << p)) = m1;
         }
@@ -823,11 +939,12 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
     };
     for (int k = M - 2; k >= 0; --k) {
       const float al = RealBits<float>::pow2(-s_expo[k]);
-      const float2 cn = s_coef[k + 1];
+      const float2 cn = s_coef[k + 1], acn = times(al, cn);
       const uint32_t mask = s_mask[k];
       const bool dead = (mask & kDead) != 0u;
       const int p = k % W;
       float t[2][2] = {};
+      const bool next_joins = p == 0 || p - 1 >= SB;  // step k - 1 reaches into other slices
       if (k > 1) prefetch(k - 1);
       if (p == W - 1) {  // the slots move
         for (uint32_t m = h_lo + tid; m < h_lo + NS / 2; m += BT) {
@@ -835,53 +952,61 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
           const float2 h0 = hist_at(k, 2 * m), h1 = hist_at(k, 2 * m + 1);
           const uint32_t s0 = sign_of((2 * m) | (1u << (W - 1)), mask);
           float2 m0, m1;
-          pair_back(a, b, cn, al, dead, s0, s0 ^ ((mask & 1u) << 31), m0, m1);
+          pair_back(a, b, cn, acn, al, dead, s0, s0 ^ ((mask & 1u) << 31), m0, m1);
           add_t(t, 0, m0, h0);
           add_t(t, 1, m1, h1);
-          *scr(2 * m) = m0;
-          *scr(2 * m + 1) = m1;
+          *reinterpret_cast<float4 *>(scr(2 * m)) = make_float4(m0.x, m0.y, m1.x, m1.y);
         }
         moved = true;
-        finish(k, t, 0);
+        finish(k, t, 0, true);
       } else if (p < LT) {
         auto direct = [&](auto first) {
           constexpr int CNT = NS / 2 / BT, U = CNT < Cfg::U ? CNT : Cfg::U;
           const int pp = p ? p - 1 : W - 2;
-          const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid;
+          const uint32_t low = (1u << p) - 1u, r0 = h_lo + tid, qt = wide_insert_bit(r0, p);
           const uint32_t z1 = ((mask >> (p + 1)) & 1u) << 31;
           const uint32_t it = ((r0 >> p) << (p + 2)) | (r0 & low) | (1u << p);
           const uint32_t st = sign_of(it, mask);
-          const float2 *hk = hist_of(k);
+          const float2 *hk = hist_of(k) + (first.value ? qt : wide_remove_bit(qt, pp));
+          const uint32_t hp = first.value ? 1u << p : wide_remove_bit(1u << p, pp);
           const uint32_t hm = first.value ? 0u : s_mask[k - 1];
           const uint32_t hz = ((hm >> (p + 1)) & 1u) << 31;
           const uint32_t ht = sign_of(it, hm);
-          const bool gone = (hm & kDead) != 0u;
+          const float live = (hm & kDead) ? 0.f : 1.f;
+          const uint32_t l0 = wide_place(qt & (NS - 1)), lp = wide_place(1u << p);
           for (int n = 0; n < CNT; n += U) {
             float2 x[U], y[U], h0[U], h1[U];
 #pragma unroll
             for (int j = 0; j < U; ++j) {
-              const uint32_t q0 = wide_insert_bit(r0 + (uint32_t)(n + j) * BT, p), q1 = q0 | (1u << p);
-              h0[j] = hk[first.value ? q0 : wide_remove_bit(q0, pp)];
-              h1[j] = hk[first.value ? q1 : wide_remove_bit(q1, pp)];
-              x[j] = *home(q0);
-              y[j] = *home(q1);
+              const uint32_t qn = wide_insert_bit((uint32_t)(n + j) * BT, p);
+              const uint32_t hn = first.value ? qn : wide_remove_bit(qn, pp);
+              h0[j] = hk[hn];
+              h1[j] = hk[hn | hp];
+              const uint32_t e = l0 ^ wide_place(qn);
+              float2 *hb = slice_at(qn);
+              x[j] = hb[e];
+              y[j] = hb[e ^ lp];
             }
 #pragma unroll
             for (int j = 0; j < U; ++j) {
-              const uint32_t rn = (uint32_t)(n + j) * BT, q0 = wide_insert_bit(r0 + rn, p);
+              const uint32_t rn = (uint32_t)(n + j) * BT, q0 = qt | wide_insert_bit(rn, p);
               const uint32_t in_ = ((rn >> p) << (p + 2)) | (rn & low);
               const uint32_t s0 = st ^ sign_of(in_, mask);
               float2 m0, m1;
-              pair_back(x[j], y[j], cn, al, dead, s0, s0 ^ z1, m0, m1);
-              if (!first.value && ((q0 >> pp) & 1u)) {
-                const uint32_t g0 = ht ^ sign_of(in_, hm);
-                h0[j] = gone ? make_float2(0.f, 0.f) : flip_sign(h0[j], g0);
-                h1[j] = gone ? make_float2(0.f, 0.f) : flip_sign(h1[j], g0 ^ hz);
+              pair_back(x[j], y[j], cn, acn, al, dead, s0, s0 ^ z1, m0, m1);
+              float f0 = 1.f, f1 = 1.f;
+              if constexpr (!first.value) {
+                if ((q0 >> pp) & 1u) {  // the copy on the entered qubit's bit
+                  f0 = sign_f(live, ht ^ sign_of(in_, hm));
+                  f1 = sign_f(f0, hz);
+                }
               }
-              add_t(t, 0, m0, h0[j]);
-              add_t(t, 1, m1, h1[j]);
-              *home(q0) = m0;
-              *home(q0 | (1u << p)) = m1;
+              add_ts(t, 0, m0, h0[j], f0);
+              add_ts(t, 1, m1, h1[j], f1);
+              const uint32_t e = l0 ^ wide_place(wide_insert_bit(rn, p));
+              float2 *hb = slice_at(wide_insert_bit(rn, p));
+              hb[e] = m0;
+              hb[e ^ lp] = m1;
             }
           }
         };
@@ -889,24 +1014,88 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
           direct(Yes{});
         else
           direct(No{});
-        finish(k, t, p);
+        finish(k, t, p, next_joins);
+      } else if (p < SB && p < LT + 3) {
+        // the two entries of a pair are 2^G apart in one thread's order: groups of
+        // 2^(G + 1) of its entries, two threads' worth (v = 2 tid, 2 tid + 1) at once
+        auto ordered = [&](auto gc, auto &&src) {
+          constexpr int GB = decltype(gc)::value, P = 1 << GB, CNT = NS / TPR / (2 * P);
+          constexpr int pb = LT + GB;  // p
+          const uint32_t v0 = q_lo + 2 * tid, hm = s_mask[k - 1];
+          const uint32_t zz = (mask & 1u) << 31, z1 = ((mask >> (pb + 1)) & 1u) << 31;
+          const uint32_t hz = (hm & 1u) << 31, h1 = ((hm >> (pb + 1)) & 1u) << 31;
+          const uint32_t it = wide_insert_bit(v0, pb) | (1u << pb), st = sign_of(it, mask), ht = sign_of(it, hm);
+          const float live = (hm & kDead) ? 0.f : 1.f;
+          const float4 *hk = reinterpret_cast<const float4 *>(hist_of(k)) + (wide_remove_bit(v0, pb - 1) >> 1);
+          for (int gi = 0; gi < CNT; ++gi) {
+            float4 x[2 * P], h[2 * P];
+#pragma unroll
+            for (int j = 0; j < 2 * P; ++j) {
+              const uint32_t qn = (uint32_t)(gi * 2 * P + j) * TPR;
+              h[j] = hk[wide_remove_bit(qn, pb - 1) >> 1];
+              x[j] = *reinterpret_cast<const float4 *>(src(v0 | qn));
+            }
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+              const uint32_t qn = (uint32_t)(gi * 2 * P + j) * TPR;
+              const uint32_t s0 = st ^ sign_of(wide_insert_bit(qn, pb), mask);
+              float2 m0, m1;
+              pair_back(make_float2(x[j].x, x[j].y), make_float2(x[j + P].x, x[j + P].y), cn, acn, al, dead, s0, s0 ^ z1, m0,
+                        m1);
+              float2 n0, n1;
+              pair_back(make_float2(x[j].z, x[j].w), make_float2(x[j + P].z, x[j + P].w), cn, acn, al, dead, s0 ^ zz,
+                        s0 ^ z1 ^ zz, n0, n1);
+              x[j] = make_float4(m0.x, m0.y, n0.x, n0.y);
+              x[j + P] = make_float4(m1.x, m1.y, n1.x, n1.y);
+              *reinterpret_cast<float4 *>(home(v0 | qn)) = x[j];
+              *reinterpret_cast<float4 *>(home(v0 | qn | (1u << pb))) = x[j + P];
+            }
+#pragma unroll
+            for (int j = 0; j < 2 * P; ++j) {
+              const uint32_t qn = (uint32_t)(gi * 2 * P + j) * TPR;
+              float f0 = 1.f, f1 = 1.f;
+              if (((v0 | qn) >> (pb - 1)) & 1u) {
+                f0 = sign_f(live, ht ^ sign_of(wide_insert_bit(qn & ~(1u << pb), pb), hm) ^ (j >= P ? h1 : 0u));
+                f1 = sign_f(f0, hz);
+              }
+              add_ts(t, 0, make_float2(x[j].x, x[j].y), make_float2(h[j].x, h[j].y), f0);
+              add_ts(t, 1, make_float2(x[j].z, x[j].w), make_float2(h[j].z, h[j].w), f1);
+            }
+          }
+        };
+        auto in_order = [&](auto gc) {
+          if constexpr (LT + decltype(gc)::value < SB) {
+            if (CS == 1 && moved)
+              ordered(gc, scr);
+            else
+              ordered(gc, home);
+          }
+        };
+        if (p == LT)
+          in_order(std::integral_constant<int, 0>{});
+        else if (p == LT + 1)
+          in_order(std::integral_constant<int, 1>{});
+        else
+          in_order(std::integral_constant<int, 2>{});
+        moved = false;
+        finish(k, t, 0, next_joins);
       } else {
         bool joined = false;
         if constexpr (CS > 1) {
           if (p >= SB) {  // after the slots moved (p = w - 2), always
             joined = true;
             if (moved)
-              bwd(scr, any, k, al, cn, mask);
+              bwd(scr, any, k, al, cn, acn, mask);
             else
-              bwd(any, any, k, al, cn, mask);
+              bwd(any, any, k, al, cn, acn, mask);
             run_barrier<CS>();
           }
         }
         if (!joined) {
           if (CS == 1 && moved)
-            bwd(scr, home, k, al, cn, mask);
+            bwd(scr, home, k, al, cn, acn, mask);
           else
-            bwd(home, home, k, al, cn, mask);
+            bwd(home, home, k, al, cn, acn, mask);
           __syncthreads();
         }
         moved = false;
@@ -914,7 +1103,7 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
         const int pp = p - 1;  // >= 1
         const uint32_t hm = s_mask[k - 1], r0 = q_lo + 2 * tid;
         const uint32_t hz = (hm & 1u) << 31;
-        const bool gone = (hm & kDead) != 0u;
+        const float live = (hm & kDead) ? 0.f : 1.f;
         const uint32_t ht = sign_of(wide_insert_bit(r0, p) | (1u << p), hm);
         const float4 *hk = reinterpret_cast<const float4 *>(hist_of(k));
         for (int n = 0; n < CNT; n += U) {
@@ -928,25 +1117,35 @@ __global__ void __launch_bounds__((WideHalfCfg<W, CS>::BT), (WideHalfCfg<W, CS>:
 #pragma unroll
           for (int j = 0; j < U; ++j) {
             const uint32_t qn = (uint32_t)(n + j) * TPR, q = r0 + qn;
-            float2 h0 = make_float2(h[j].x, h[j].y), h1 = make_float2(h[j].z, h[j].w);
+            float f0 = 1.f, f1 = 1.f;
             if ((q >> pp) & 1u) {
-              const uint32_t g0 = ht ^ sign_of(wide_insert_bit(qn, p), hm);
-              h0 = gone ? make_float2(0.f, 0.f) : flip_sign(h0, g0);
-              h1 = gone ? make_float2(0.f, 0.f) : flip_sign(h1, g0 ^ hz);
+              f0 = sign_f(live, ht ^ sign_of(wide_insert_bit(qn, p), hm));
+              f1 = sign_f(f0, hz);
             }
-            add_t(t, 0, make_float2(x[j].x, x[j].y), h0);
-            add_t(t, 1, make_float2(x[j].z, x[j].w), h1);
+            add_ts(t, 0, make_float2(x[j].x, x[j].y), make_float2(h[j].x, h[j].y), f0);
+            add_ts(t, 1, make_float2(x[j].z, x[j].w), make_float2(h[j].z, h[j].w), f1);
           }
         }
-        finish(k, t, 0);
+        finish(k, t, 0, next_joins);
       }
     }
+    run_barrier<CS>();
     if (crank == 0) {
-      __syncthreads();
       for (int k = tid; k < M; k += BT) {
         const int ai = s_aidx[k];
         if (ai < 0) continue;
-        const float2 c = s_coef[k], t01 = hist_of(k)[0];  // scaled by alpha_k
+        const float2 c = s_coef[k];
+        const float2 *pk = part + (size_t)k * CS * VW;
+        float2 t01 = make_float2(0.f, 0.f);  // scaled by alpha_k
+        for (int rk = 0; rk < CS; ++rk) {
+          float2 u = make_float2(0.f, 0.f);
+          for (int w = 0; w < VW; ++w) {
+            u.x += pk[rk * VW + w].x;
+            u.y += pk[rk * VW + w].y;
+          }
+          t01.x += u.x;
+          t01.y += u.y;
+        }
         const double g = (double)c.x * t01.y + (double)c.y * t01.x;  // alpha Im(c t)
         if (fid)
           atomicAdd(&A.grad[vrow * NA + ai], g);
