@@ -1,7 +1,16 @@
 // Wide-window statevector sweep (windows 8..30): the state streams through a
 // device workspace in passes of several fused steps.
 //
-// The window of every run is a 2^w complex64 vector in the workspace.  A pass
+// The window of every run is a 2^w complex64 vector in the workspace; windows
+// from 11 on keep half of it (HALF).  After step k the window is phi_k and its
+// signed copy on the entering qubit's bit, so phi_k's 2^(w-1) amplitudes say it
+// all, and step k turns a pair (a, b) of phi_{k-1} over the measured bit into
+//   phi_k[entered 0] = a + c b,  phi_k[entered 1] = s (a +- c b)
+// in place: qubit s of the schedule is stored at bit (s - 1) mod (w - 1), step k
+// works on bit (k - 1) mod (w - 1) with the signs of the qubit entered at k - 1.
+// Half the traffic between the L2 and the SMs and half the tiles, the same
+// arithmetic: grid 16 x 10, 64 runs 796 -> 633 us a call (passes 25 -> 22 us for
+// five high steps, 41 -> 34 us for ten), 14 x 10, 256 runs 656 -> 509 us.  A pass
 // applies consecutive steps to tiles whose lanes are index bits 0..4 (32
 // consecutive complex64: one fully coalesced 256-byte access per register):
 //   * windows >= 10, mixed pass: up to ten steps of the form high* low* high*
@@ -38,12 +47,13 @@ constexpr int kLowRegs = 3;     // extra register bits of a low pass
 struct StreamArgs {
   const DevStep *steps;  // this circuit's steps
   int W, M, n_in, n_out;
+  int S;                 // log2 of a run's amplitudes in the workspace: W - 1 (half) or W
   int64_t B;
   const double *angles;
   int64_t astride;
   const float2 *psi_in;
   int64_t istride;
-  float2 *state;   // [B][2^W]
+  float2 *state;   // [B][2^S]
   double *norms;   // [3][B]
   int32_t *expo;   // [B] total applied exponent
   int8_t in_bits[32];
@@ -72,6 +82,7 @@ struct MixDesc {
   int lbits[5];       // low bits of the nl low steps, in step order
   uint32_t mask[10];  // step masks (dead flag in bit 31)
   uint32_t ptab[10];  // sign pattern over the five register-side bits of each step
+  uint32_t cpl;       // HALF: bit j = step j's entering qubit is coupled to the measured one
   int nrng;           // tile bits: ranges of free index bits (>= 5, not registers)
   int rpos[6], rlen[6];
 };
@@ -80,6 +91,43 @@ __device__ __forceinline__ uint32_t scatter_bits(uint32_t v, const int *bits, in
   uint32_t r = 0;
   for (int i = 0; i < n; ++i) r |= ((v >> i) & 1u) << bits[i];
   return r;
+}
+
+// a pass step on register bit J (lower half amp = 1 unless GEN)
+template <bool GEN, int R, int J>
+__device__ __forceinline__ void pass_reg_step(float2 (&v)[R], float2 c, float amp, uint32_t ts, bool dead) {
+  if constexpr (GEN)
+    reg_step_g<float, R, J>(v, c, amp, ts, dead);
+  else
+    reg_step<float, R, J>(v, c, ts, dead);
+}
+// The same on a pair of phi_{k-1} that becomes a pair of phi_k (HALF): both halves
+// of the entered qubit, the second with the sign of its CZs and c1 = -c where one
+// of them is with the measured qubit.
+template <bool GEN, int R, int J>
+__device__ __forceinline__ void pass_half_step(float2 (&v)[R], float2 c, float amp, uint32_t flip, uint32_t ts,
+                                               bool dead) {
+  const float2 c1 = flip_sign(c, flip);
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    if (j & (1 << J)) continue;
+    const int jh = j | (1 << J);
+    const float2 x0 = v[j], x1 = v[jh];
+    float2 o;
+    if constexpr (GEN) {
+      v[j] = make_float2(amp * x0.x + c.x * x1.x - c.y * x1.y, amp * x0.y + c.x * x1.y + c.y * x1.x);
+      o = make_float2(amp * x0.x + c1.x * x1.x - c1.y * x1.y, amp * x0.y + c1.x * x1.y + c1.y * x1.x);
+    } else {
+      v[j] = make_float2(x0.x + c.x * x1.x - c.y * x1.y, x0.y + c.x * x1.y + c.y * x1.x);
+      o = make_float2(x0.x + c1.x * x1.x - c1.y * x1.y, x0.y + c1.x * x1.y + c1.y * x1.x);
+    }
+    v[jh] = sign_bit_flip(o, ts * (1u << (31 - jh)));
+  }
+  if (dead) {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (j & (1 << J)) v[j] = make_float2(0.f, 0.f);
+  }
 }
 
 // First window: amplitude idx = psi_in[x(idx)] * (-1)^Q(idx), x gathering
@@ -102,6 +150,11 @@ struct InitDesc {
   uint32_t smask;
 };
 
+//
+// HALF: phi_0 = v[0] + c_0 v[1] over window bit 0 (in S, the lowest) is written
+// instead, index idx >> 1; a block takes consecutive chunks, so that it makes the
+// coefficient of a run once.
+template <bool HALF, bool GEN>
 __global__ void __launch_bounds__(kInitThreads) stream_init(StreamArgs a, InitDesc id) {
   __shared__ uint32_t s_t[1 << kInitLo];
   __shared__ uint32_t s_dep[1 << (kInitLo - 5)];  // window bits of l >> 5
@@ -125,24 +178,59 @@ __global__ void __launch_bounds__(kInitThreads) stream_init(StreamArgs a, InitDe
   }
   const int hlog = a.W - K;
   const int64_t n_chunks = a.B << hlog;
-  for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+  const int lane = tid & 31;
+  const bool free_bit = lane < a.W && !((id.smask >> lane) & 1u);
+  const int hi_rank = __popc(~id.smask & ((1u << lane) - 1u));
+  const uint32_t my_cz = lane < a.W ? a.init_cz[lane] : 0u;
+  const int my_pos = lane < K ? id.pos[lane] : 0, my_in = lane < a.n_in ? a.in_bits[lane] : 0;
+  const uint32_t pos_cz = a.init_cz[my_pos];
+  __shared__ float s_c[3];
+  int64_t c_run = -1;
+  const int64_t c_lo = HALF ? blockIdx.x * n_chunks / gridDim.x : blockIdx.x;
+  const int64_t c_hi = HALF ? (blockIdx.x + 1) * n_chunks / gridDim.x : n_chunks;
+  for (int64_t c = c_lo; c < c_hi; c += HALF ? 1 : gridDim.x) {
     const int64_t run = c >> hlog;
-    uint32_t hi = 0;  // chunk bits deposited on the window bits outside S
-    for (int q = 0, t = 0; q < a.W; ++q)
-      if (!((id.smask >> q) & 1u)) hi |= (uint32_t)((c >> t++) & 1) << q;
-    uint32_t acc = 0;
-    for (int q = 0; q < a.W; ++q)
-      if ((hi >> q) & 1u) acc ^= a.init_cz[q];
-    uint32_t m = 0;
-    for (int i = 0; i < K; ++i) m |= (((acc >> id.pos[i]) ^ (uint32_t)__popc(hi & a.init_cz[id.pos[i]])) & 1u) << i;
-    const uint32_t qhi = init_parity(hi, a.init_cz, a.W);
-    const uint32_t xhi = (uint32_t)gather_bits(hi, a.in_bits, a.n_in);
+    if (HALF && run != c_run) {
+      __syncthreads();
+      if (tid == 0) {
+        const DevStep st = a.steps[0];
+        const double th = st.aidx >= 0 ? a.angles[run * a.astride + st.aidx] : st.fixed;
+        float2 co, ph;
+        float amp = 1.f;
+        if constexpr (GEN)
+          sv_coef_gen(st.plane, th, false, co, amp, ph);
+        else
+          sv_coef(st.plane, th, false, co, ph);
+        s_c[0] = co.x;
+        s_c[1] = co.y;
+        s_c[2] = amp;
+      }
+      c_run = run;
+      __syncthreads();
+    }
+    // a bit of each per lane: the chunk bits on the window bits outside S, the
+    // couplings and signs they make, their input index
+    const uint32_t hi = __ballot_sync(0xffffffffu, free_bit && ((c >> hi_rank) & 1));
+    const uint32_t acc = __reduce_xor_sync(0xffffffffu, (hi >> lane) & 1u ? my_cz : 0u);
+    const uint32_t m = __ballot_sync(0xffffffffu, lane < K && (((acc >> my_pos) ^ (uint32_t)__popc(hi & pos_cz)) & 1u));
+    const uint32_t qhi = (uint32_t)__popc(__ballot_sync(0xffffffffu, ((hi >> lane) & 1u) && (__popc(hi & my_cz) & 1))) & 1u;
+    const uint32_t xhi = a.n_in ? __brev(__ballot_sync(0xffffffffu, lane < a.n_in && ((hi >> my_in) & 1u))) >> (32 - a.n_in) : 0u;
     const float2 *in = a.psi_in + (a.istride ? run * a.istride : 0);
-    float2 *out = a.state + (run << a.W) + hi;
-    for (int l = tid; l < (1 << K); l += kInitThreads) {
+    float2 *out = a.state + (run << a.S) + (HALF ? hi >> 1 : hi);
+    auto entry = [&](int l) {
       const uint32_t t = s_t[l];
       const uint32_t par = qhi ^ (t >> 31) ^ (__popc((uint32_t)l & m) & 1u);
-      out[(uint32_t)(l & 31) | s_dep[l >> 5]] = flip_sign(__ldg(in + (xhi | (t & 0x7fffffffu))), par << 31);
+      return flip_sign(__ldg(in + (xhi | (t & 0x7fffffffu))), par << 31);
+    };
+    if constexpr (HALF) {
+      const float2 co = make_float2(s_c[0], s_c[1]);
+      for (int l = 2 * tid; l < (1 << K); l += 2 * kInitThreads) {
+        float2 v[2] = {entry(l), entry(l + 1)};
+        pass_reg_step<GEN, 2, 0>(v, co, s_c[2], 0u, false);
+        out[((uint32_t)(l & 31) | s_dep[l >> 5]) >> 1] = v[0];
+      }
+    } else {
+      for (int l = tid; l < (1 << K); l += kInitThreads) out[(uint32_t)(l & 31) | s_dep[l >> 5]] = entry(l);
     }
   }
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + tid; r < a.B; r += (int64_t)gridDim.x * blockDim.x) {
@@ -238,14 +326,6 @@ __device__ __forceinline__ float2 bcast(float2 c, int j) {
   return make_float2(__shfl_sync(0xffffffffu, c.x, j), __shfl_sync(0xffffffffu, c.y, j));
 }
 
-// a pass step on register bit J (lower half amp = 1 unless GEN)
-template <bool GEN, int R, int J>
-__device__ __forceinline__ void pass_reg_step(float2 (&v)[R], float2 c, float amp, uint32_t ts, bool dead) {
-  if constexpr (GEN)
-    reg_step_g<float, R, J>(v, c, amp, ts, dead);
-  else
-    reg_step<float, R, J>(v, c, ts, dead);
-}
 template <bool GEN, int R, int Q>
 __device__ __forceinline__ void pass_lane_step(float2 (&v)[R], float2 c, float amp, uint32_t ts, bool dead,
                                                int lane) {
@@ -489,15 +569,15 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // 16-byte asynchronous copies).  A bulk-copy wait that exceeds its bound
 // poisons the warp's tiles with NaN (the runs end with status MBQC_RUN_NAN)
 // after a bounded wait for the copies still in flight.
-template <bool TMA, bool GEN>
-__global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a, MixDesc d) {
+template <bool TMA, bool GEN, bool HALF>
+__global__ void __launch_bounds__(32 * kMixWarps, HALF ? 7 : 1) stream_pass_mixed(StreamArgs a, MixDesc d) {
   extern __shared__ __align__(16) float2 s_mix[];  // [warp][2][32 rows x 34]
   __shared__ __align__(8) uint64_t s_mbar[kMixWarps][2];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int BUF = TMA ? kMixBuf : 1024;  // float2 per tile buffer
   float2 *buf = s_mix + (size_t)wid * 2 * BUF;
   uint64_t *mbar = s_mbar[wid];
-  const int tlog = a.W - 10;
+  const int tlog = a.S - 10;
   const int64_t n_tiles = a.B << tlog;
   const int64_t n_warps = (int64_t)gridDim.x * kMixWarps;
   const int64_t w = (int64_t)blockIdx.x * kMixWarps + wid;
@@ -531,10 +611,10 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
     if constexpr (TMA) {  // lane r copies row r of tile g
       if (lane == 0) mbar_expect_tx(&mbar[b], 32 * 256);
       __syncwarp();
-      const float2 *src = a.state + ((g >> tlog) << a.W) + (tile_bits(g) | lane_roff);
+      const float2 *src = a.state + ((g >> tlog) << a.S) + (tile_bits(g) | lane_roff);
       bulk_row_copy(dst + lane * kMixRow, src, 256, &mbar[b]);
     } else {  // lane: pair lane & 15 of rows 2i + (lane >> 4)
-      const float2 *st = a.state + ((g >> tlog) << a.W) + tile_bits(g);
+      const float2 *st = a.state + ((g >> tlog) << a.S) + tile_bits(g);
       const int pr = lane & 15;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -604,8 +684,11 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
       constexpr int J = decltype(jc)::value;
       const uint32_t m = d.mask[j];
       const uint32_t ts = d.ptab[j] ^ (0u - (__popc(nbase & m & ~kDead) & 1u));
-      pass_reg_step<GEN, 32, J>(v, bcast(cl, j), GEN ? __shfl_sync(0xffffffffu, al, j) : 1.f, ts,
-                                (m & kDead) != 0u);
+      const float am = GEN ? __shfl_sync(0xffffffffu, al, j) : 1.f;
+      if constexpr (HALF)
+        pass_half_step<GEN, 32, J>(v, bcast(cl, j), am, (d.cpl >> j) << 31, ts, (m & kDead) != 0u);
+      else
+        pass_reg_step<GEN, 32, J>(v, bcast(cl, j), am, ts, (m & kDead) != 0u);
     };
 #define MBQC_MSTEP(J) \
   if (J < d.n1) hstep(std::integral_constant<int, J>{}, J);
@@ -631,12 +714,20 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
         const float2 c = bcast(cl, js);
         const float am = GEN ? __shfl_sync(0xffffffffu, al, js) : 1.f;
         const bool dead = (m & kDead) != 0u;
+        const uint32_t flip = HALF ? (d.cpl >> js) << 31 : 0u;
+        auto lstep = [&](auto qc) {
+          constexpr int Q = decltype(qc)::value;
+          if constexpr (HALF)
+            pass_half_step<GEN, 32, Q>(v, c, am, flip, ts, dead);
+          else
+            pass_reg_step<GEN, 32, Q>(v, c, am, ts, dead);
+        };
         switch (d.lbits[j]) {
-          case 0: pass_reg_step<GEN, 32, 0>(v, c, am, ts, dead); break;
-          case 1: pass_reg_step<GEN, 32, 1>(v, c, am, ts, dead); break;
-          case 2: pass_reg_step<GEN, 32, 2>(v, c, am, ts, dead); break;
-          case 3: pass_reg_step<GEN, 32, 3>(v, c, am, ts, dead); break;
-          default: pass_reg_step<GEN, 32, 4>(v, c, am, ts, dead); break;
+          case 0: lstep(std::integral_constant<int, 0>{}); break;
+          case 1: lstep(std::integral_constant<int, 1>{}); break;
+          case 2: lstep(std::integral_constant<int, 2>{}); break;
+          case 3: lstep(std::integral_constant<int, 3>{}); break;
+          default: lstep(std::integral_constant<int, 4>{}); break;
         }
       }
       __syncwarp();  // back to the normal layout
@@ -655,7 +746,7 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
     MBQC_MSTEP(3)
     MBQC_MSTEP(4)
 #undef MBQC_MSTEP
-    float2 *st = a.state + (run << a.W);
+    float2 *st = a.state + (run << a.S);
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
       part += v[r].x * v[r].x + v[r].y * v[r].y;
@@ -673,7 +764,7 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
     mbar_wait(&mbar[1], parity[1]);
     const float2 bad = make_float2(NAN, NAN);
     for (int64_t g = g0; g < g1; ++g) {
-      float2 *st = a.state + ((g >> tlog) << a.W);
+      float2 *st = a.state + ((g >> tlog) << a.S);
       const uint32_t nbase = tile_bits(g) | (uint32_t)lane;
       for (int r = 0; r < 32; ++r) st[nbase | roff(r)] = bad;
     }
@@ -684,9 +775,11 @@ __global__ void __launch_bounds__(32 * kMixWarps) stream_pass_mixed(StreamArgs a
 
 // Epilogue: normalise (float-pair sums: FP64-level accuracy), apply the
 // reference global phase and write the outputs in the reference's order.
-// The outputs of a run are split into chunks of 2^K consecutive output
-// indices y (y bits 0..K-1 vary; their window bits, sorted, enumerate the
-// chunk so that reads follow the window order).  Two grid-wide kernels:
+// The outputs of a run are split into chunks of 2^K output indices y that differ
+// in a bit set T: bits 0..4 of y (runs of 32 consecutive outputs are written) and
+// the bits that lie on bits 0..4 of the state (runs of 32 amplitudes are read),
+// then the lowest others.  The chunk is enumerated in state order for reads and in
+// output order for writes.  Two grid-wide kernels:
 // stream_out_norm writes each chunk's partial squared norm (and, per run,
 // the phase product and the input norm); stream_out_write sums a run's
 // partials in a fixed order (deterministic), scales, and writes its chunk
@@ -695,15 +788,22 @@ constexpr int kOutLo = 10;
 constexpr int kOutThreads = 256;
 struct OutDesc {
   int K, nch_log;        // chunk bits; log2 of the chunks per run
-  uint32_t wlo[32], whi[32];  // window offset of chunk-local index bits 0..4 / 5..9 (window order)
-  uint16_t ylo[32], yhi[32];  // output offset of the same
-  int ywin[32];               // window bit of output bit j (j < n_out)
+  uint32_t wlo[32], whi[32];  // state offset of chunk-local index bits 0..4 / 5..9 (state order)
+  uint16_t ylo[32], yhi[32];  // chunk-local index in output order of the same
+  uint32_t yout[32];          // output offset of bits 5..9 of that index
+  int rest[32];               // the output bits outside T
+  int ywin[32];               // state bit of output bit j (j < n_out)
 };
 
-__device__ __forceinline__ uint32_t chunk_window_base(const OutDesc &od, int n_out, uint32_t y) {
+// state and output offset of chunk ch
+__device__ __forceinline__ uint32_t chunk_base(const OutDesc &od, uint32_t ch, uint32_t &y) {
   uint32_t w = 0;
-  for (int j = od.K; j < n_out; ++j)
-    if ((y >> j) & 1u) w |= 1u << od.ywin[j];
+  y = 0;
+  for (int i = 0; i < od.nch_log; ++i)
+    if ((ch >> i) & 1u) {
+      w |= 1u << od.ywin[od.rest[i]];
+      y |= 1u << od.rest[i];
+    }
   return w;
 }
 
@@ -730,8 +830,9 @@ __global__ void __launch_bounds__(kOutThreads) stream_out_norm(StreamArgs a, Out
   const int tid = threadIdx.x;
   if (tid < 64) s_w[tid] = tid < 32 ? od.wlo[tid] : od.whi[tid - 32];
   __syncthreads();
-  const uint32_t wbase = chunk_window_base(od, a.n_out, ch << od.K);
-  const float2 *st = a.state + (run << a.W) + wbase;
+  uint32_t y0;
+  const uint32_t wbase = chunk_base(od, ch, y0);
+  const float2 *st = a.state + (run << a.S) + wbase;
   float2 acc = make_float2(0.f, 0.f);
   for (int l = tid; l < (1 << od.K); l += kOutThreads) {
     const float2 x = st[s_w[l & 31] | s_w[32 + (l >> 5)]];
@@ -777,15 +878,16 @@ __global__ void __launch_bounds__(kOutThreads) stream_out_norm(StreamArgs a, Out
 __global__ void __launch_bounds__(kOutThreads) stream_out_write(StreamArgs a, OutDesc od, const float2 *part,
                                                        const float2 *phase, const double *nin, float2 *out,
                                                        int32_t lp_const, double *logprob, int32_t *status) {
-  __shared__ float2 s_buf[1 << kOutLo];
+  __shared__ float2 s_buf[(1 << kOutLo) + 32];  // a pad per 32: either order may go by 32
   __shared__ float2 s_n2;
-  __shared__ uint32_t s_w[64], s_y[64];
+  __shared__ uint32_t s_w[64], s_y[64], s_o[32];
   const int64_t run = blockIdx.x >> od.nch_log;
   const uint32_t ch = blockIdx.x & ((1u << od.nch_log) - 1u);
   const int tid = threadIdx.x, nch = 1 << od.nch_log;
   if (tid < 64) {
     s_w[tid] = tid < 32 ? od.wlo[tid] : od.whi[tid - 32];
     s_y[tid] = tid < 32 ? od.ylo[tid] : od.yhi[tid - 32];
+    if (tid < 32) s_o[tid] = od.yout[tid];
   }
   if (tid < 32) {  // the run's squared norm: its partials in a fixed order
     const float2 *pr = part + (run << od.nch_log);
@@ -804,13 +906,15 @@ __global__ void __launch_bounds__(kOutThreads) stream_out_write(StreamArgs a, Ou
   inv = ok ? inv * (1.5f - 0.5f * n2 * inv * inv) : NAN;  // one Newton step
   const float2 ph = phase[run];
   const float2 sc = make_float2(ph.x * inv, ph.y * inv);
-  const uint32_t y0 = ch << od.K;
-  const float2 *st = a.state + (run << a.W) + chunk_window_base(od, a.n_out, y0);
+  uint32_t y0;
+  const uint32_t wbase = chunk_base(od, ch, y0);
+  const float2 *st = a.state + (run << a.S) + wbase;
+  auto pad = [](uint32_t i) { return i + (i >> 5); };
   for (int l = tid; l < (1 << od.K); l += kOutThreads)
-    s_buf[s_y[l & 31] | s_y[32 + (l >> 5)]] = cmul(st[s_w[l & 31] | s_w[32 + (l >> 5)]], sc);
+    s_buf[pad(s_y[l & 31] | s_y[32 + (l >> 5)])] = cmul(st[s_w[l & 31] | s_w[32 + (l >> 5)]], sc);
   __syncthreads();
   float2 *o = out + (run << a.n_out) + y0;
-  for (int j = tid; j < (1 << od.K); j += blockDim.x) o[j] = s_buf[j];
+  for (int j = tid; j < (1 << od.K); j += blockDim.x) o[(uint32_t)(j & 31) | s_o[j >> 5]] = s_buf[pad(j)];
   if (ch == 0 && tid == 0) {
     if (status) status[run] = ok ? MBQC_RUN_OK : (isnan(n2) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
     if (logprob) {
@@ -820,15 +924,42 @@ __global__ void __launch_bounds__(kOutThreads) stream_out_write(StreamArgs a, Ou
   }
 }
 
-static OutDesc make_out_desc(const DevCircuit &hc) {
+// HALF: the workspace bit of the qubit at a window bit after `done` steps.  The
+// window holds the qubits done .. done + w - 1 of the schedule at bit (index mod w);
+// all but the last are stored, qubit s at bit (s - 1) mod (w - 1): the bit of the
+// measured qubit is the entering one's.
+static int half_bit(int pos, int done, int w) {
+  const int s = done + ((pos - done) % w + w) % w;
+  return (s - 1) % (w - 1);
+}
+
+static OutDesc make_out_desc(const DevCircuit &hc, bool half) {
   OutDesc od{};
   const int n_out = hc.n_out, K = n_out < kOutLo ? n_out : kOutLo;
   od.K = K;
   od.nch_log = n_out - K;
-  for (int j = 0; j < n_out; ++j) od.ywin[j] = hc.out_bits[n_out - 1 - j];  // output j is bit n_out-1-j of y
-  // chunk-local index bits in window order: the window bits of y bits 0..K-1, sorted
-  int order[kOutLo];
-  for (int i = 0; i < K; ++i) order[i] = i;
+  for (int j = 0; j < n_out; ++j) {  // output j is bit n_out-1-j of y
+    const int pos = hc.out_bits[n_out - 1 - j];
+    od.ywin[j] = half ? half_bit(pos, hc.n_steps, hc.w) : pos;
+  }
+  uint32_t T = 0;
+  for (int j = 0; j < 5 && j < n_out; ++j) T |= 1u << j;
+  for (int j = 0; j < n_out; ++j)
+    if (od.ywin[j] < 5 && __builtin_popcount(T) < K) T |= 1u << j;
+  for (int j = 0; j < n_out && __builtin_popcount(T) < K; ++j) T |= 1u << j;
+  int order[kOutLo], rank[32], nt = 0, nr = 0;
+  for (int j = 0; j < n_out; ++j) {
+    if ((T >> j) & 1u) {
+      rank[j] = nt;
+      order[nt++] = j;
+    } else {
+      od.rest[nr++] = j;
+    }
+  }
+  for (int v = 0; v < 32; ++v)
+    for (int i = 5; i < K; ++i)
+      if ((v >> (i - 5)) & 1) od.yout[v] |= 1u << order[i];
+  // chunk-local index bits in state order
   std::sort(order, order + K, [&](int p, int q) { return od.ywin[p] < od.ywin[q]; });
   for (int v = 0; v < 32; ++v) {
     uint32_t wl = 0, wh = 0;
@@ -837,11 +968,11 @@ static OutDesc make_out_desc(const DevCircuit &hc) {
       if (!((v >> i) & 1)) continue;
       if (i < K) {
         wl |= 1u << od.ywin[order[i]];
-        yl |= 1u << order[i];
+        yl |= 1u << rank[order[i]];
       }
       if (i + 5 < K) {
         wh |= 1u << od.ywin[order[i + 5]];
-        yh |= 1u << order[i + 5];
+        yh |= 1u << rank[order[i + 5]];
       }
     }
     od.wlo[v] = wl;
@@ -864,9 +995,13 @@ static uint32_t host_parity_table(uint32_t side) {
 // the form high* low* high* with at most five high and five low bits; the
 // register bits are the high bits in step order, padded with the lowest free
 // high bits
-static std::vector<MixDesc> make_mixed_passes(int W, int M, const DevStep *steps) {
+//
+// half: the steps after the first, step k on bit (k - 1) mod (w - 1) of the stored
+// half with the signs of the qubit entered at step k - 1, moved to the stored bits.
+static std::vector<MixDesc> make_mixed_passes(int w, int M, const DevStep *steps, bool half) {
   std::vector<MixDesc> out;
-  int k = 0;
+  const int W = half ? w - 1 : w, first = half ? 1 : 0;
+  int k = first;
   while (k < M) {
     MixDesc d{};
     int rbits[5] = {0, 0, 0, 0, 0};
@@ -874,7 +1009,7 @@ static std::vector<MixDesc> make_mixed_passes(int W, int M, const DevStep *steps
     d.index = (int)out.size();
     int phase = 0, nh = 0;  // phase 0: first high run, 1: low run, 2: second high run
     while (k < M) {
-      const int b = k % W;
+      const int b = (k - first) % W;
       if (b < kLowLanes) {
         if (phase == 2 || d.nl == 5) break;
         phase = 1;
@@ -901,7 +1036,19 @@ static std::vector<MixDesc> make_mixed_passes(int W, int M, const DevStep *steps
       used |= d.bv[i];
     }
     for (int j = 0; j < d.nsteps; ++j) {
-      const uint32_t m = steps[d.k0 + j].mask;
+      const int kj = d.k0 + j;
+      uint32_t m = 0;
+      bool own = false;
+      if (half) {
+        const uint32_t prev = steps[kj - 1].mask;
+        m = prev & kDead;
+        for (int q = kj + 1; q <= kj + w - 2; ++q)
+          if ((prev >> (q % w)) & 1u) m |= 1u << half_bit(q % w, kj, w);
+        if ((prev >> (kj % w)) & 1u) d.cpl |= 1u << j;
+        own = (prev >> ((kj - 1) % w)) & 1u;
+      } else {
+        m = steps[kj].mask;
+      }
       d.mask[j] = m;
       uint32_t side = 0;  // the step's mask bits on the register side of its layout
       if (j >= d.n1 && j < d.n1 + d.nl) {
@@ -910,7 +1057,7 @@ static std::vector<MixDesc> make_mixed_passes(int W, int M, const DevStep *steps
         for (int i = 0; i < 5; ++i)
           if (m & d.bv[i]) side |= 1u << i;
       }
-      d.ptab[j] = host_parity_table(side);
+      d.ptab[j] = host_parity_table(side) ^ (own ? ~0u : 0u);
     }
     for (int b = kLowLanes; b < W;) {  // free bits as ranges
       if ((used >> b) & 1u) {
@@ -949,16 +1096,23 @@ static std::vector<PassDesc> make_passes(int W, int M) {
   return out;
 }
 
-// workspace: state [B][2^w] | norms [3][B] | expo [B] | (16-byte aligned)
+// Half the window is kept (HALF) where it holds a whole mixed tile (windows >= 11)
+// and the last step lets no qubit in, so that the outputs are all in the half: every
+// plan whose window is wider than its outputs.
+static bool stream_half(const DevCircuit &hc, const DevStep *steps) {
+  return hc.w >= 11 && hc.n_steps >= 1 && (steps[hc.n_steps - 1].mask & kDead) != 0u;
+}
+
+// workspace: state [B][2^S] | norms [3][B] | expo [B] | (16-byte aligned)
 // epilogue partials [B][2^(n_out - K)] | phases [B] | input norms [B]
-static size_t stream_ws_head(int W, int64_t B) {
-  const size_t h = (size_t)B * ((size_t)1 << W) * sizeof(float2) + (size_t)3 * B * sizeof(double) +
+static size_t stream_ws_head(int S, int64_t B) {
+  const size_t h = (size_t)B * ((size_t)1 << S) * sizeof(float2) + (size_t)3 * B * sizeof(double) +
                    (size_t)B * sizeof(int32_t);
   return (h + 15) & ~(size_t)15;
 }
-static size_t stream_ws_bytes(const DevCircuit &hc, int64_t B) {
+static size_t stream_ws_bytes(const DevCircuit &hc, int S, int64_t B) {
   const int K = hc.n_out < kOutLo ? hc.n_out : kOutLo;
-  return stream_ws_head(hc.w, B) + ((size_t)B << (hc.n_out - K)) * sizeof(float2) + (size_t)B * sizeof(float2) +
+  return stream_ws_head(S, B) + ((size_t)B << (hc.n_out - K)) * sizeof(float2) + (size_t)B * sizeof(float2) +
          (size_t)B * sizeof(double) + 256;
 }
 
@@ -973,7 +1127,7 @@ int mbqc_sv_stream_workspace(const mbqc_plan *plan, int64_t batch, size_t *bytes
   const DevCircuit &hc = host_circuit(plan, 0);
   if (hc.w < kStreamMinWindow)
     return fail(MBQC_E_UNSUPPORTED, "stream_workspace: window %d < %d", hc.w, kStreamMinWindow);
-  *bytes = stream_ws_bytes(hc, batch);
+  *bytes = stream_ws_bytes(hc, hc.w - (stream_half(hc, host_steps(plan, 0)) ? 1 : 0), batch);
   return MBQC_OK;
 }
 
@@ -995,7 +1149,9 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
     return fail(MBQC_E_INVALID, "sv_forward_stream: bad angle array");
   if (in_stride != 0 && in_stride < ((int64_t)1 << hc.n_in))
     return fail(MBQC_E_INVALID, "sv_forward_stream: input stride too small");
-  const size_t need = stream_ws_bytes(hc, batch);
+  const bool half = stream_half(hc, host_steps(plan, 0));
+  const int S = hc.w - (half ? 1 : 0);
+  const size_t need = stream_ws_bytes(hc, S, batch);
   if (!workspace || workspace_bytes < need)
     return fail(MBQC_E_INVALID, "sv_forward_stream: workspace of %zu bytes, %zu needed", workspace_bytes,
                 need);
@@ -1003,6 +1159,7 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
   StreamArgs a{};
   a.steps = v.d_steps + hc.step_off;
   a.W = hc.w;
+  a.S = S;
   a.M = hc.n_steps;
   a.n_in = hc.n_in;
   a.n_out = hc.n_out;
@@ -1013,7 +1170,7 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
   a.istride = in_stride;
   char *ws = static_cast<char *>(workspace);
   a.state = reinterpret_cast<float2 *>(ws);
-  size_t off = (size_t)batch * ((size_t)1 << hc.w) * sizeof(float2);
+  size_t off = (size_t)batch * ((size_t)1 << S) * sizeof(float2);
   a.norms = reinterpret_cast<double *>(ws + off);
   off += (size_t)3 * batch * sizeof(double);
   a.expo = reinterpret_cast<int32_t *>(ws + off);
@@ -1026,7 +1183,8 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
   const InitDesc id = make_init_desc(hc);
   const int64_t chunks = batch << (hc.w - id.K);
   const int64_t blocks = std::min<int64_t>(std::max<int64_t>(chunks, (batch + 255) / 256), (int64_t)sm_count() * 8);
-  stream_init<<<(int)blocks, kInitThreads, 0, s>>>(a, id);
+  auto kinit = half ? (gen ? stream_init<true, true> : stream_init<true, false>) : stream_init<false, false>;
+  kinit<<<(int)blocks, kInitThreads, 0, s>>>(a, id);
   int rc = check_launch("stream_init");
   if (rc) return rc;
   // plain launches: as programmatic dependents these multi-wave passes ran
@@ -1034,8 +1192,12 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
   if (hc.w >= 10) {
     // persistent grid: as many blocks as are resident at once
     const bool tma = (flags & MBQC_F_STREAM_TMA) != 0u;
-    auto kmix = tma ? (gen ? stream_pass_mixed<true, true> : stream_pass_mixed<true, false>)
-                    : (gen ? stream_pass_mixed<false, true> : stream_pass_mixed<false, false>);
+    auto pick = [&](auto h) {
+      constexpr bool H = decltype(h)::value;
+      return tma ? (gen ? stream_pass_mixed<true, true, H> : stream_pass_mixed<true, false, H>)
+                 : (gen ? stream_pass_mixed<false, true, H> : stream_pass_mixed<false, false, H>);
+    };
+    auto kmix = half ? pick(std::true_type{}) : pick(std::false_type{});
     const size_t smem = (size_t)kMixWarps * 2 * (tma ? kMixBuf : 1024) * sizeof(float2);
     int occ = 0;
     rc = cuda_check(cudaFuncSetAttribute(kmix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1044,9 +1206,9 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
     rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kmix, 32 * kMixWarps, smem),
                     "stream_pass_mixed occupancy");
     if (rc) return rc;
-    const int64_t need = ((batch << (hc.w - 10)) + kMixWarps - 1) / kMixWarps;
+    const int64_t need = ((batch << (S - 10)) + kMixWarps - 1) / kMixWarps;
     const int64_t nb = std::min<int64_t>(need, (int64_t)sm_count() * std::max(occ, 1));
-    for (const MixDesc &d : make_mixed_passes(hc.w, hc.n_steps, host_steps(plan, 0))) {
+    for (const MixDesc &d : make_mixed_passes(hc.w, hc.n_steps, host_steps(plan, 0), half)) {
       kmix<<<(int)nb, 32 * kMixWarps, smem, s>>>(a, d);
       rc = check_launch("stream_pass_mixed");
       if (rc) return rc;
@@ -1067,8 +1229,8 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
       if (rc) return rc;
     }
   }
-  const OutDesc od = make_out_desc(hc);
-  char *ep = ws + stream_ws_head(hc.w, batch);
+  const OutDesc od = make_out_desc(hc, half);
+  char *ep = ws + stream_ws_head(S, batch);
   float2 *part = reinterpret_cast<float2 *>(ep);
   float2 *phase = part + ((size_t)batch << od.nch_log);
   double *nin = reinterpret_cast<double *>(phase + batch);
