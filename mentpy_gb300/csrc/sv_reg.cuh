@@ -95,10 +95,11 @@ __host__ __device__ constexpr int sv_al16(int b) { return (b + 15) & ~15; }
 __host__ __device__ constexpr bool sv_stage_ang(int ll, int kc) { return (32 >> ll) * kc * 8 <= 4096; }
 // Shared memory of one warp for a chunk of kc steps: coefficients [kc][runs],
 // amp [kc][runs] (general planes), CZ masks and register parity tables [kc],
-// input/output rows [runs][2^w] (when staged), angle rows [runs][<= kc].
+// input/output rows [runs][2^w] (when staged), angle rows [runs][<= kc]; each
+// part a multiple of 16 bytes, so that every warp's rows take 16-byte accesses.
 __host__ __device__ constexpr int sv_warp_smem(int w, int ll, int cplx_bytes, int kc, bool gen) {
   return sv_al16(kc * (32 >> ll) * cplx_bytes) + (gen ? sv_al16(kc * (32 >> ll) * cplx_bytes / 2) : 0) +
-         2 * sv_al16(kc * 4) + sv_io_bytes(w, ll, cplx_bytes) + (sv_stage_ang(ll, kc) ? (32 >> ll) * kc * 8 : 0);
+         2 * sv_al16(kc * 4) + sv_io_bytes(w, ll, cplx_bytes) + (sv_stage_ang(ll, kc) ? sv_al16((32 >> ll) * kc * 8) : 0);
 }
 // Steps per chunk for a circuit of M steps.
 __host__ __device__ constexpr int sv_kc(int w, int ll, int cplx_bytes, int M) {
