@@ -1,5 +1,6 @@
 // Wide-window statevector sweep (windows 8..30): the state streams through a
-// device workspace in passes of several fused steps.
+// device workspace in passes of several fused steps (windows 11..17 in XY, X and Y
+// stay on chip: sv_chip.cu).
 //
 // The window of every run is a 2^w complex64 vector in the workspace; windows
 // from 11 on keep half of it (HALF).  After step k the window is phi_k and its
@@ -36,30 +37,13 @@
 #include <vector>
 
 #include "dispatch.h"
-#include "sv_reg.cuh"
+#include "sv_stream.cuh"
 
 namespace mbqc {
 
 constexpr int kStreamMinWindow = 8;
 constexpr int kLowLanes = 5;    // index bits 0..4 are lane bits
 constexpr int kLowRegs = 3;     // extra register bits of a low pass
-
-struct StreamArgs {
-  const DevStep *steps;  // this circuit's steps
-  int W, M, n_in, n_out;
-  int S;                 // log2 of a run's amplitudes in the workspace: W - 1 (half) or W
-  int64_t B;
-  const double *angles;
-  int64_t astride;
-  const float2 *psi_in;
-  int64_t istride;
-  float2 *state;   // [B][2^S]
-  double *norms;   // [3][B]
-  int32_t *expo;   // [B] total applied exponent
-  int8_t in_bits[32];
-  int8_t out_bits[32];
-  uint32_t init_cz[32];
-};
 
 struct PassDesc {
   int k0, nsteps, index;  // first step, steps in the pass, pass number
@@ -91,43 +75,6 @@ __device__ __forceinline__ uint32_t scatter_bits(uint32_t v, const int *bits, in
   uint32_t r = 0;
   for (int i = 0; i < n; ++i) r |= ((v >> i) & 1u) << bits[i];
   return r;
-}
-
-// a pass step on register bit J (lower half amp = 1 unless GEN)
-template <bool GEN, int R, int J>
-__device__ __forceinline__ void pass_reg_step(float2 (&v)[R], float2 c, float amp, uint32_t ts, bool dead) {
-  if constexpr (GEN)
-    reg_step_g<float, R, J>(v, c, amp, ts, dead);
-  else
-    reg_step<float, R, J>(v, c, ts, dead);
-}
-// The same on a pair of phi_{k-1} that becomes a pair of phi_k (HALF): both halves
-// of the entered qubit, the second with the sign of its CZs and c1 = -c where one
-// of them is with the measured qubit.
-template <bool GEN, int R, int J>
-__device__ __forceinline__ void pass_half_step(float2 (&v)[R], float2 c, float amp, uint32_t flip, uint32_t ts,
-                                               bool dead) {
-  const float2 c1 = flip_sign(c, flip);
-#pragma unroll
-  for (int j = 0; j < R; ++j) {
-    if (j & (1 << J)) continue;
-    const int jh = j | (1 << J);
-    const float2 x0 = v[j], x1 = v[jh];
-    float2 o;
-    if constexpr (GEN) {
-      v[j] = make_float2(amp * x0.x + c.x * x1.x - c.y * x1.y, amp * x0.y + c.x * x1.y + c.y * x1.x);
-      o = make_float2(amp * x0.x + c1.x * x1.x - c1.y * x1.y, amp * x0.y + c1.x * x1.y + c1.y * x1.x);
-    } else {
-      v[j] = make_float2(x0.x + c.x * x1.x - c.y * x1.y, x0.y + c.x * x1.y + c.y * x1.x);
-      o = make_float2(x0.x + c1.x * x1.x - c1.y * x1.y, x0.y + c1.x * x1.y + c1.y * x1.x);
-    }
-    v[jh] = sign_bit_flip(o, ts * (1u << (31 - jh)));
-  }
-  if (dead) {
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-      if (j & (1 << J)) v[j] = make_float2(0.f, 0.f);
-  }
 }
 
 // First window: amplitude idx = psi_in[x(idx)] * (-1)^Q(idx), x gathering
@@ -924,15 +871,6 @@ __global__ void __launch_bounds__(kOutThreads) stream_out_write(StreamArgs a, Ou
   }
 }
 
-// HALF: the workspace bit of the qubit at a window bit after `done` steps.  The
-// window holds the qubits done .. done + w - 1 of the schedule at bit (index mod w);
-// all but the last are stored, qubit s at bit (s - 1) mod (w - 1): the bit of the
-// measured qubit is the entering one's.
-static int half_bit(int pos, int done, int w) {
-  const int s = done + ((pos - done) % w + w) % w;
-  return (s - 1) % (w - 1);
-}
-
 static OutDesc make_out_desc(const DevCircuit &hc, bool half) {
   OutDesc od{};
   const int n_out = hc.n_out, K = n_out < kOutLo ? n_out : kOutLo;
@@ -1180,6 +1118,13 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
     a.init_cz[i] = hc.init_cz[i];
   }
   cudaStream_t s = (cudaStream_t)stream;
+  // one launch on chip where the half window fits a cluster of four blocks (sv_chip.cu);
+  // XZ / YZ planes and the bulk-copy staging option keep the passes
+  if (half && !gen && !(flags & MBQC_F_STREAM_TMA)) {
+    size_t smem = 0;
+    if (const int cs = chip_plan(hc, batch, &smem))
+      return launch_sv_chip(a, hc, cs, smem, flags, reinterpret_cast<float2 *>(psi_out), logprob, status, s);
+  }
   const InitDesc id = make_init_desc(hc);
   const int64_t chunks = batch << (hc.w - id.K);
   const int64_t blocks = std::min<int64_t>(std::max<int64_t>(chunks, (batch + 255) / 256), (int64_t)sm_count() * 8);

@@ -1,7 +1,9 @@
-"""Streamed sweep, windows 11 and up, where the workspace keeps half the window:
-steps on the stored half's bits at every offset (short and long wires, uneven
-ones with steps that no qubit enters, more steps than the window), outputs on
-rotated bits, XZ / YZ planes, both staging paths; against the complex128 oracle
+"""Wide sweep, windows 11 and up, where half the window is kept: on chip (the
+default up to window 17) and in streamed passes (the bulk-copy staging, XZ / YZ
+planes, wider windows).  Steps on the stored half's bits at every offset (short
+and long wires, uneven ones with steps that no qubit enters, more steps than the
+window), outputs on rotated bits; on chip every number of blocks a run (1, 2, 4
+and 8, by window and batch) and every slice size; against the complex128 oracle
 at the amplitude bound of the other streamed tests."""
 import numpy as np
 import pytest
@@ -30,7 +32,14 @@ CASES = [  # circuit, runs, general planes
     (lambda r: C.many_wires([5, 2, 3] * 4), 5, False),          # uneven wires
     (lambda r: C.many_wires([7, 6, 5, 4, 3, 2] * 2), 3, False),
     (lambda r: C.grid_cluster(13, 5), 2, False),
-    (lambda r: C.many_wires([2, 3] * 8), 2, False),             # w = 17
+    (lambda r: C.many_wires([2, 3] * 8), 2, False),             # w = 17, eight blocks a run on chip
+    (lambda r: C.grid_cluster(16, 3), 20, False),               # w = 17, four
+    (lambda r: C.grid_cluster(15, 3), 3, False),                # w = 16, four
+    (lambda r: C.many_wires([3] * 15), 40, False),              # w = 16, two
+    (lambda r: C.grid_cluster(14, 4), 5, False),                # w = 15, two
+    (lambda r: C.many_wires([3] * 14), 80, False),              # w = 15, one
+    (lambda r: C.grid_cluster(11, 12), 2, False),               # w = 12, many cycles
+    (lambda r: C.many_wires([3] * 17), 1, False),               # w = 18: streamed
     (lambda r: _planes(C.grid_cluster(10, 4), r), 3, True),
     (lambda r: _planes(C.many_wires([4] * 12), r), 2, True),
 ]
@@ -46,9 +55,10 @@ def test_half_window_against_oracle(case, tma):
     assert sw.plan.window >= 11
     ang = rng.uniform(0, 2 * np.pi, size=(B, sw.n_angles))
     psi = haar_states(rng, sw.n_in, B)
-    out, st, _ = sw.forward(ang, psi, stream_tma=tma)
+    out, st, lp = sw.forward(ang, psi, stream_tma=tma, logprob=True)
     assert (st.cpu().numpy() == 0).all()
     out = out.cpu().numpy()
     r = B - 1
-    ref, _, _ = oracle.run_sv(circ, ang[r], psi[r], output_form="sv")
+    ref, _, probs = oracle.run_sv(circ, ang[r], psi[r], output_form="sv")
     assert np.abs(out[r] - ref).max() < TOL_AMP_C64
+    assert abs(float(lp[r]) - np.log(probs).sum()) < 1e-4
