@@ -837,7 +837,7 @@ def bench_adjoint(dev, fp32_peak, flush, reps=5):
 
 
 def bench_wide(dev, hbm_peak, flush, reps=7):
-    """Streamed wide window: grid_cluster(16, 10), w=17, 64 runs, |+>^16 input."""
+    """Wide window: grid_cluster(16, 10), w=17, 64 runs, |+>^16 input."""
     import torch
 
     from mentpy_gb300 import circuit as C
@@ -862,35 +862,15 @@ def bench_wide(dev, hbm_peak, flush, reps=7):
     out_np, ang_np = out.cpu().numpy(), ang.cpu().numpy()
     pick = np.random.default_rng(SEED + 30).choice(B, 8, replace=False)
     tasks = [("sv", ("grid", 16, 10), ang_np[r:r + 1], None, out_np[r:r + 1], None) for r in pick]
-    n_pass = 0
-    k = 0
-    while k < M:  # the kernel's mixed-pass grouping (windows >= 10): high* low* high*, <= 5 + 5 bits
-        phase, nh, nl = 0, 0, 0
-        while k < M:
-            if (k % w) < 5:
-                if phase == 2 or nl == 5:
-                    break
-                phase, nl = 1, nl + 1
-            else:
-                if nh == 5:
-                    break
-                phase, nh = (2 if phase == 1 else phase), nh + 1
-            k += 1
-        n_pass += 1
-    moved = B * 2**w * 8 * (2 * n_pass + 2)
-    dram = profile_traffic("stream_grid16x10_batch")
-    roof = {"bound": "hbm", "peak": hbm_peak, "unit": "GB/s", "traffic": dram,
-            "achieved": None if dram is None else dram / (ms * 1e-3) / 1e9,
-            "frac": None if dram is None else dram / (ms * 1e-3) / 1e9 / hbm_peak,
-            "note": "achieved = DRAM bytes of one batch (ncu dram__bytes_read.sum + dram__bytes_write.sum over "
-                    "every launch of the batch, profiles/stream_pass_grid16x10.md) / batch time; the 64 MiB "
-                    "state is partly L2-resident between passes",
-            "l2_pass_bytes_per_batch": moved, "l2_pass_gbs": moved / (ms * 1e-3) / 1e9,
-            "l2_pass_note": "one read + one write of every window per pass (what the SMs move; mostly served "
-                            "by L2), not an HBM figure",
+    moved = B * (2**sw.n_in + 2**sw.n_out) * 8 + B * sw.n_angles * 8
+    roof = {"bound": "hbm", "peak": hbm_peak, "unit": "GB/s", "traffic": None,
+            "achieved": moved / (ms * 1e-3) / 1e9, "frac": moved / (ms * 1e-3) / 1e9 / hbm_peak,
+            "note": "achieved = input, angle and output bytes of one batch / batch time; the kept half of each "
+                    "run's window (2^(w-1) complex64) stays in the shared memory of a cluster of blocks for the "
+                    "whole sweep, so barriers and latency bound it, not HBM",
             "per_step_model_gbs": alg / (ms * 1e-3) / 1e9,
             "per_step_model_note": "16*2^w bytes per measurement step, the reference algorithm's traffic; the "
-                                   "kernel fuses up to 10 steps per pass, so this is not a roofline fraction"}
+                                   "kernel keeps the window on chip, so this is not a roofline fraction"}
     # adjoint of the same batch (a block per run, per-step history in the workspace)
     gout_np = (rng.standard_normal((B, 2**sw.n_out)) + 1j * rng.standard_normal((B, 2**sw.n_out))) / 2**sw.n_out
     gout = torch.tensor(gout_np.astype(np.complex64), device=dev)
@@ -899,7 +879,7 @@ def bench_wide(dev, hbm_peak, flush, reps=7):
     torch.cuda.synchronize()
     assert int((ast != 0).sum()) == 0
     adj_ms = _time_cuda(lambda: sw.adjoint(ang, None, gout, status=ast), reps, flush)
-    hist = B * M * 2 * 2 ** (w - 1) * 8  # every step's half-state written once and read once
+    hist = B * M * 2 * 2 ** (w - 2) * 8  # a quarter of the window per step written once and read once
     grad_np = grad.cpu().numpy()
     drng = np.random.default_rng(SEED + 31)
     for r in pick[:4]:
@@ -909,28 +889,24 @@ def bench_wide(dev, hbm_peak, flush, reps=7):
                       1e-4, float(grad_np[r] @ d), float(np.abs(grad_np[r]).max())))
     fd_ms = ms * (2 * sw.n_angles + 1)  # batched device FD: (2A + 1) forward runs per gradient, same batch
     adjoint = {
-        "workload": "generic adjoint (dL = Re <g|dz>) of the same 64 runs: a cluster of two 1024-thread "
-                    "blocks per run (128 of the SMs), window and per-step half-states in the workspace",
+        "workload": "generic adjoint (dL = Re <g|dz>) of the same 64 runs: a cluster of two 512-thread "
+                    "blocks per run (128 of the SMs), half the window on chip as far as it fits, the per-step "
+                    "history in the workspace",
         "grads_per_s": B / (adj_ms * 1e-3),
         "ms_per_launch": adj_ms,
         "speedup_vs_batched_device_fd": fd_ms / adj_ms,
-        "batched_device_fd_note": "(2A+1) = 289 forward runs of the streamed kernel per gradient at the batch "
+        "batched_device_fd_note": "(2A+1) = 289 forward runs of the on-chip sweep per gradient at the batch "
                                   "time above",
         "roofline": {"bound": "hbm", "peak": hbm_peak, "unit": "GB/s",
                      "achieved": hist / (adj_ms * 1e-3) / 1e9, "frac": hist / (adj_ms * 1e-3) / 1e9 / hbm_peak,
-                     "traffic": (None if profile_traffic("sv_adj_wide_grid16x10_per_run") is None
-                                 else profile_traffic("sv_adj_wide_grid16x10_per_run") * B),
-                     "traffic_note": "ncu DRAM read + write per run (profiles/sv_adj_wide_grid16x10.md, a "
-                                     "16-run capture) x the launch's runs",
-                     "note": "algorithmic bytes = the history (2^(w-1) complex64 per step and run, written "
-                             "forward, read backward) over the launch time; the 1 MB window per block stays "
-                             "in L2"},
+                     "traffic": None,
+                     "note": "algorithmic bytes = the history (2^(w-2) complex64 per step and run, written "
+                             "forward, read backward) over the launch time"},
     }
     return {
-        "workload": "streamed statevector: grid_cluster(16,10), w=17 (2^17 complex64 per run), 144 angles, 64 runs",
+        "workload": "wide statevector sweep: grid_cluster(16,10), w=17 (2^17 complex64 per run, half of them kept), 144 angles, 64 runs",
         "runs_per_s": B / (ms * 1e-3),
         "ms_per_batch": ms,
-        "passes": n_pass,
         "roofline": roof,
         "adjoint": adjoint,
     }, tasks

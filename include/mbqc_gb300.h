@@ -307,10 +307,12 @@ int mbqc_sv_forward(const mbqc_plan *plan, int64_t batch, const double *angles,
 
 /*
  * Wide windows (8..30; the register kernel covers <= 10): the same sweep with
- * each run's 2^w window streamed through ``workspace`` in passes of up to ten
- * fused steps (five for windows 8 and 9).  Same arguments and results as
- * mbqc_sv_forward plus the workspace, sized by mbqc_sv_stream_workspace
- * (batch * 2^w * 8 bytes plus per-run bookkeeping and epilogue partials).  The reference cannot run these windows: its dense
+ * each run's window (from 11 on the half of it that determines the other) on
+ * chip (windows 11..17 in XY, X and Y: one launch) or streamed through
+ * ``workspace`` in passes of up to ten fused steps (five for windows 8 and 9).
+ * Same arguments and results as mbqc_sv_forward plus the workspace, sized by
+ * mbqc_sv_stream_workspace (batch * 2^(w-1) * 8 bytes, 2^w below window 11,
+ * plus per-run bookkeeping and epilogue partials).  The reference cannot run these windows: its dense
  * 2^w x 2^w operators (gates.py:62-72,127-143) need 256 GiB at w = 17.
  */
 int mbqc_sv_stream_workspace(const mbqc_plan *plan, int64_t batch, size_t *bytes);
@@ -415,8 +417,9 @@ int mbqc_dm_forward_ex(const mbqc_plan *plan, int64_t batch, int32_t window,
 
 /*
  * mbqc_dm_forward_ex for every window 1..11: windows 9..11 keep the factored
- * matrix (4^(w-1) complex64: 512 KB to 8 MB per run) in ``workspace``, one
- * 1024-thread block per resident run (mbqc_dm_forward_workspace gives the
+ * matrix (4^(w-1) complex64: 512 KB to 8 MB per run) in the shared memory of a
+ * thread-block cluster (9 and 10) or in ``workspace``, a cluster of blocks per
+ * resident run (mbqc_dm_forward_workspace gives the
  * bytes for ``batch`` runs; a smaller workspace runs fewer runs at a time,
  * the minimum is one run's matrix).  Windows <= 8 ignore the workspace.  The
  * reference runs these windows with dense 4^w x 4^w operators

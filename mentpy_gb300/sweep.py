@@ -301,7 +301,7 @@ class StatevectorSweep:
     # ------------------------------------------------------------ autotuning
     def variants(self):
         """Register-kernel variants (log2 lanes per run) valid for this window;
-        windows above 10 have the streamed kernel only."""
+        windows above 10 have the wide kernels only."""
         w = self.plan.window
         if w > REGISTER_MAX_WINDOW or self.dtype != torch.complex64:
             return []
@@ -453,8 +453,8 @@ class PreparedSweep:
     A register-kernel batch is one launch: its C entry point and arguments
     are resolved once and each call makes only that call (a few microseconds
     of host work; consecutive launches on a stream overlap their prologues).
-    A streamed batch (tens of launches) is recorded into a CUDA graph and
-    replayed.  Buffers that the sweep would first convert (another dtype or
+    A wide batch (one launch on chip, tens when streamed) is recorded into a
+    CUDA graph and replayed.  Buffers that the sweep would first convert (another dtype or
     device, lazy conjugate views) are also handled by the graph, which then
     records the conversion too."""
 
