@@ -35,7 +35,7 @@ def units():
     """(source, object, extra flags) for every translation unit."""
     out = []
     for name in ("plan.cu", "sv_api.cu", "adj_api.cu", "adj_noalloc.cu", "dm.cu", "dm_batch.cu", "dm_adj.cu",
-                 "sv_stream.cu", "sv_chip.cu", "graph_compile.cu", "train.cu", "sv_sampled.cu",
+                 "sv_stream.cu", "sv_chip.cu", "sv_half.cu", "graph_compile.cu", "train.cu", "sv_sampled.cu",
                  "sv_adj_wide.cu"):
         out.append((os.path.join(CSRC, name), os.path.join(BUILD, name[:-3] + ".o"), []))
     for w in SV_REG_WINDOWS:

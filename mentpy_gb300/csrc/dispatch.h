@@ -79,6 +79,11 @@ int wide_adj_threads(int w);
 size_t wide_adj_smem(int w, int M, bool gen);
 int wide_adj_resident(int w, int M, bool gen, int cluster, size_t limit);
 
+// Windows 9 and 10 on the kept half of the window (sv_half.cu).
+struct SvArgs;
+bool sv_half_ok(const DevCircuit &hc, const DevStep *steps, int64_t batch, uint32_t flags);
+int launch_sv_half(int w, int ll, const SvArgs &a, cudaStream_t s);
+
 int sm_count();
 
 // Programmatic dependent launch: a kernel launched this way may start while

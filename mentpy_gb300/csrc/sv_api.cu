@@ -75,13 +75,15 @@ struct mbqc_sv_call {
   int ll, blocks, threads;
   mbqc::sv_launcher fn;
   mbqc::sv_gen_launcher gfn;
-  bool empty;
+  bool empty, half;  // half: the kept-half kernel (sv_half.cu)
+  int w;
 };
 
 namespace mbqc {
 
 static int sv_exec(const mbqc_sv_call &c, cudaStream_t stream) {
   if (c.empty) return MBQC_OK;
+  if (c.half) return launch_sv_half(c.w, c.ll, c.a, stream);
   if (c.gfn) return c.gfn(c.a, c.blocks, c.threads, stream);
   return c.fn(c.ll, c.a, c.blocks, c.threads, stream);
 }
@@ -90,6 +92,7 @@ static int sv_build(const mbqc_plan *plan, int64_t batch, const double *angles, 
                     const void *psi_in, int64_t istride, void *psi_out, uint32_t flags, int variant,
                     double *logprob, int32_t *status, bool f64, mbqc_sv_call &c) {
   c.empty = true;
+  c.half = false;
   c.fn = nullptr;
   c.gfn = nullptr;
   if (!plan) return fail(MBQC_E_INVALID, "sv_forward: null plan");
@@ -160,6 +163,8 @@ static int sv_build(const mbqc_plan *plan, int64_t batch, const double *angles, 
     c.fn = pick(hc.w, f64);
     if (!c.fn) return fail(MBQC_E_UNSUPPORTED, "sv_forward: window %d", hc.w);
   }
+  c.w = hc.w;
+  c.half = !f64 && !gen && variant < 0 && sv_half_ok(hc, host_steps(plan, 0), batch, flags);
   c.empty = false;
   return MBQC_OK;
 }
