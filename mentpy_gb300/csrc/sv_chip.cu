@@ -193,8 +193,28 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
     if (lane == 0) s_ph[wid] = ph;
     __syncthreads();
 
-    // ---- phi_0 from the input: index parts as in stream_init
+    auto pair_sum = [&](float2 t) {  // over the block, in s_red[0]'s order for every thread
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1)
+        two_sum_acc(t.x, t.y, __shfl_xor_sync(0xffffffffu, t.x, o), __shfl_xor_sync(0xffffffffu, t.y, o));
+      __syncthreads();
+      if (lane == 0) s_pair[wid] = t;
+      __syncthreads();
+      t = s_pair[0];
+      for (int i = 1; i < NW; ++i) two_sum_acc(t.x, t.y, s_pair[i].x, s_pair[i].y);
+      return t;
+    };
     const float2 *in = a.psi_in + (a.istride ? run * a.istride : 0);
+    float2 nin = make_float2(1.f, 0.f);  // before any output: the outputs may lie on the inputs
+    if (logprob && crank == 0) {
+      nin.x = 0.f;
+      for (int x = tid; x < (1 << a.n_in); x += BT) {
+        const float2 v = in[x];
+        two_sum_acc(nin.x, nin.y, v.x * v.x + v.y * v.y, 0.f);
+      }
+      nin = pair_sum(nin);
+    }
+    // ---- phi_0 from the input: index parts as in stream_init
     {
       const uint32_t x0 = s_thr[tid], x1 = s_thr[BT + tid], a0 = s_thr[2 * BT + tid], a1 = s_thr[3 * BT + tid];
       const uint32_t et = s_thr[4 * BT + tid], q0 = (et >> 30) & 1u, q1 = et >> 31, e = et & (NS - 1);
@@ -337,17 +357,6 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
     }
 
     // ---- normalise (float-pair sums), phase, outputs in the reference's order
-    auto pair_sum = [&](float2 t) {  // over the block, in s_red[0]'s order for every thread
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1)
-        two_sum_acc(t.x, t.y, __shfl_xor_sync(0xffffffffu, t.x, o), __shfl_xor_sync(0xffffffffu, t.y, o));
-      __syncthreads();
-      if (lane == 0) s_pair[wid] = t;
-      __syncthreads();
-      t = s_pair[0];
-      for (int i = 1; i < NW; ++i) two_sum_acc(t.x, t.y, s_pair[i].x, s_pair[i].y);
-      return t;
-    };
     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 8
     for (int i = 0; i < 32; ++i) {
@@ -379,23 +388,11 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
       for (int i = 0; i < 32; ++i)
         if ((uint32_t)(tid + i * BT) < cnt) o[yt | s_it[128 + i]] = cmul(s[et ^ s_it[96 + i]], sc);
     }
-    if (crank == 0) {
-      double nin = 1.0;
-      if (logprob) {  // uniform
-        float2 ni = make_float2(0.f, 0.f);
-        for (int x = tid; x < (1 << a.n_in); x += BT) {
-          const float2 v = in[x];
-          two_sum_acc(ni.x, ni.y, v.x * v.x + v.y * v.y, 0.f);
-        }
-        const float2 tn = pair_sum(ni);
-        nin = (double)tn.x + (double)tn.y;
-      }
-      if (tid == 0) {
-        if (status) status[run] = ok ? MBQC_RUN_OK : (isnan(n2) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
-        if (logprob)
-          logprob[run] =
-              log((double)n2p.x + (double)n2p.y) - log(nin) + 0.6931471805599453 * (2.0 * expo + lp_const);
-      }
+    if (crank == 0 && tid == 0) {
+      if (status) status[run] = ok ? MBQC_RUN_OK : (isnan(n2) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
+      if (logprob)
+        logprob[run] = log((double)n2p.x + (double)n2p.y) - log((double)nin.x + (double)nin.y) +
+                       0.6931471805599453 * (2.0 * expo + lp_const);
     }
     run_barrier<CS>();  // the next run overwrites the tables; other blocks have read this one's norm
   }

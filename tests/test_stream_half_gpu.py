@@ -62,3 +62,17 @@ def test_half_window_against_oracle(case, tma):
     ref, _, probs = oracle.run_sv(circ, ang[r], psi[r], output_form="sv")
     assert np.abs(out[r] - ref).max() < TOL_AMP_C64
     assert abs(float(lp[r]) - np.log(probs).sum()) < 1e-4
+
+
+@pytest.mark.parametrize("build", [lambda: C.grid_cluster(10, 3), lambda: C.grid_cluster(15, 3)])
+def test_outputs_on_the_inputs(build):
+    """One buffer for inputs and outputs: the input (and its norm) is read first."""
+    sw = StatevectorSweep(build())
+    rng = np.random.default_rng(499)
+    B = 20
+    ang = rng.uniform(0, 2 * np.pi, size=(B, sw.n_angles))
+    psi = torch.as_tensor(3.0 * haar_states(rng, sw.n_in, B), dtype=torch.complex64, device="cuda")
+    want, _, wlp = sw.forward(ang, psi, logprob=True)
+    got, st, lp = sw.forward(ang, psi, logprob=True, out=psi)
+    assert (st == 0).all()
+    assert torch.equal(got, want) and torch.equal(lp, wlp)
