@@ -402,9 +402,12 @@ class StatevectorSweep:
         grad = make((B, self.n_angles), dtype=torch.float64, device=self.device)
         if B == 0:
             return grad
-        if stream is not None and not written:
-            stream.wait_stream(torch.cuda.current_stream(self.device))  # the zeros before the kernel
         ws = self._workspace(B)
+        if stream is not None:
+            # what the current stream still does to the operands (the default
+            # input's fill, conversions, the zeros, the caller's own work) and to
+            # earlier owners of grad's and the workspace's memory comes before the kernel
+            stream.wait_stream(torch.cuda.current_stream(self.device))
         fn = _native.lib().mbqc_sv_adjoint if self.dtype == torch.complex64 else _native.lib().mbqc_sv_adjoint_f64
         _native.check(fn(self.dplan.handle, B, _ptr(ang), max(ang.shape[1], 1), _ptr(inp), istride, _ptr(g),
                          _ptr(grad), _ptr(status), _ptr(ws), ws.numel(), _stream_ptr(stream)))
