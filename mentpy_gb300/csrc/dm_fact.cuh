@@ -526,14 +526,15 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
 // position bits, so positions 0..4 pair rows of one block; B by their lowest
 // bits, so positions 5.. do.  Steps meet the positions cyclically, so a run
 // stays in a layout for 5 steps, then for n - 5: the last step before a change
-// writes its rows straight to their new owners (distributed shared memory).
+// writes its rows straight to their new owners (distributed shared memory) once
+// every block's loads have been released to the others.
 // A step is then: one warp sums the block's diagonal pairs and sends the
 // partial to every block, one cluster barrier, the pass over the block's rows.
 // What bounds it is that chain (cycles a step at window 9: ~1,300 to the
 // barrier's end, 250 the sum, 970 the pass, 1,400 the layout changes' share);
 // the workspace kernel below pays two round trips to the L2 and the slice's
 // traffic through it at every step.  Window 9, 40 steps: 228 us for 1 to 8
-// runs and 325 us for 24 there, 117 and 183 us here; window 10, 36 steps, 4
+// runs and 325 us for 24 there, 117 and 186 us here; window 10, 36 steps, 4
 // runs: 424 and 189 us.
 template <int W> struct DmClCfg {
   static constexpr int N = W - 1, LB = 5, OB = N - LB, CS = 1 << OB;  // positions, local and owner row bits
@@ -802,7 +803,7 @@ __global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_
         float4 x[4], y[4];
         unit(l0, x);
         unit(l1, y);
-        cluster_arrive_relaxed();
+        cluster_arrive();  // release: this block's loads come before the others' stores
         cluster_wait();
         auto row_ptr = [&](uint32_t l) {
           const uint32_t i = row_of(lb, l), owner = lb ? i >> LB : i & (CS - 1), q = lb ? i & (RL - 1) : i >> OB;
