@@ -677,13 +677,18 @@ __global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_
         }
         return sum;
       };
-      // the sum over the cluster; only warp 0 has something to publish
+      // the sum over the cluster.  Warp 0 publishes the partial; the other warps'
+      // reads of the buffer that the next exchange but one writes are released by
+      // the block barrier that ends the step and warp 0's next arrival, but a
+      // step's further exchanges have no such barrier before them.
       auto exchange = [&](int what) {
         if (tid < 32) {
           send(partial(what));
           cluster_arrive();
-        } else {
+        } else if (what == 0) {
           cluster_arrive_relaxed();
+        } else {
+          cluster_arrive();
         }
         cluster_wait();
         return collect();

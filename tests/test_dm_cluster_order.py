@@ -4,8 +4,11 @@ the memory model: a store into another block's shared memory has to come after
 every earlier read of that place.  The kernel's accesses and barriers are replayed
 with vector clocks, the arrival's form (release or relaxed: a relaxed arrival
 orders nothing before it) read from the source (no GPU)."""
+import itertools
 import os
 import re
+
+import pytest
 
 SRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "mentpy_gb300", "csrc", "dm_fact.cuh")
 BLOCKS, WARPS = 2, 2  # warp 0 sends and arrives apart from the others
@@ -67,4 +70,26 @@ def test_layout_change_stores_after_every_load():
         for t, b, w in c.warps():
             c.write(t, ("rows", 1 - b, w))
         c.cluster_barrier(lambda w: True)
+    assert not c.races
+
+
+@pytest.mark.parametrize("kinds", list(itertools.product([(0,), (0, 1), (0, 2), (0, 1, 2)], repeat=3)))
+def test_partials_are_sent_after_every_read_of_their_buffer(kinds):
+    """kinds: the exchanges of each step (a Z step needs the trace, outcome 1 prob1)."""
+    text = _source("auto exchange", "return collect();")
+    assert len(re.findall(r"cluster_arrive", text)) == 3 and "if (tid < 32)" in text
+    relaxed = re.search(r"else if \(what == (\d)\) \{\s*cluster_arrive_relaxed\(\);", text)
+    c, par = Cluster(), 0
+    for what in kinds + kinds[:1]:
+        for x in what:
+            for t, b, w in c.warps():
+                if w == 0:
+                    for other in range(BLOCKS):
+                        c.write(t, (other, par, b))
+            c.cluster_barrier(lambda w: w == 0 or x != int(relaxed.group(1)))
+            for t, b, w in c.warps():
+                for r in range(BLOCKS):
+                    c.read(t, (b, par, r))
+            par ^= 1
+        c.block_barrier()  # the pass
     assert not c.races
