@@ -509,8 +509,10 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     ridx[y] = ri;
   }
   group_sync(TPR, group);
+  const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
   if (A.probs)
-    for (int k = tid; k < n_rec; k += TPR) A.probs[run * A.ostride + k] = prob_record(sF[k]);
+    for (int k = tid; k < n_rec; k += TPR)
+      A.probs[run * A.ostride + k] = prob_record(sF[k], ratio && (sSt[k].x & kFactZ) != 0u);
   float2 *out = A.rho_out + run * A.out_stride;
   for (int e = tid; e < dout * dout; e += TPR) {
     const int yi = e >> n_out, yj = e & (dout - 1);
@@ -884,8 +886,10 @@ __global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_
       rinv[ri] = y;
     }
     __syncthreads();
+    const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
     if (rank == 0 && A.probs)
-      for (int k = tid; k < n_rec; k += BT) A.probs[run * A.ostride + k] = prob_record(sF[k - 1]);
+      for (int k = tid; k < n_rec; k += BT)
+        A.probs[run * A.ostride + k] = prob_record(sF[k - 1], ratio && (sSt[k].x & kFactZ) != 0u);
     float2 *out = A.rho_out + run * A.out_stride;
     for (int e = tid; e < RL << n_out; e += BT) {
       const int l = e >> n_out, yj = e & (dout - 1), yi = rinv[row_of(lb, (uint32_t)l)];
@@ -1188,8 +1192,10 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       ridx[y] = ri;
     }
     __syncthreads();
+    const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
     if (crank == 0 && A.probs)
-      for (int k = tid; k < n_rec; k += BT) A.probs[run * A.ostride + k] = prob_record(sF[k]);
+      for (int k = tid; k < n_rec; k += BT)
+        A.probs[run * A.ostride + k] = prob_record(sF[k], ratio && (sSt[k].x & kFactZ) != 0u);
     float2 *out = A.rho_out + run * A.out_stride;
     for (int e = g; e < dout * dout; e += TT) {
       const int yi = e >> n_out, yj = e & (dout - 1);
