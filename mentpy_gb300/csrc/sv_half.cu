@@ -144,6 +144,13 @@ __global__ void __launch_bounds__(32 * kHalfWarps, 4) sv_half(SvArgs a) {
     }
     for (int x = li; x < din; x += LR) s[x] = in[x];
     __syncwarp();
+    // the input's norm, as sv_fwd_reg sums it, before any output is written (they
+    // may lie on the inputs); kept in the row's padding
+    if (a.logprob && li == 0) {
+      float nin = 0.f;
+      for (int x = 0; x < din; ++x) nin += fmaf(s[x].x, s[x].x, __fmul_rn(s[x].y, s[x].y));
+      s[NS].x = nin;
+    }
 
     float2 v[32];
     {  // phi_0, bits 0..4 in registers
@@ -282,10 +289,8 @@ __global__ void __launch_bounds__(32 * kHalfWarps, 4) sv_half(SvArgs a) {
       if (li == 0) {
         if (a.status) a.status[run] = ok ? MBQC_RUN_OK : (isnan(n2) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
         if (a.logprob) {  // as sv_fwd_reg
-          float nin = 0.f;
-          for (int x = 0; x < din; ++x) nin += fmaf(in[x].x, in[x].x, __fmul_rn(in[x].y, in[x].y));
           int e1, e2;
-          const float m1 = frexpf(n2, &e1), m2 = frexpf(nin, &e2);
+          const float m1 = frexpf(n2, &e1), m2 = frexpf(s[NS].x, &e2);
           const double ln2 = 0.6931471805599453;
           a.logprob[run] = (double)(logf(m1) - logf(m2)) + (double)n2lo / (double)n2 +
                            ln2 * (double)(e1 - e2 + 2 * expo + a.lp_const);
