@@ -742,9 +742,21 @@ __global__ void __maxnreg__((sv_maxnreg<T, W, LL, GEN, HOST>())) sv_fwd_reg(cons
   const CT sc = mk<T>(phase.x * inv, phase.y * inv);
   if (inputs_ready) griddep_wait();  // before the first write
 
+  if (valid && li == 0 && args.logprob) {  // before any output: the outputs may lie on the inputs
+    // ln(n2 / |in|^2) + ln2 * (2 e_applied + lp_const): exact exponents,
+    // float logs of the mantissas
+    const CT *in = reinterpret_cast<const CT *>(args.psi_in) + (args.istride ? run * args.istride : 0);
+    T nin = T(0);
+    for (int x = 0; x < (1 << args.n_in); ++x) nin += in[x].x * in[x].x + in[x].y * in[x].y;
+    int e1, e2;
+    const float m1 = frexpf((float)n2t, &e1), m2 = frexpf((float)nin, &e2);
+    const double ln2 = 0.6931471805599453;
+    args.logprob[run] = (double)(logf(m1) - logf(m2)) + (double)n2lo / (double)n2t +
+                        ln2 * (double)(e1 - e2 + 2 * e_applied + args.lp_const);
+  }
+  __syncwarp();
   if constexpr (kIO) {
     // outputs: scattered into the staging rows, then coalesced row stores
-    __syncwarp();
 #pragma unroll
     for (int j = 0; j < R; ++j)
       if (my[j] >= 0) s_io[sub * (1 << W) + my[j]] = cmul(a[j], sc);
@@ -763,22 +775,8 @@ __global__ void __maxnreg__((sv_maxnreg<T, W, LL, GEN, HOST>())) sv_fwd_reg(cons
       for (int j = 0; j < R; ++j)
         if (my[j] >= 0) out[my[j]] = cmul(a[j], sc);
     }
-    if (li == 0) {
-      if (args.status)
-        args.status[run] = ok ? MBQC_RUN_OK : (isnan(n2t) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
-      if (args.logprob) {
-        // ln(n2 / |in|^2) + ln2 * (2 e_applied + lp_const): exact exponents,
-        // float logs of the mantissas
-        const CT *in = reinterpret_cast<const CT *>(args.psi_in) + (args.istride ? run * args.istride : 0);
-        T nin = T(0);
-        for (int x = 0; x < (1 << args.n_in); ++x) nin += in[x].x * in[x].x + in[x].y * in[x].y;
-        int e1, e2;
-        const float m1 = frexpf((float)n2t, &e1), m2 = frexpf((float)nin, &e2);
-        const double ln2 = 0.6931471805599453;
-        args.logprob[run] = (double)(logf(m1) - logf(m2)) + (double)n2lo / (double)n2t +
-                            ln2 * (double)(e1 - e2 + 2 * e_applied + args.lp_const);
-      }
-    }
+    if (li == 0 && args.status)
+      args.status[run] = ok ? MBQC_RUN_OK : (isnan(n2t) ? MBQC_RUN_NAN : MBQC_RUN_ZERO_NORM);
   }
 }
 

@@ -25,3 +25,17 @@ def _check(circ, B, **kw):
 @pytest.mark.parametrize("rows,B", [(8, 2435), (9, 1219)])
 def test_half_window_kernel(rows, B):
     _check(C.grid_cluster(rows, 4), B)
+
+
+@pytest.mark.parametrize("kw", [{}, dict(dtype=torch.complex128), dict(extended_planes=True)])
+@pytest.mark.parametrize("rows,B", [(1, 3), (2, 5000), (4, 700), (7, 300), (8, 20), (9, 20)])
+def test_register_kernel(rows, B, kw):
+    circ = C.grid_cluster(rows, 4)
+    if "extended_planes" in kw:
+        circ[1] = C.Ment("XZ")
+    _check(circ, B, **kw)
+
+
+@pytest.mark.parametrize("rows,B", [(10, 20), (17, 2)])  # on chip; streamed
+def test_wide_kernels(rows, B):
+    _check(C.many_wires([3] * rows), B)
