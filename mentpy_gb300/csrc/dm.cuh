@@ -145,8 +145,11 @@ __device__ __forceinline__ float2 group_sum2(float v, float2 *scratch, int tid, 
 // 1e-6 (relative) of t, where hi - tf is exact and the remainders decide.  All
 // in float: as an FP64 comparison on that branch the compiler ran it on every
 // thread at every step (two conversions, an add and a compare on a pipe of
-// 1/64 the FP32 rate: ~1,400 cycles a step with 16 warps on an SM).
-__device__ __forceinline__ bool pair_ge(float2 p, double t) {
+// 1/64 the FP32 rate: ~1,400 cycles a step with 16 warps on an SM).  At t = 1e-4
+// every renormalised pair (|lo| <= half an ulp of hi) decides as its FP64 sum: hi
+// = tf leaves lo >= tl, and tf + tl is t rounded up on lo's grid (2^-62); any other hi is half
+// an ulp or more away from t, out of lo's reach.
+__host__ __device__ __forceinline__ bool pair_ge(float2 p, double t) {
   const float tf = (float)t, tl = (float)(t - (double)tf);
   const float d = p.x - tf;
   if (fabsf(d) > 1e-6f * tf) return d > 0.f;
