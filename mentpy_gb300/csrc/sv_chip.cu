@@ -136,9 +136,16 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
         y_rank |= 1u << d.rank_y[r];
     }
 
+  // Norms that choose a scale are float sums over a warp (as the streamed passes'),
+  // a block and a cluster.  Only their exponent is used and the scale is exact, so
+  // their rounding reaches no result; their range has to be that of the warps'
+  // parts: a total that a float cannot hold is kept as minus its 2^-8 times.
+  constexpr float kDown = 0.00390625f;
   auto renorm_of = [](float t) {  // half the exponent of a norm
+    const int up = t < 0.f ? 8 : 0;
+    t = up ? -t : t;
     if (!RealBits<float>::finite_pos(t)) return 0;
-    const int f = RealBits<float>::expo(t) >> 1;
+    const int f = (RealBits<float>::expo(t) + up) >> 1;
     return f > 100 ? 100 : (f < -100 ? -100 : f);
   };
   // norm of the amplitudes a thread holds, and the block's in s_part[x]
@@ -154,15 +161,28 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
   auto block_total = [&](int x) {
     float t = 0.f;
     for (int i = 0; i < NW; ++i) t += s_part[x][i];
+    if (t > 3.0e38f) {
+      t = 0.f;
+      for (int i = 0; i < NW; ++i) t -= kDown * s_part[x][i];
+    }
     return t;
   };
   auto run_total = [&](int x) {  // the same in every block
     if constexpr (CS == 1) {
       return block_total(x);
     } else {
-      float t = 0.f;
+      float q[CS], t = 0.f, low = 0.f;
 #pragma unroll
-      for (int r = 0; r < CS; ++r) t += *cg::this_cluster().map_shared_rank(&s_tot[x], r);
+      for (int r = 0; r < CS; ++r) {
+        q[r] = *cg::this_cluster().map_shared_rank(&s_tot[x], r);
+        t += q[r];
+        low = fminf(low, q[r]);
+      }
+      if (low < 0.f || t > 3.0e38f) {
+        t = 0.f;
+#pragma unroll
+        for (int r = 0; r < CS; ++r) t += q[r] < 0.f ? q[r] : -kDown * q[r];
+      }
       return t;
     }
   };
