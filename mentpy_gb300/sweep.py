@@ -310,7 +310,9 @@ class StatevectorSweep:
     def tune(self, angles, inputs=None, reps: int = 5, stream=None, inputs_ready: bool = False) -> int:
         """Time every variant on this batch (CUDA events, back-to-back
         launches after a warm-up) and keep the fastest for batches of this
-        size (power-of-two bucket).  ``inputs_ready`` times the launches in
+        size (power-of-two bucket).  At windows 9 and 10 the default (-1) is a
+        candidate of its own: large batches take a kernel there that no lane
+        count names (csrc/sv_half.cu).  ``inputs_ready`` times the launches in
         that mode (they overlap, which can favour another variant); the
         choice serves both modes, so the declaration never changes results.
         Returns the chosen variant; ``forward(variant=-1)`` uses it."""
@@ -321,6 +323,9 @@ class StatevectorSweep:
         if ang.dim() == 1:
             ang = ang.unsqueeze(0)
         B = ang.shape[0]
+        if self.plan.window >= 9:
+            cand.append(-1)
+            _TUNED.pop(self._tune_key(B), None)  # -1 is the default rule, not an earlier choice
         out = torch.empty((B, 2 ** self.n_out), dtype=self.dtype, device=self.device)
         st = torch.empty((B,), dtype=torch.int32, device=self.device)
         best, best_ms = -1, float("inf")
