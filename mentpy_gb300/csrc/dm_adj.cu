@@ -36,7 +36,7 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
   if (occ < 1) return fail(MBQC_E_UNSUPPORTED, "dm_adjoint: kernel does not fit on an SM");
   int groups = ACfg::GROUPS;
   size_t per_slot = ((size_t)maxm + (ACfg::kWs ? 1 : 0)) * Cfg::N * sizeof(float2);
-  if constexpr (W >= 3 && W <= 7) {
+  if constexpr (W >= kDmAdjFactMinWindow && W <= kDmAdjFactMaxWindow) {
     if (g.fact) {
       auto kf = dm_adj_fact<W>;
       groups = AdjFactCfg<W>::GROUPS;
@@ -67,7 +67,7 @@ static int dm_adj_geom(int64_t batch, int maxm, size_t ws_cap, DmAdjGeometry &g)
 
 template <int W>
 static int dm_adj_launch(DmAdjArgs a, const DmAdjGeometry &g, cudaStream_t s) {
-  if constexpr (W >= 3 && W <= 7) {
+  if constexpr (W >= kDmAdjFactMinWindow && W <= kDmAdjFactMaxWindow) {
     if (g.fact) {
       dm_adj_fact<W><<<g.blocks, AdjFactCfg<W>::GROUPS * AdjFactCfg<W>::TPR, g.smem, s>>>(a);
       return check_launch("dm_adj_fact");

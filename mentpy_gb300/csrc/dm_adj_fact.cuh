@@ -1,6 +1,13 @@
 // Adjoint of the (noisy) density-matrix sweep on the factored matrix, windows
-// 3..7 whose last step shrinks the window (dm_adj.cuh takes the others; the
+// 5..7 whose last step shrinks the window (dm_adj.cuh takes the others; the
 // derivation of the adjoint chain is there).
+//
+// Why from window 5 on: below it a run has fewer tiles than the warp has threads (1
+// at window 3, 4 at window 4) and the whole matrix is small anyway.  Grids of 12
+// columns, noise 0.01, full matrix against this: window 3, 500 runs 33 and 54 us,
+// 16,000 runs 197 and 603; window 4, 500 runs 68 and 86, 16,000 runs 516 and 1,007;
+// window 5, 500 runs 299 and 120, 16,000 runs 2,850 and 1,526; window 6, 500 runs
+// 546 and 239; window 7, 500 runs 3,736 and 788.
 //
 // After step k every entry of the full 2^w x 2^w matrix is +-sigma_k[r, c], 0 or
 // a sign of it: sigma_k is the (w-1)-qubit matrix over the bits other than the
@@ -34,14 +41,16 @@
 
 namespace mbqc {
 
+constexpr int kDmAdjFactMinWindow = 5, kDmAdjFactMaxWindow = 7;
+
 template <int W> struct AdjFactCfg {
-  static_assert(W >= 3 && W <= 7, "factored adjoint: windows 3..7");
+  static_assert(W >= kDmAdjFactMinWindow && W <= kDmAdjFactMaxWindow, "factored adjoint: windows 5..7");
   static constexpr int N = W - 1, D = 1 << N, T = D / 4;
   static constexpr int TPR = DmCfg<W>::TPR;
   static constexpr int GROUPS = TPR == 32 ? 2 : 1;  // runs per block: small blocks spread a batch over the SMs
-  static constexpr int NB = D * D, NI = NB >= TPR ? NB / TPR : 1;  // derivative terms, terms a thread
-  static constexpr int RS = TPR / D > 0 ? TPR / D : 1;             // row step between a thread's terms
-  static constexpr int HIST = 8 * T * T;                            // float4 a step
+  static constexpr int NB = D * D, NI = NB / TPR;  // derivative terms, terms a thread
+  static constexpr int RS = TPR / D;               // row step between a thread's terms
+  static constexpr int HIST = 8 * T * T;           // float4 a step
 };
 
 // shared memory of one run
@@ -549,15 +558,13 @@ __global__ void __launch_bounds__(AdjFactCfg<W>::TPR *AdjFactCfg<W>::GROUPS, 512
       if (tid == 0 && k + 1 < M && (sSt[k + 1].x & kAdjOff)) finish(k + 1);
       if (ss.x & kAdjOff) {
         float g = 0.f;
-        if (NB >= TPR || tid < NB) {
-          const uint32_t c = (uint32_t)tid % D, r0 = (uint32_t)tid / D;
-          const uint32_t at = r0 * D + (N == 6 ? c ^ ((c >> 5) * 10u) ^ ((__popc(r0) & 1u) * 21u) : c);
+        const uint32_t c = (uint32_t)tid % D, r0 = (uint32_t)tid / D;
+        const uint32_t at = r0 * D + (N == 6 ? c ^ ((c >> 5) * 10u) ^ ((__popc(r0) & 1u) * 21u) : c);
 #pragma unroll
-          for (int i = 0; i < NI; ++i) {
-            constexpr uint32_t step = (uint32_t)RS * D;
-            const uint32_t odd = ((i ^ (i >> 1) ^ (i >> 2) ^ (i >> 3)) & 1) && N == 6 ? 21u : 0u;
-            g += tb[(at ^ odd) + i * step];
-          }
+        for (int i = 0; i < NI; ++i) {
+          constexpr uint32_t step = (uint32_t)RS * D;
+          const uint32_t odd = ((i ^ (i >> 1) ^ (i >> 2) ^ (i >> 3)) & 1) && N == 6 ? 21u : 0u;
+          g += tb[(at ^ odd) + i * step];
         }
         float hi = g, lo = 0.f;
 #pragma unroll
