@@ -57,6 +57,14 @@ def mapped_ptr(t: torch.Tensor) -> ctypes.c_void_p:
     return out
 
 
+def _keep_for(stream, *tensors) -> None:
+    """Memory of the current stream that a kernel on ``stream`` uses: not handed
+    out again before that kernel is done."""
+    for t in tensors:
+        if t.is_cuda:
+            t.record_stream(stream)
+
+
 def _mapped_or_device(x, dtype, device, what: str) -> torch.Tensor:
     """``x`` itself when it is a pinned CPU tensor of ``dtype`` (accessed in
     place), else the usual device copy."""
@@ -413,6 +421,7 @@ class StatevectorSweep:
             # input's fill, conversions, the zeros, the caller's own work) and to
             # earlier owners of grad's and the workspace's memory comes before the kernel
             stream.wait_stream(torch.cuda.current_stream(self.device))
+            _keep_for(stream, ang, inp, g, grad, ws)
         fn = _native.lib().mbqc_sv_adjoint if self.dtype == torch.complex64 else _native.lib().mbqc_sv_adjoint_f64
         _native.check(fn(self.dplan.handle, B, _ptr(ang), max(ang.shape[1], 1), _ptr(inp), istride, _ptr(g),
                          _ptr(grad), _ptr(status), _ptr(ws), ws.numel(), _stream_ptr(stream)))

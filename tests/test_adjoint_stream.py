@@ -32,13 +32,15 @@ def test_the_stream_waits_for_the_current_one_before_the_launch(monkeypatch, row
         n._obj.value = 64
         return 0
 
+    kept, args = [], []
     monkeypatch.setattr(_native, "lib", lambda: SimpleNamespace(
-        mbqc_sv_adjoint_workspace=workspace, mbqc_sv_adjoint=lambda *a: log.append("launch") or 0))
+        mbqc_sv_adjoint_workspace=workspace, mbqc_sv_adjoint=lambda *a: log.append("launch") or args.extend(a) or 0))
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "current")
     for name in ("as_device", "torch.empty", "torch.zeros"):  # work and memory of the current stream
         owner, attr = (torch, name[6:]) if name.startswith("torch.") else (sweep, name)
         real = getattr(owner, attr)
         monkeypatch.setattr(owner, attr, lambda *a, _real=real, **k: log.append("made") or _real(*a, **k))
+    monkeypatch.setattr(sweep, "_keep_for", lambda s, *ts: kept.extend(t.data_ptr() for t in ts))
     sw = _bare_sweep(C.many_wires([4] * rows))
     B, d = 3, 2 ** sw.n_in
     psi = None if inputs is None else torch.ones(B, d, dtype=torch.complex128)
@@ -46,6 +48,8 @@ def test_the_stream_waits_for_the_current_one_before_the_launch(monkeypatch, row
     side = SimpleNamespace(cuda_stream=7, wait_stream=lambda s: log.append("wait " + s))
     sw.adjoint(torch.zeros(B, sw.n_angles, dtype=torch.float32), psi, g, stream=side)
     assert log[-2:] == ["wait current", "launch"] and log.count("wait current") == 1
+    ptrs = [args[i].value for i in (2, 4, 6, 7, 9)]  # angles, inputs, grad_out, gradient, workspace
+    assert sorted(kept) == sorted(ptrs)  # the allocator keeps them for the launch's stream
 
 
 @pytest.mark.gpu
