@@ -400,7 +400,12 @@ class CudaSimulatorSV(BaseSimulator):
         form = output_form.lower()
         if form not in ("dm", "densitymatrix", "sv", "statevector"):
             raise ValueError(f"Output form {output_form} is not supported.")
-        psi, status = self._run_one(np.asarray(angles, dtype=np.float64))
+        ang = np.asarray(angles, dtype=np.float64)
+        if ang.size != self._sweep.n_angles:  # one value a node (an [A, 0] or [A, 2] array has none or two)
+            raise ValueError(
+                f"Number of angles ({ang.size}) does not match number of trainable nodes ({self._sweep.n_angles})."
+            )
+        psi, status = self._run_one(ang)
         self.current_measurement = len(self.schedule_measure)
         self.outcomes = {node: 0 for node in self.plan.outcome_nodes()}
         if status != _native.RUN_OK:
