@@ -422,11 +422,11 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     if (take1) {  // outcome 1 with P1 = I - P0
       G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
       const float2 prob1 = diagonal(2);
-      if (tid == 0) sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      if (tid == 0) sF[k] = make_float4(prob.x, prob.y, kNoTrace, 0.f);
       prob = prob1;
       outcome = 1;
     } else if (tid == 0 && !unprojected) {
-      sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      sF[k] = make_float4(prob.x, prob.y, kNoTrace, 0.f);
     }
     n_rec = k + 1;
     if (tid == 0 && A.outcomes) A.outcomes[run * A.ostride + k] = (int8_t)outcome;
@@ -509,10 +509,9 @@ __device__ __forceinline__ void dm_fact_run(const DmArgs &A, int64_t slot, int t
     ridx[y] = ri;
   }
   group_sync(TPR, group);
-  const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
   if (A.probs)
     for (int k = tid; k < n_rec; k += TPR)
-      A.probs[run * A.ostride + k] = prob_record(sF[k], ratio && (sSt[k].x & kFactZ) != 0u);
+      A.probs[run * A.ostride + k] = prob_record(sF[k]);
   float2 *out = A.rho_out + run * A.out_stride;
   for (int e = tid; e < dout * dout; e += TPR) {
     const int yi = e >> n_out, yj = e & (dout - 1);
@@ -719,7 +718,7 @@ __global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_
       } else {
         take1 = !pair_ge(prob, 1e-4);  // prob0 < 1e-4 (or NaN): outcome 1 (np_simulator_dm.py:335-338)
       }
-      if (tid == 0 && !unprojected) sF[k - 1] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      if (tid == 0 && !unprojected) sF[k - 1] = make_float4(prob.x, prob.y, kNoTrace, 0.f);
       n_rec = k + 1;
       if (take1) {  // outcome 1 with P1 = I - P0
         G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
@@ -886,10 +885,9 @@ __global__ void __launch_bounds__(DmClCfg<W>::BT, 1024 / DmClCfg<W>::BT) dm_fwd_
       rinv[ri] = y;
     }
     __syncthreads();
-    const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
     if (rank == 0 && A.probs)
       for (int k = tid; k < n_rec; k += BT)
-        A.probs[run * A.ostride + k] = prob_record(sF[k - 1], ratio && (sSt[k].x & kFactZ) != 0u);
+        A.probs[run * A.ostride + k] = prob_record(sF[k - 1]);
     float2 *out = A.rho_out + run * A.out_stride;
     for (int e = tid; e < RL << n_out; e += BT) {
       const int l = e >> n_out, yj = e & (dout - 1), yi = rinv[row_of(lb, (uint32_t)l)];
@@ -1050,7 +1048,7 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       } else {
         take1 = !pair_ge(prob, 1e-4);  // prob0 < 1e-4 (or NaN): outcome 1 (np_simulator_dm.py:335-338)
       }
-      if (tid == 0 && !unprojected) sF[k] = make_float4(prob.x, prob.y, 0.f, 0.f);
+      if (tid == 0 && !unprojected) sF[k] = make_float4(prob.x, prob.y, kNoTrace, 0.f);
       n_rec = k + 1;
       if (take1) {  // outcome 1 with P1 = I - P0
         G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
@@ -1192,10 +1190,9 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       ridx[y] = ri;
     }
     __syncthreads();
-    const bool ratio = (A.flags & MBQC_F_DM_EXPECTATION) != 0u;
     if (crank == 0 && A.probs)
       for (int k = tid; k < n_rec; k += BT)
-        A.probs[run * A.ostride + k] = prob_record(sF[k], ratio && (sSt[k].x & kFactZ) != 0u);
+        A.probs[run * A.ostride + k] = prob_record(sF[k]);
     float2 *out = A.rho_out + run * A.out_stride;
     for (int e = g; e < dout * dout; e += TT) {
       const int yi = e >> n_out, yj = e & (dout - 1);
