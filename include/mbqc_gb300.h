@@ -311,8 +311,9 @@ int mbqc_sv_forward(const mbqc_plan *plan, int64_t batch, const double *angles,
  * chip (windows 11..17 in XY, X and Y: one launch) or streamed through
  * ``workspace`` in passes of up to ten fused steps (five for windows 8 and 9).
  * Same arguments and results as mbqc_sv_forward plus the workspace, sized by
- * mbqc_sv_stream_workspace (batch * 2^(w-1) * 8 bytes, 2^w below window 11,
- * plus per-run bookkeeping and epilogue partials).  The reference cannot run these windows: its dense
+ * mbqc_sv_stream_workspace (batch * 2^(w-1) * 8 bytes, 2^w below window 11 and
+ * for batches of some 15 MB at most, plus per-run bookkeeping and epilogue
+ * partials; a call that stays on chip leaves it untouched).  The reference cannot run these windows: its dense
  * 2^w x 2^w operators (gates.py:62-72,127-143) need 256 GiB at w = 17.
  */
 int mbqc_sv_stream_workspace(const mbqc_plan *plan, int64_t batch, size_t *bytes);

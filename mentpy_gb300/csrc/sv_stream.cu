@@ -2,8 +2,8 @@
 // device workspace in passes of several fused steps (windows 11..17 in XY, X and Y
 // stay on chip: sv_chip.cu).
 //
-// The window of every run is a 2^w complex64 vector in the workspace; windows
-// from 11 on keep half of it (HALF).  After step k the window is phi_k and its
+// The window of every run is a 2^w complex64 vector in the workspace; from window
+// 11 on large batches keep half of it (HALF, stream_half_pays).  After step k the window is phi_k and its
 // signed copy on the entering qubit's bit, so phi_k's 2^(w-1) amplitudes say it
 // all, and step k turns a pair (a, b) of phi_{k-1} over the measured bit into
 //   phi_k[entered 0] = a + c b,  phi_k[entered 1] = s (a +- c b)
@@ -1034,11 +1034,21 @@ static std::vector<PassDesc> make_passes(int W, int M) {
   return out;
 }
 
-// Half the window is kept (HALF) where it holds a whole mixed tile (windows >= 11)
+// Half the window can be kept (HALF) where it holds a whole mixed tile (windows >= 11)
 // and the last step lets no qubit in, so that the outputs are all in the half: every
 // plan whose window is wider than its outputs.
 static bool stream_half(const DevCircuit &hc, const DevStep *steps) {
   return hc.w >= 11 && hc.n_steps >= 1 && (steps[hc.n_steps - 1].mask & kDead) != 0u;
+}
+// In the streamed passes it pays once the whole window's tiles (2^10 amplitudes) are
+// more than the warps resident at once, twelve an SM: below, a warp has one tile or
+// none either way and only the half's longer steps are left.  XZ / YZ plans on grids
+// of 10 columns, whole against half: w = 17, 8 runs (1,024 tiles) 277 and 297 us, 16
+// (2,048) 381 and 324; w = 15, 8 runs 192 and 206, 32 (1,024) 215 and 223, 64 311 and
+// 252; w = 13, 64 runs (512) 156 and 174, 256 256 and 215.  XY, X and Y from w = 18 on: half at any batch
+// (grid 17 x 8, 1 run 260 and 264 us, 8 runs 347 and 298; 18 x 3, 1 run 254 and 245).
+static bool stream_half_pays(const DevCircuit &hc, int64_t batch) {
+  return (hc.sv_planes_ok && hc.w >= 18) || (batch << (hc.w - 10)) > (int64_t)12 * sm_count();
 }
 
 // workspace: state [B][2^S] | norms [3][B] | expo [B] | (16-byte aligned)
@@ -1065,7 +1075,8 @@ int mbqc_sv_stream_workspace(const mbqc_plan *plan, int64_t batch, size_t *bytes
   const DevCircuit &hc = host_circuit(plan, 0);
   if (hc.w < kStreamMinWindow)
     return fail(MBQC_E_UNSUPPORTED, "stream_workspace: window %d < %d", hc.w, kStreamMinWindow);
-  *bytes = stream_ws_bytes(hc, hc.w - (stream_half(hc, host_steps(plan, 0)) ? 1 : 0), batch);
+  const bool half = stream_half(hc, host_steps(plan, 0)) && stream_half_pays(hc, batch);
+  *bytes = stream_ws_bytes(hc, hc.w - (half ? 1 : 0), batch);
   return MBQC_OK;
 }
 
@@ -1087,7 +1098,12 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
     return fail(MBQC_E_INVALID, "sv_forward_stream: bad angle array");
   if (in_stride != 0 && in_stride < ((int64_t)1 << hc.n_in))
     return fail(MBQC_E_INVALID, "sv_forward_stream: input stride too small");
-  const bool half = stream_half(hc, host_steps(plan, 0));
+  // one launch on chip where the half window fits a cluster of four blocks (sv_chip.cu);
+  // XZ / YZ planes and the bulk-copy staging option keep the passes
+  const bool can_half = stream_half(hc, host_steps(plan, 0));
+  size_t chip_smem = 0;
+  const int cs = can_half && !gen && !(flags & MBQC_F_STREAM_TMA) ? chip_plan(hc, batch, &chip_smem) : 0;
+  const bool half = can_half && (cs || stream_half_pays(hc, batch));
   const int S = hc.w - (half ? 1 : 0);
   const size_t need = stream_ws_bytes(hc, S, batch);
   if (!workspace || workspace_bytes < need)
@@ -1118,13 +1134,8 @@ int mbqc_sv_forward_stream(const mbqc_plan *plan, int64_t batch, const double *a
     a.init_cz[i] = hc.init_cz[i];
   }
   cudaStream_t s = (cudaStream_t)stream;
-  // one launch on chip where the half window fits a cluster of four blocks (sv_chip.cu);
-  // XZ / YZ planes and the bulk-copy staging option keep the passes
-  if (half && !gen && !(flags & MBQC_F_STREAM_TMA)) {
-    size_t smem = 0;
-    if (const int cs = chip_plan(hc, batch, &smem))
-      return launch_sv_chip(a, hc, cs, smem, flags, reinterpret_cast<float2 *>(psi_out), logprob, status, s);
-  }
+  if (cs)
+    return launch_sv_chip(a, hc, cs, chip_smem, flags, reinterpret_cast<float2 *>(psi_out), logprob, status, s);
   const InitDesc id = make_init_desc(hc);
   const int64_t chunks = batch << (hc.w - id.K);
   const int64_t blocks = std::min<int64_t>(std::max<int64_t>(chunks, (batch + 255) / 256), (int64_t)sm_count() * 8);
