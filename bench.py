@@ -619,7 +619,7 @@ def run_ours(args, rank, world, local_rank):
     extra = {}
     if not args.headline_only:
         for name, fn in (("adjoint_many_wires_6x12", lambda: bench_adjoint(dev, fp32_peak, flush)),
-                         ("wide_window_grid_16x10", lambda: bench_wide(dev, hbm_peak, flush)),
+                         ("wide_window_grid_16x10", lambda: bench_wide(dev, hbm_peak, fp32_peak, flush)),
                          ("uneven_dm_2048_circuits", lambda: bench_uneven_dm(dev, fp32_peak, flush))):
             extra[name], tasks[name] = fn()
         # the wide workload's adjoint checks are reported inside its "adjoint" object
@@ -836,7 +836,7 @@ def bench_adjoint(dev, fp32_peak, flush, reps=5):
     }, tasks
 
 
-def bench_wide(dev, hbm_peak, flush, reps=7):
+def bench_wide(dev, hbm_peak, fp32_peak, flush, reps=7):
     """Wide window: grid_cluster(16, 10), w=17, 64 runs, |+>^16 input."""
     import torch
 
@@ -862,12 +862,15 @@ def bench_wide(dev, hbm_peak, flush, reps=7):
     out_np, ang_np = out.cpu().numpy(), ang.cpu().numpy()
     pick = np.random.default_rng(SEED + 30).choice(B, 8, replace=False)
     tasks = [("sv", ("grid", 16, 10), ang_np[r:r + 1], None, out_np[r:r + 1], None) for r in pick]
-    moved = B * (2**sw.n_in + 2**sw.n_out) * 8 + B * sw.n_angles * 8
-    roof = {"bound": "hbm", "peak": hbm_peak, "unit": "GB/s", "traffic": None,
-            "achieved": moved / (ms * 1e-3) / 1e9, "frac": moved / (ms * 1e-3) / 1e9 / hbm_peak,
-            "note": "achieved = input, angle and output bytes of one batch / batch time; the kept half of each "
-                    "run's window (2^(w-1) complex64) stays in the shared memory of a cluster of blocks for the "
-                    "whole sweep, so barriers and latency bound it, not HBM",
+    flops = B * M * 12 * 2**w  # contraction, expansion, norm and rescale of each window amplitude a step
+    moved = (2**sw.n_in + B * 2**sw.n_out) * 8 + B * sw.n_angles * 8  # one broadcast input row
+    roof = {"bound": "fp32", "achieved": flops / (ms * 1e-3) / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
+            "frac": flops / (ms * 1e-3) / 1e12 / fp32_peak, "traffic": None,
+            "note": "12 flops per amplitude of the whole 2^w window and step, of which the kernel makes half; the "
+                    "kept half of each run's window (2^(w-1) complex64) stays in the shared memory of a cluster of "
+                    "blocks for the whole sweep, so barriers and latency bound it",
+            "compulsory_gbs": moved / (ms * 1e-3) / 1e9,
+            "compulsory_note": "input, angle and output bytes of one batch / batch time",
             "per_step_model_gbs": alg / (ms * 1e-3) / 1e9,
             "per_step_model_note": "16*2^w bytes per measurement step, the reference algorithm's traffic; the "
                                    "kernel keeps the window on chip, so this is not a roofline fraction"}
