@@ -7,9 +7,13 @@ name the case they captured).
 Cases (seeded synthetic inputs with the shapes of the configuration):
   sv_mw4x8     statevector sweep, many_wires([8]*4), 4096 runs (--variant: lanes per run)
   adjoint_mw6x12 fused fidelity adjoint, many_wires([12]*6), 128 vectors x 256 inputs
-  wide_grid16x10 streamed statevector, grid_cluster(16, 10), w=17, 64 runs
+  half_grid8x10 statevector sweep, grid_cluster(8, 10), w=9, 5000 runs
+  wide_grid16x10 statevector sweep on chip, grid_cluster(16, 10), w=17, 64 runs
   adjoint_wide_grid16x10 generic adjoint of grid_cluster(16, 10), w=17, 16 runs
+  adjoint_wide_grid16x4 generic adjoint of grid_cluster(16, 4), w=17, 64 runs
   dm_mw6x12    density matrix, many_wires([12]*6) (w=7), 512 runs, noise 0.01
+  dm_adjoint_mw6x12 its adjoint, 512 runs
+  dm_grid8x6   density matrix, grid_cluster(8, 6) (w=9), 24 runs, noise 0.01
 
 Used for profiling (each case exits 0 when its kernels report no failed run).
 """
@@ -87,25 +91,60 @@ def case_wide_grid16x10(reps):
     return int((st != 0).sum())
 
 
-def case_dm_mw6x12(reps):
+def case_half_grid8x10(reps):
+    from mentpy_gb300.sweep import StatevectorSweep
+
+    rng = np.random.default_rng(7)
+    sw = StatevectorSweep(C.grid_cluster(8, 10))
+    ang = torch.tensor(rng.uniform(0, 2 * np.pi, size=(5000, sw.n_angles)), device="cuda")
+    for _ in range(reps):
+        _, st, _ = sw.forward(ang, None, logprob=True)
+    return int((st != 0).sum())
+
+
+def case_dm_mw6x12(reps, adjoint=False):
     from mentpy_gb300.dm import DensityMatrixSweep
 
     rng = np.random.default_rng(4)
     sw = DensityMatrixSweep(C.many_wires([12] * 6))
     ang = torch.tensor(rng.uniform(0, 2 * np.pi, size=(512, sw.n_angles)), device="cuda")
     inp = torch.as_tensor(_haar(rng, 6, 512), dtype=torch.complex64, device="cuda")
+    gout = torch.eye(64, dtype=torch.complex64, device="cuda").expand(512, 64, 64).contiguous()
+    gout[:, 0, 0] = 2.0
     for _ in range(reps):
-        _, _, st, _ = sw.forward(ang, inp, noise=0.01)
+        if adjoint:
+            _, _, st = sw.adjoint(ang, inp, gout, noise=0.01)
+        else:
+            _, _, st, _ = sw.forward(ang, inp, noise=0.01)
     return int((st != 0).sum())
 
 
-def case_adjoint_wide_grid16x10(reps):
+def case_dm_adjoint_mw6x12(reps):
+    return case_dm_mw6x12(reps, adjoint=True)
+
+
+def case_dm_grid8x6(reps):
+    from mentpy_gb300.dm import DensityMatrixSweep
+
+    rng = np.random.default_rng(8)
+    sw = DensityMatrixSweep(C.grid_cluster(8, 6))
+    ang = torch.tensor(rng.uniform(0, 2 * np.pi, size=(24, sw.n_angles)), device="cuda")
+    for _ in range(reps):
+        _, _, st, _ = sw.forward(ang, None, noise=0.01, want_probs=True)
+    return int((st != 0).sum())
+
+
+def case_adjoint_wide_grid16x4(reps):
+    """Generic adjoint of grid_cluster(16, 4) (w = 17), 64 runs (a cluster of two blocks per run)."""
+    return case_adjoint_wide_grid16x10(reps, cols=4, B=64)
+
+
+def case_adjoint_wide_grid16x10(reps, cols=10, B=16):
     """Generic adjoint of grid_cluster(16, 10) (w = 17), 16 runs (a cluster of four blocks per run)."""
     from mentpy_gb300.sweep import StatevectorSweep
 
     rng = np.random.default_rng(6)
-    sw = StatevectorSweep(C.grid_cluster(16, 10))
-    B = 16
+    sw = StatevectorSweep(C.grid_cluster(16, cols))
     ang = torch.tensor(rng.uniform(0, 2 * np.pi, size=(B, sw.n_angles)), device="cuda")
     g = rng.standard_normal((B, 2**sw.n_out)) + 1j * rng.standard_normal((B, 2**sw.n_out))
     gout = torch.tensor(g.astype(np.complex64), device="cuda")
@@ -117,7 +156,8 @@ def case_adjoint_wide_grid16x10(reps):
 
 CASES = {"sv_mw4x8": case_sv_mw4x8, "sv_latency": case_sv_latency, "adjoint_mw6x12": case_adjoint_mw6x12,
          "wide_grid16x10": case_wide_grid16x10, "adjoint_wide_grid16x10": case_adjoint_wide_grid16x10,
-         "dm_mw6x12": case_dm_mw6x12}
+         "adjoint_wide_grid16x4": case_adjoint_wide_grid16x4, "half_grid8x10": case_half_grid8x10,
+         "dm_mw6x12": case_dm_mw6x12, "dm_adjoint_mw6x12": case_dm_adjoint_mw6x12, "dm_grid8x6": case_dm_grid8x6}
 
 
 def main(argv=None):
