@@ -18,9 +18,9 @@
 // and log-probability are those of the streamed sweep, the amplitudes its bits.
 //
 // What bounds it is the alternation of load, compute and store phases between the
-// barriers: a group of five steps on 16,384 amplitudes takes ~5 us, 40 % of it issue
-// (two blocks an SM, windows up to 14, overlap them: a quarter better); a pass
-// between four blocks ~6.6 us.  Against the streamed passes: grid 16 x 10 (w = 17),
+// barriers: w = 17, 64 runs issue in 38 % of the slots at one block (16 warps) an SM,
+// shared memory and DRAM far from their rates (two blocks an SM, windows up to 14,
+// overlap the phases: a quarter better).  Against the streamed passes: grid 16 x 10 (w = 17),
 // 64 runs 577 -> 453 us (two rounds of 38 clusters), 16 runs 264 -> 214; 14 x 10,
 // 256 runs 509 -> 274; 12 x 10 (w = 13), 1,000 runs 594 (whole window streamed) ->
 // 240; 10 x 10, 512 runs 149 -> 77 us.  w = 18 (eight blocks a run) was slower, 64
@@ -420,7 +420,10 @@ __global__ void __launch_bounds__(1 << (SB - 5), SB >= 14 ? 1 : 512 >> (SB - 5))
 
 // Blocks per run: as few as hold the half window at 2^14 amplitudes each, 4 at most
 // (eight lose to the streamed passes, see above); twice as many (2^13 each) while the
-// batch leaves SMs idle (w = 17, 16 runs: 4 blocks 240, 8 blocks 214 us).
+// batch leaves SMs idle (w = 17, 16 runs: 4 blocks 240, 8 blocks 214 us).  At any batch:
+// one run of grid 10 x 10 (w = 11) 121 us on streamed whole windows, 117 on half, 56
+// here; 13 x 10 168, 170 and 76; 16 x 10 252, 254 and 139; of 3 columns 43, 45 and 25
+// (w = 11), 113, 115 and 57 (w = 17); 128 runs of 16 x 10 1,399, 1,066 and 901.
 int chip_plan(const DevCircuit &hc, int64_t batch, size_t *smem) {
   const int H = hc.w - 1;
   if (H < 10 || H > 16) return 0;

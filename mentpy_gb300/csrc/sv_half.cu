@@ -15,8 +15,10 @@
 // here takes V of those lanes in turn.
 //
 // Against sv_reg: grid 8 x 10 (w = 9), 5,000 runs 105 -> 68 us, 2,500 runs 68 -> 54;
-// grid 9 x 10, 5,000 runs 201 -> 140, 1,700 runs 85 -> 62.  Issue-bound at 16 warps
-// an SM.  Smaller batches stay there: a run here has a quarter to a half of the
+// grid 9 x 10, 5,000 runs 201 -> 140, 1,700 runs 85 -> 62; grids and wires of 3 to 6
+// columns, 1,217 to 16,384 runs, no slower than its lane variants.  Latency-bound: 35 %
+// of the issue slots at eight warps an SM (5,000 runs), the longest stall for
+// instructions (the steps' straight-line code).  Smaller batches stay there: a run here has a quarter to a half of the
 // lanes, so that one alone takes 48 us against 21 (sv_half_ok).
 #include <cuda_runtime.h>
 
