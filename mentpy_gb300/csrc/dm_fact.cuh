@@ -915,7 +915,7 @@ constexpr int kFactWsThreads = 512;
 
 // Sum of the hi + lo pairs of the block's threads, the same bits in each
 // (two-sum at every addition); scratch double-buffered as in group_sum2_db.
-__device__ __forceinline__ float2 block_pair_sum(float hi, float lo, float2 *scratch, int &par) {
+__device__ __forceinline__ float2 block_sum2_db(float hi, float lo, float2 *scratch, int &par) {
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
@@ -1030,12 +1030,12 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
         two_sum_acc(o_hi, o_lo, drop_coh ? tr_noise * tr - v : tr_noise * tr - v - off, 0.f);
       }
       if (k > 0) cluster_arrive();  // this block has read its diagonal
-      float2 prob = block_pair_sum(p_hi, p_lo, sRed, par);
+      float2 prob = block_sum2_db(p_hi, p_lo, sRed, par);
       float4 G = F;
       int outcome = 0;
       bool take1 = false, unprojected = false;
       if (zstep) {
-        const float2 tot = block_pair_sum(t_hi, t_lo, sRed, par);
+        const float2 tot = block_sum2_db(t_hi, t_lo, sRed, par);
         if (A.flags & MBQC_F_DM_EXPECTATION) {
           if (tid == 0) sF[k] = make_float4(prob.x, prob.y, tot.x, tot.y);
           G = make_float4(1.f, 1.f, 0.f, 0.f);
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(kFactWsThreads, 2) dm_fwd_fact_ws(DmArgs A, fl
       n_rec = k + 1;
       if (take1) {  // outcome 1 with P1 = I - P0
         G = make_float4(tr_noise - F.x, tr_noise - F.y, -F.z, -F.w);
-        prob = block_pair_sum(o_hi, o_lo, sRed, par);
+        prob = block_sum2_db(o_hi, o_lo, sRed, par);
         outcome = 1;
       }
       if (g == 0 && A.outcomes) A.outcomes[run * A.ostride + k] = (int8_t)outcome;

@@ -364,6 +364,9 @@ __global__ void __launch_bounds__(WideAdjCfg<W>::TPR) sv_adj_wide_gen(SvAdjArgs 
 // Both halves kept, one or two steps a pass: w = 17, 64 runs 4.98 ms; w = 15, 256
 // runs 2.80 -> 1.77; w = 12, 512 runs 0.60 -> 0.52; w = 19, 32 runs of 18 x 6 9.44 ->
 // 4.32 ms.  Loading the history a batch ahead was slower (2.64 ms).
+// Short circuits in small batches pay for the set-up and the sums at the run's end: w =
+// 9, 16 steps, 1 run 21.0 -> 22.8 us on the device, 64 runs 22.3 -> 25.1; w = 10, 18
+// steps 25.1 -> 27.2; from 24 steps on no case is slower.
 template <int W, int CS> struct WideHalfCfg {
   static constexpr int D = 1 << W, N = D / 2, NS = N / CS;
   static constexpr int LT = W <= 9 ? 7 : (W == 10 ? 8 : (W == 11 ? 9 : 10));
